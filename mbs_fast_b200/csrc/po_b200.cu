@@ -718,6 +718,28 @@ cudaError_t launch_diffract(int precision, int variant, bool ns, const KParams &
     }
 }
 
+// Polar rows: as many warps per orientation as leave each lane about two
+// beams (one, when the chunk has too few orientations to fill the CTA), and
+// only as many warps as the chunk's orientations use.
+cudaError_t launch_pole(const KParams &P, const LaunchPlan &L, int64_t n_beams, int n_orient,
+                        const int32_t *pole_rows, int n_pole, bool ns, cudaStream_t st)
+{
+    constexpr int kWarps = kPoleThreads / 32;
+    const int64_t mean = n_beams / std::max(1, n_orient);
+    int slices = 1;
+    while (slices < kWarps
+           && (slices * 64 < mean || (slices * 32 < mean && slices * L.orient_per_chunk < kWarps)))
+        slices *= 2;
+    const int groups = std::max(1, std::min(kWarps / slices, L.orient_per_chunk));
+    const dim3 pg((unsigned)L.n_chunks, (unsigned)n_pole);
+    const int threads = 32 * slices * groups;
+    if (ns)
+        po_pole_kernel<true><<<pg, threads, 0, st>>>(P, pole_rows, slices);
+    else
+        po_pole_kernel<false><<<pg, threads, 0, st>>>(P, pole_rows, slices);
+    return cudaGetLastError();
+}
+
 Variant shape_of(int pi, int variant, bool ns)
 {
     if (ns)
@@ -792,12 +814,8 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
     // polar rows on the side stream, concurrently with the main kernel
     if (ctx->grid.n_pole > 0) {
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
-        dim3 pg((unsigned)L.n_chunks, (unsigned)ctx->grid.n_pole);
-        if (ns)
-            po_pole_kernel<true><<<pg, 256, 0, ctx->side>>>(P, ctx->grid.pole_rows);
-        else
-            po_pole_kernel<false><<<pg, 256, 0, ctx->side>>>(P, ctx->grid.pole_rows);
-        CK(cudaGetLastError(), "pole kernel launch");
+        CK(launch_pole(P, L, s->n_beams, s->n_orient, ctx->grid.pole_rows, ctx->grid.n_pole, ns, ctx->side),
+           "pole kernel launch");
         CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
         ++launches;
     }
@@ -1869,12 +1887,8 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     if (ctx->grid.n_pole > 0) {
         CK(cudaEventRecord(ctx->ev[0], st), "event");
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
-        dim3 pg((unsigned)L.n_chunks, (unsigned)ctx->grid.n_pole);
-        if (ns)
-            po_pole_kernel<true><<<pg, 256, 0, ctx->side>>>(P, ctx->grid.pole_rows);
-        else
-            po_pole_kernel<false><<<pg, 256, 0, ctx->side>>>(P, ctx->grid.pole_rows);
-        CK(cudaGetLastError(), "pole kernel launch");
+        CK(launch_pole(P, L, s->n_beams, s->n_orient, ctx->grid.pole_rows, ctx->grid.n_pole, ns, ctx->side),
+           "pole kernel launch");
         CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
     }
     CK(cudaMemsetAsync(work, 0, sizeof(int), st), "memset work counter");

@@ -1788,56 +1788,89 @@ constexpr size_t diffract_smem_bytes()
 // Polar zenith rows (row_kind 1): every azimuth bin has the same direction
 // and polarisation basis there (Handler.h:147-160), so the row is evaluated
 // once per orientation in FP64 and written to all azimuth bins.  Grid:
-// x = orientation chunk, y = polar row index; threads stride over the
-// chunk's orientations, then a fixed-order tree sums them.
+// x = orientation chunk, y = polar row index.  An orientation's beams are
+// spread over `slices` warps (lanes stride over the beams, shuffle sums), the
+// CTA's warp groups take the chunk's orientations in turn, and every sum runs
+// in a fixed order (deterministic).  The beams' general evaluation is a chain
+// of loads and FP64 operations of a few microseconds, so what bounds the
+// kernel is how many beams one lane walks in turn: with one thread per
+// orientation (all its beams in turn) it took 204 us for one orientation of
+// 80 beams, longer than the diffraction kernel beside it (176 us), and
+// 5,990 us for 12 orientations of 1,200 beams.
+constexpr int kPoleThreads = 256;
+
 template <bool NS>
-__global__ void __launch_bounds__(256) po_pole_kernel(KParams P, const int32_t *pole_rows)
+__global__ void __launch_bounds__(kPoleThreads) po_pole_kernel(KParams P, const int32_t *pole_rows, int slices)
 {
-    __shared__ double red[256];
+    constexpr int kN = NS ? 16 : 8;
+    __shared__ double part[kPoleThreads / 32][kN];    // Jones sums per warp
+    __shared__ double msum[kPoleThreads / 32][2 * kN];  // Mueller sums per warp group
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int groups = (blockDim.x >> 5) / slices;     // orientations in flight
+    const int grp = warp / slices, slice = warp - grp * slices;
     const int chunk = blockIdx.x;
     const int t = pole_rows[blockIdx.y];
     int o0, o1;
     chunk_range(P, chunk, o0, o1);
     DirFull dc;
     dir_full(P, 0, t, dc);
-    double M[16], Mn[NS ? 16 : 1];
+    // Mueller sums of this group's orientations, held by the group's first lane
+    double M[2 * kN];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) M[i] = 0.0;
-    if (NS) {
+    for (int i = 0; i < 2 * kN; ++i) M[i] = 0.0;
+    for (int ob = o0; ob < o1; ob += groups) {
+        const int o = ob + grp;
+        double J[kN];
 #pragma unroll
-        for (int i = 0; i < (NS ? 16 : 1); ++i) Mn[i] = 0.0;
-    }
-    for (int o = o0 + threadIdx.x; o < o1; o += blockDim.x) {
-        double J[8] = {0, 0, 0, 0, 0, 0, 0, 0}, Jn[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int b = P.beam_off[o]; b < P.beam_off[o + 1]; ++b) {
-            double d[8];
-            if (beam_general(P.beams[b], P.verts, dc, P.wc, d)) {
-                for (int q = 0; q < 8; ++q) J[q] += d[q];
-                if (NS && !(P.beams[b].flags & MBS_PO_BEAM_EXTERNAL))
-                    for (int q = 0; q < 8; ++q) Jn[q] += d[q];
+        for (int q = 0; q < kN; ++q) J[q] = 0.0;
+        if (o < o1) {
+            const int b1 = P.beam_off[o + 1];
+            for (int b = P.beam_off[o] + slice * 32 + lane; b < b1; b += slices * 32) {
+                double d[8];
+                if (beam_general(P.beams[b], P.verts, dc, P.wc, d)) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) J[q] += d[q];
+                    if (NS && !(P.beams[b].flags & MBS_PO_BEAM_EXTERNAL)) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) J[NS ? 8 + q : q] += d[q];
+                    }
+                }
             }
         }
-        const double wgt = P.weight[o] * 0.25;
-        mueller_add(J, wgt, M);
-        if (NS)
-            mueller_add(Jn, wgt, Mn);
+#pragma unroll
+        for (int q = 0; q < kN; ++q) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1)
+                J[q] += __shfl_xor_sync(0xffffffffu, J[q], off);
+            if (lane == 0)
+                part[warp][q] = J[q];
+        }
+        __syncthreads();
+        if (slice == 0 && lane == 0 && o < o1) {
+            for (int s = 1; s < slices; ++s)
+#pragma unroll
+                for (int q = 0; q < kN; ++q)
+                    J[q] += part[warp + s][q];
+            const double wgt = P.weight[o] * 0.25;
+            mueller_add(J, wgt, M);
+            if (NS)
+                mueller_add(J + (NS ? 8 : 0), wgt, M + (NS ? 16 : 0));
+        }
+        __syncthreads();   // the partial sums are read before the next round
     }
+    if (slice == 0 && lane == 0)
+#pragma unroll
+        for (int i = 0; i < 2 * kN; ++i)
+            msum[grp][i] = M[i];
+    __syncthreads();
     const size_t G = (size_t)P.n_az * P.n_t;
-    for (int set = 0; set < (NS ? 2 : 1); ++set) {
-        double *out = (set == 0 ? P.partial : P.partial_ns) + (size_t)chunk * 16 * G;
-        for (int i = 0; i < 16; ++i) {
-            red[threadIdx.x] = set == 0 ? M[i] : Mn[NS ? i : 0];
-            __syncthreads();
-            for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-                if ((int)threadIdx.x < s)
-                    red[threadIdx.x] += red[threadIdx.x + s];
-                __syncthreads();
-            }
-            const double v = red[0];
-            for (int pp = threadIdx.x; pp < P.n_az; pp += blockDim.x)
-                out[(size_t)i * G + (size_t)pp * P.n_t + t] = v;
-            __syncthreads();
-        }
+    for (int i = threadIdx.x; i < 2 * kN * P.n_az; i += blockDim.x) {
+        const int e = i / P.n_az, pp = i - e * P.n_az;
+        double v = msum[0][e];
+        for (int g = 1; g < groups; ++g)
+            v += msum[g][e];
+        double *out = (e < 16 ? P.partial : P.partial_ns) + (size_t)chunk * 16 * G;
+        out[(size_t)(e & 15) * G + (size_t)pp * P.n_t + t] = v;
     }
 }
 

@@ -1,0 +1,40 @@
+"""The device paths at the sizes where their work splits change, on synthetic
+batches, against the CPU oracle (run on the B200: pytest -m gpu)."""
+import numpy as np
+import pytest
+
+import oracle
+from mbs_fast_b200 import abi
+from mbs_fast_b200.handler import GpuHandlerPO
+from tests import synthetic as S
+
+# FP64 against the oracle: both carry vertex phases of up to 1.3e3 rad with
+# rounding errors near 2e-13 rad; the gate of the traced FP64 parity tests
+# (tests/test_parity_gpu.py).
+FP64_L2 = 1e-8
+
+
+def _l2(a, b):
+    a, b = np.asarray(a), np.asarray(b)
+    return float(np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_orient,beams", [(1, 2), (1, 33), (3, 70), (9, 31), (20, 64), (40, 8), (2, 700)])
+def test_polar_rows(n_orient, beams):
+    """Polar rows: one warp to a whole CTA per orientation, ragged and empty
+    orientations, with and without the sums over internal beams."""
+    b = S.ragged(n_orient, beams, 20.0, 3 + n_orient + beams)
+    g, w = S.grid(5, 3), S.wave()
+    M0, N0 = oracle.po_diffract(b, g, w, noshadow=True)
+    h = GpuHandlerPO(g, w)
+    M, N, P = h.new_mueller(), h.new_mueller(), h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, N, precision=abi.FP64)
+    assert h.handle_orientations_to_local_gpu(b, P, precision=abi.FP64)
+    h.close()
+    for t in (0, 3):
+        assert _l2(M[:, t], M0[:, t]) < FP64_L2
+        assert _l2(P[:, t], M0[:, t]) < FP64_L2
+        assert _l2(N[:, t], N0[:, t]) < FP64_L2
+        assert all(np.array_equal(M[0, t], M[p, t]) for p in range(5))
+    assert _l2(M, M0) < FP64_L2
