@@ -637,12 +637,18 @@ struct LaunchPlan {
 // 1 % longer FP32C and FP64 steps on the column; 32: 3 %), at 256 planes of
 // 11 MB on the headline grid.
 constexpr int kMaxChunks = 256;
+// Small batches split down to single orientations until a resident CTA has
+// about this many items.  With at least 8 orientations per chunk whatever the
+// batch, 16 orientations on 48 x 181 directions made 96 items for 592 resident
+// CTAs (FP64 834 us, now 292), 12 aggregate orientations on 48 x 1801 240 for
+// 444 (FP32C 10.28 ms, now 7.29), 96 column orientations 5,760 for 592 (FP64
+// 11.38 ms, now 11.14; 4 items: 11.38, 8: 11.39, 32: 11.12).
+constexpr int kMinItems = 16;
 
 // Orientation chunks per output set: enough work items (chunk x azimuth x
 // zenith tile) for about kMaxChunks / 2 per resident CTA of the persistent
 // kernel, at most kMaxChunks chunks per set (each chunk owns a partial
 // plane).  n_orient is per set; n_chunks counts all sets.
-
 LaunchPlan plan_launch(int n_az, int n_t, int n_orient, int dirs_per_cta, int ctas_per_sm,
                        int n_sets = 1)
 {
@@ -659,11 +665,15 @@ LaunchPlan plan_launch(int n_az, int n_t, int n_orient, int dirs_per_cta, int ct
     n_sets = std::max(1, n_sets);
     const long long target = (long long)sms * ctas_per_sm * (kMaxChunks / 2);
     long long chunks = (target + ctas_per_chunk * n_sets - 1) / (ctas_per_chunk * n_sets);
-    // at least 8 orientations per chunk: small calls (the drop-in's first,
-    // growing batches) keep few partial planes, so the context's partial
-    // buffer does not grow through many large allocations
+    // At least 8 orientations per chunk: small calls (the drop-in's first,
+    // growing batches) keep few partial planes.  Unless that leaves too few
+    // work items per resident CTA: then down to one orientation per chunk, up
+    // to the 64 planes that the context's first partial buffer holds anyway.
     chunks = std::max<long long>(1, std::min<long long>(chunks, std::max(1, n_orient / 8)));
-    chunks = std::min<long long>(chunks, kMaxChunks);
+    const long long few = ((long long)sms * ctas_per_sm * kMinItems + ctas_per_chunk * n_sets - 1)
+                        / (ctas_per_chunk * n_sets);
+    chunks = std::max(chunks, std::min<long long>({few, (long long)n_orient, (long long)std::max(1, 64 / n_sets)}));
+    chunks = std::max<long long>(1, std::min<long long>(chunks, kMaxChunks));
     L.orient_per_chunk = (int)((n_orient + chunks - 1) / chunks);
     L.chunks_per_set = (int)((n_orient + L.orient_per_chunk - 1) / std::max(1, L.orient_per_chunk));
     if (L.chunks_per_set < 1) L.chunks_per_set = 1;

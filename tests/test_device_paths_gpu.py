@@ -38,3 +38,38 @@ def test_polar_rows(n_orient, beams):
         assert _l2(N[:, t], N0[:, t]) < FP64_L2
         assert all(np.array_equal(M[0, t], M[p, t]) for p in range(5))
     assert _l2(M, M0) < FP64_L2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_orient", [1, 7, 13, 65, 130])
+@pytest.mark.parametrize("precision", [abi.FP64, abi.FP32C])
+def test_small_batches_split_into_single_orientations(n_orient, precision):
+    """Few orientations on a small grid: one to a few orientations per chunk,
+    up to 64 chunk planes, ragged beam counts, empty orientations.  FP32C: the
+    gate of the traced FP32C parity tests on the whole grid's L2."""
+    b = S.ragged(n_orient, 9, 15.0, 100 + n_orient)
+    g, w = S.grid(3, 6), S.wave()
+    M0, N0 = oracle.po_diffract(b, g, w, noshadow=True)
+    h = GpuHandlerPO(g, w)
+    M, N, P = h.new_mueller(), h.new_mueller(), h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, N, precision=precision)
+    assert h.handle_orientations_to_local_gpu(b, P, precision=precision)
+    h.close()
+    gate = FP64_L2 if precision == abi.FP64 else 2e-5
+    assert _l2(M, M0) < gate and _l2(P, M0) < gate
+    assert _l2(N, N0) < (gate if precision == abi.FP64 else 1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_sizes", [1, 3, 65])
+def test_small_multisize_batches(n_sizes):
+    """Chunk planes shared by the sizes: up to 64 in all, then one per size."""
+    b = S.batch(4, 6, 5.0, 7, raw=True, absorbing=True)
+    g, w = S.grid(3, 5), S.wave(True)
+    scales = np.geomspace(0.5, 3.0, n_sizes)
+    h = GpuHandlerPO(g, w)
+    ms = [h.new_mueller() for _ in scales]
+    assert h.handle_orientations_to_local_gpu_multik(b, 0, 4, scales, w.wave_index, ms)
+    h.close()
+    for s, M in list(zip(scales, ms))[::16] + [(scales[-1], ms[-1])]:
+        assert _l2(M, oracle.po_diffract(oracle.scale_batch(b, s, w.wave_index, w.abs_coeff), g, w)) < FP64_L2
