@@ -477,8 +477,20 @@ namespace {
 // the wave constants set when it was staged.  With `scales` the batch is
 // staged once per size factor (instance i = scales[i]); instance i's
 // orientations are [i nO, (i+1) nO) and its results go to output set i.
+// `what`: the records the call reads (a batch kept for later calls has all;
+// one staged for a single call leaves out what its kernels do not read).
+constexpr unsigned kStageDiffract = 1;   // BeamRec and VertRec
+constexpr unsigned kStageMoments = 2;    // FP32C near-forward moments
+constexpr unsigned kStageAll = kStageDiffract | kStageMoments;
+
+unsigned stage_for(int precision)
+{
+    return precision == MBS_PO_FP64 ? kStageDiffract : kStageAll;
+}
+
 int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStream_t st,
-               const double *scales = nullptr, int n_scales = 0, double k_rephase = 0.0)
+               const double *scales = nullptr, int n_scales = 0, double k_rephase = 0.0,
+               unsigned what = kStageAll)
 {
     int rc = validate(ctx, b);
     if (rc)
@@ -597,16 +609,15 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
         P.wc = ctx->wc;
         P.beams = s->beams;
         P.verts = s->verts;
-        P.brec = s->brec;
-        P.vrec = s->vrec;
+        P.brec = what & kStageDiffract ? s->brec : nullptr;
+        P.vrec = what & kStageDiffract ? s->vrec : nullptr;
         P.brec_stride = iB;
         P.vrec_stride = iV;
-        P.moments = s->moments;
+        P.moments = what & kStageMoments ? s->moments : nullptr;
         P.vbeg = s->vbeg;
         P.status = ctx->d_status;
-        const int threads = 128;
-        const dim3 blocks((unsigned)((nB + 1 + threads - 1) / threads), (unsigned)nI);
-        po_pack_kernel<<<blocks, threads, 0, st>>>(P);
+        const dim3 blocks((unsigned)((nB + kPackBeams - 1) / kPackBeams), (unsigned)nI);
+        po_pack_kernel<<<blocks, kPackThreads, 0, st>>>(P);
         CK(cudaGetLastError(), "pack kernel launch");
         int status = 0;
         CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
@@ -1186,7 +1197,8 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
     for (double &v : ctx->prof)
         v = 0.0;
     CK(cudaEventRecord(ctx->ev[3], st), "event");
-    if (!pre && (rc = stage_into(ctx, beams, &ctx->host_staged, st, scales, n_scales, k_rephase)))
+    if (!pre && (rc = stage_into(ctx, beams, &ctx->host_staged, st, scales, n_scales, k_rephase,
+                                 stage_for(precision))))
         return rc;
     const double td0 = host_ms();
     CK(cudaEventRecord(ctx->ev[4], st), "event");
@@ -1564,7 +1576,7 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
         sub.beam_raw = nullptr;
         sub.abs_offsets = nullptr;
         sub.abs_paths = nullptr;
-        if ((rc = stage_into(ctx, &sub, &ctx->host_staged, st)))
+        if ((rc = stage_into(ctx, &sub, &ctx->host_staged, st, nullptr, 0, 0.0, stage_for(precision))))
             break;
         if (sub.n_beams == 0)
             continue;
@@ -1608,7 +1620,7 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         m11_out[i] = 0.0;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     cudaStream_t st = ctx->stream;
-    int rc = stage_into(ctx, beams, &ctx->host_staged, st);
+    int rc = stage_into(ctx, beams, &ctx->host_staged, st, nullptr, 0, 0.0, 0);
     if (rc)
         return rc;
     const mbs_po_staged &s = ctx->host_staged;
@@ -1669,7 +1681,7 @@ extern "C" int mbs_po_extinction(mbs_po_ctx *ctx, const mbs_po_beams *beams, dou
     if (beams->n_orient == 0)
         return MBS_PO_OK;
     cudaStream_t st = ctx->stream;
-    int rc = stage_into(ctx, beams, &ctx->host_staged, st);
+    int rc = stage_into(ctx, beams, &ctx->host_staged, st, nullptr, 0, 0.0, 0);
     if (rc)
         return rc;
     double *d = nullptr;

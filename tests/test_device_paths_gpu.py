@@ -73,3 +73,51 @@ def test_small_multisize_batches(n_sizes):
     h.close()
     for s, M in list(zip(scales, ms))[::16] + [(scales[-1], ms[-1])]:
         assert _l2(M, oracle.po_diffract(oracle.scale_batch(b, s, w.wave_index, w.abs_coeff), g, w)) < FP64_L2
+
+
+def _with_nv(n_beams, nv, size, seed):
+    """One orientation whose beams are regular-ish polygons of nv vertices
+    (the generator's polygons stop at 8)."""
+    b = S.batch(1, n_beams, size, seed)
+    rng = np.random.default_rng(seed)
+    n = b.n_beams
+    ang = (np.arange(nv)[None, :] + rng.uniform(-0.3, 0.3, (n, nv))) * (2 * np.pi / nv)
+    r = size * rng.uniform(0.05, 0.6, (n, 1))
+    x, y = r * np.cos(ang), 0.6 * r * np.sin(ang)
+    dx, dy = np.roll(x, -1, 1) - x, np.roll(y, -1, 1) - y
+    b.vert_offsets = np.arange(n + 1, dtype=np.int64) * nv
+    c = lambda a: np.ascontiguousarray(a.ravel())
+    b.vx, b.vy, b.slope_yx, b.slope_xy = c(x), c(y), c(dy / dx), c(dx / dy)
+    b.edge_flags = np.full(n * nv, 3, np.uint8)
+    g = b.beam_geom.copy()
+    g[:, abi.G_AREA] = 0.5 * np.sum(x * np.roll(y, -1, 1) - np.roll(x, -1, 1) * y, 1)
+    b.beam_geom = g
+    return b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_beams,nv", [(1, 3), (15, 31), (16, 8), (17, 9), (33, 4), (160, 31)])
+def test_packed_records(n_beams, nv):
+    """Record building 16 beams at a time: beam counts around the group, 3 to
+    31 vertices (fewer and more than the 8 lanes of a beam).  FP64 without
+    moments, FP32C with them, and the staged batch, which has both, bit for
+    bit as the host calls.  The FP32C gate is that of the traced parity tests,
+    whose apertures have 3 to 12 vertices, so it is asked of those here."""
+    import torch
+    b = _with_nv(n_beams, nv, 6.0, 11 * n_beams + nv)
+    g, w = S.grid(4, 12, plates=True), S.wave()
+    M0 = oracle.po_diffract(b, g, w)
+    h = GpuHandlerPO(g, w)
+    st = h.stage(b)
+    for prec, gate in ((abi.FP64, FP64_L2), (abi.FP32C, 2e-5)):
+        M = h.new_mueller()
+        assert h.handle_orientations_to_local_gpu(b, M, precision=prec)
+        if prec == abi.FP64 or nv <= 12:
+            assert _l2(M, M0) < gate
+            assert _l2(M[:, :4], M0[:, :4]) < gate
+        acc = torch.zeros(M.size, dtype=torch.float64, device="cuda:0")
+        h.diffract_staged(st, acc.data_ptr(), precision=prec)
+        torch.cuda.synchronize()
+        assert np.array_equal(acc.cpu().numpy(), M.ravel())
+    st.free()
+    h.close()
