@@ -1688,10 +1688,14 @@ extern "C" int mbs_po_extinction(mbs_po_ctx *ctx, const mbs_po_beams *beams, dou
     size_t cap = 0;
     if ((rc = ensure(ctx, d, cap, (size_t)beams->n_orient, "cext")))
         return rc;
-    const int th = 128;
-    po_extinction_kernel<<<(beams->n_orient + th - 1) / th, th, 0, st>>>(
+    // a warp per orientation, more where that leaves a lane over four beams
+    int slices = 1;
+    while (slices < kExtThreads / 32 && (int64_t)slices * 128 * beams->n_orient < beams->n_beams)
+        slices *= 2;
+    const int per_cta = kExtThreads / 32 / slices;
+    po_extinction_kernel<<<(beams->n_orient + per_cta - 1) / per_cta, kExtThreads, 0, st>>>(
         ctx->host_staged.beams, ctx->host_staged.verts, ctx->host_staged.beam_off,
-        ctx->host_staged.weight, beams->n_orient, ctx->wc, d);
+        ctx->host_staged.weight, beams->n_orient, slices, ctx->wc, d);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(cext_out, d, beams->n_orient * sizeof(double), cudaMemcpyDeviceToHost, st);

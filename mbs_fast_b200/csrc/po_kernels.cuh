@@ -550,16 +550,18 @@ __device__ __forceinline__ void dir_full(const KParams &P, int p, int t, DirFull
 // One beam's Jones contribution d[8] to one direction in FP64.  Returns
 // false when the reference would skip the beam (NaN integral).
 // `singular` = false drops nearly singular edges (|C_e| <= eps1) instead of
-// taking their stable quotient, the reference's singularCorrection = 0.
+// taking their stable quotient, the reference's singularCorrection = 0;
+// `common` = false leaves out an internal beam's common phase.
 __device__ __noinline__ bool beam_general(const DevBeam &g, const DevVert *gv, const DirFull &dc,
-                                          const WaveConst &wc, double *d, bool singular = true)
+                                          const WaveConst &wc, double *d, bool singular = true,
+                                          bool common = true)
 {
     const double k = wc.k;
     const double a_sin = -dc.cp * g.h[0] - dc.sp * g.h[1];
     const double b_sin = -dc.cp * g.v[0] - dc.sp * g.v[1];
     const double A = fma(dc.st, a_sin, fma(dc.ct, g.h[2], g.a0));
     const double B = fma(dc.st, b_sin, fma(dc.ct, g.v[2], g.b0));
-    const bool internal = !(g.flags & MBS_PO_BEAM_EXTERNAL);
+    const bool internal = common && !(g.flags & MBS_PO_BEAM_EXTERNAL);
     const double cm = internal ? -k * (dc.st * (dc.cp * g.c[0] + dc.sp * g.c[1]) + dc.ct * (-g.c[2])) : 0.0;
     const DevVert *v = gv + g.vbeg;
     const int nv = g.nv;
@@ -2176,15 +2178,22 @@ __global__ void po_thetas_sum_kernel(const double *partial, int n_chunks, int n_
 }
 
 // --------------------------------------------------------- extinction
-// One thread per orientation: HandlerPO::ComputeForwardExtinctionOt
-// (reference HandlerPO.cpp:1812-2009) at zenith 0, azimuth 0.
-__global__ void po_extinction_kernel(const DevBeam *beams, const DevVert *verts,
-                                     const int32_t *beam_off, const double *weight,
-                                     int n_orient, WaveConst wc, double *cext)
+// HandlerPO::ComputeForwardExtinctionOt (reference HandlerPO.cpp:1812-2009) at
+// zenith 0, azimuth 0: `slices` warps per orientation, lanes striding over its
+// beams, sums in a fixed order.  Each beam is one general evaluation (a chain
+// of loads and FP64 operations), so the time is the number of beams a lane
+// takes in turn: one thread per orientation took 1,186 us for 1,024
+// orientations of 87 beams.
+constexpr int kExtThreads = 128;
+
+__global__ void __launch_bounds__(kExtThreads) po_extinction_kernel(
+    const DevBeam *beams, const DevVert *verts, const int32_t *beam_off, const double *weight,
+    int n_orient, int slices, WaveConst wc, double *cext)
 {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= n_orient)
-        return;
+    __shared__ double part[kExtThreads / 32][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = warp / slices, slice = warp - grp * slices;
+    const int o = blockIdx.x * ((kExtThreads / 32) / slices) + grp;
     const double k = wc.k;
     DirFull dc;
     dc.st = 0.0; dc.ct = 1.0; dc.cp = 1.0; dc.sp = 0.0;
@@ -2193,27 +2202,26 @@ __global__ void po_extinction_kernel(const DevBeam *beams, const DevVert *verts,
     cross3(dc.vf, dc.dir, dc.u);
     dc.vt[0] = dc.u[0]; dc.vt[1] = dc.u[1]; dc.vt[2] = dc.u[2];
     cross3(dc.vt, dc.dir, dc.w);
-    double f00r = 0, f00i = 0, f11r = 0, f11i = 0;
-    for (int b = beam_off[o]; b < beam_off[o + 1]; ++b) {
-        DevBeam g = beams[b];
+    double f[4] = {0.0, 0.0, 0.0, 0.0};   // S00 and S11 (re, im)
+    const int b1 = o < n_orient ? beam_off[o + 1] : 0;
+    for (int b = (o < n_orient ? beam_off[o] : 0) + slice * 32 + lane; b < b1; b += slices * 32) {
+        const DevBeam &g = beams[b];
         const bool external = (g.flags & MBS_PO_BEAM_EXTERNAL) != 0;
         if (wc.ot_phase_avg && !external)
             continue;
         // The extinction phase reference differs from the scattering one
         // (HandlerPO.cpp:1965-1977): external beams take exp(-ik opticalPath),
-        // internal ones exp(-ik(cos t dp_cos + farReference)).  beam_general
-        // is run on a copy flagged external (no common phase), and the
-        // reference's factor is applied here.
+        // internal ones exp(-ik(cos t dp_cos + farReference)), so beam_general
+        // runs without the common phase and that factor is applied here.
         const double ref = external ? g.opath : wc.ot_far_ref;
-        g.flags |= MBS_PO_BEAM_EXTERNAL;
         // The reference drops beams whose 1/A or 1/B divisor is nearly
         // singular at this direction (HandlerPO.cpp:1920-1921, 1945-1946).
         const double A = g.h[2] + g.a0, B = g.v[2] + g.b0;
         double dd[8], pr, pi;
-        const bool small = small_phase_factor(verts + g.vbeg, g.nv, A, B, k, pr, pi);
-        if (!small && ((fabs(B) > fabs(A)) ? fabs(B) <= wc.eps1 : fabs(A) <= wc.eps1))
+        if (((fabs(B) > fabs(A)) ? fabs(B) <= wc.eps1 : fabs(A) <= wc.eps1)
+            && !small_phase_factor(verts + g.vbeg, g.nv, A, B, k, pr, pi))
             continue;
-        if (!beam_general(g, verts, dc, wc, dd))
+        if (!beam_general(g, verts, dc, wc, dd, true, false))
             continue;
         double ph = 0.0;
         if (!external)
@@ -2224,10 +2232,25 @@ __global__ void po_extinction_kernel(const DevBeam *beams, const DevVert *verts,
         if (ph != 0.0)
             sincos_rad(ph, s, c);
         // the CPU rotation carries 0.5 (HandlerPO_fast.h:643-646)
-        f00r += 0.5 * (dd[0] * c - dd[1] * s); f00i += 0.5 * (dd[0] * s + dd[1] * c);
-        f11r += 0.5 * (dd[6] * c - dd[7] * s); f11i += 0.5 * (dd[6] * s + dd[7] * c);
+        f[0] += 0.5 * (dd[0] * c - dd[1] * s); f[1] += 0.5 * (dd[0] * s + dd[1] * c);
+        f[2] += 0.5 * (dd[6] * c - dd[7] * s); f[3] += 0.5 * (dd[6] * s + dd[7] * c);
     }
-    const double fwr = f00r + f11r, fwi = f00i + f11i;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            f[i] += __shfl_xor_sync(0xffffffffu, f[i], off);
+        if (lane == 0)
+            part[warp][i] = f[i];
+    }
+    __syncthreads();
+    if (slice != 0 || lane != 0 || o >= n_orient)
+        return;
+    for (int s = 1; s < slices; ++s)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            f[i] += part[warp + s][i];
+    const double fwr = f[0] + f[2], fwi = f[1] + f[3];
     double amp = fwi;
     if (wc.ot_ping != 0.0) {
         double sn, cs;

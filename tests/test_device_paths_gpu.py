@@ -121,3 +121,20 @@ def test_packed_records(n_beams, nv):
         assert np.array_equal(acc.cpu().numpy(), M.ravel())
     st.free()
     h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_orient,beams", [(1, 2), (3, 40), (5, 127), (5, 300), (70, 33), (2, 1300)])
+@pytest.mark.parametrize("phase_average", [0, 1])
+def test_extinction_splits(n_orient, beams, phase_average):
+    """Extinction with one to four warps per orientation, ragged and empty
+    orientations, with and without the phase-averaged form.  Both sides sum
+    the same terms; internal beams carry a phase of k (1e4 um + ...) = 1.2e5
+    rad (rounding 1.5e-11): 1e-9 of the largest orientation's value."""
+    b, w = S.ragged(n_orient, beams, 20.0, 5 + n_orient + beams), S.wave()
+    w.ot_phase_average = phase_average
+    want = oracle.po_extinction(b, w)
+    h = GpuHandlerPO(S.grid(1, 2), w)
+    got = h.extinction(b)
+    h.close()
+    assert np.max(np.abs(got - want)) <= 1e-9 * np.max(np.abs(want))
