@@ -1620,7 +1620,7 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         m11_out[i] = 0.0;
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     cudaStream_t st = ctx->stream;
-    int rc = stage_into(ctx, beams, &ctx->host_staged, st, nullptr, 0, 0.0, 0);
+    int rc = stage_into(ctx, beams, &ctx->host_staged, st, nullptr, 0, 0.0, kStageDiffract);
     if (rc)
         return rc;
     const mbs_po_staged &s = ctx->host_staged;
@@ -1639,33 +1639,57 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         tab[n + i] = std::cos(th);
     }
     const int nAz = ctx->grid.n_az;
-    const int64_t pairs = s.n_beams * nAz;
-    // chunks of about 64 (beam, azimuth) pairs per thread, at most 4096
-    int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(4096, pairs / (256 * 64)));
-    const int bpc = (int)((s.n_beams + chunks - 1) / chunks);
+    // three points per thread where a tile of 192 is mostly used; beam chunks
+    // for about 16 CTAs per resident one, whole stages each
+    const int dpt = n > 2 * kThetaTpb ? 3 : 1;
+    const int tiles = (n + dpt * kThetaTpb - 1) / (dpt * kThetaTpb);
+    int64_t chunks = std::max<int64_t>(1, (int64_t)148 * 4 * 16 / ((int64_t)tiles * nAz));
+    chunks = std::min<int64_t>(chunks, (s.n_beams + kThetaBeams - 1) / kThetaBeams);
+    int64_t bpc = (s.n_beams + chunks - 1) / chunks;
+    bpc = (bpc + kThetaBeams - 1) / kThetaBeams * kThetaBeams;
     chunks = (s.n_beams + bpc - 1) / bpc;
+    const int64_t rows = chunks * nAz;
+    // scratch from the context's pool: the partial sums take megabytes, and a
+    // cudaMalloc and cudaFree of that size per call took longer than the kernel
     double *buf = nullptr;
-    size_t cap = 0;
-    const size_t need = 2 * (size_t)n + (size_t)chunks * n + n;
-    if ((rc = ensure(ctx, buf, cap, need, "theta scan")))
-        return rc;
-    double *d_st = buf, *d_ct = buf + n, *part = buf + 2 * n, *d_m11 = part + (size_t)chunks * n;
-    cudaError_t e = cudaMemcpyAsync(buf, tab.data(), 2 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st);
+    const size_t need = 2 * (size_t)n + (size_t)rows * n + n;
+    cudaError_t e = cudaMallocFromPoolAsync((void **)&buf, need * sizeof(double), ctx->pool, st);
+    if (e != cudaSuccess)
+        return fail(ctx, MBS_PO_ENOMEM, std::string("theta scan scratch: ") + cudaGetErrorString(e));
+    double *d_st = buf, *d_ct = buf + n, *part = buf + 2 * n, *d_m11 = part + (size_t)rows * n;
+    KParams P{};
+    P.beams = s.beams;
+    P.verts = s.verts;
+    P.brec = s.brec;
+    P.vrec = s.vrec;
+    P.brec_stride = s.n_beams;
+    P.vrec_stride = s.n_verts;
+    P.vbeg = s.vbeg;
+    P.beam_off = s.beam_off;
+    P.weight = s.weight;
+    P.sphi = ctx->grid.sphi;
+    P.cphi = ctx->grid.cphi;
+    P.n_az = nAz;
+    P.n_orient = s.n_orient;
+    P.wc = ctx->wc;
+    e = cudaMemcpyAsync(buf, tab.data(), 2 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        po_thetas_kernel<<<dim3((unsigned)n, (unsigned)chunks), 256, 0, st>>>(
-            s.beams, s.verts, s.beam_off, s.weight, s.n_orient, s.n_beams, bpc, d_st, d_ct,
-            ctx->grid.sphi, ctx->grid.cphi, nAz, n, ctx->wc, part);
+        const dim3 g((unsigned)(tiles * nAz), (unsigned)chunks);
+        if (dpt == 3)
+            po_thetas_kernel<3><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, tiles, d_st, d_ct, n, part);
+        else
+            po_thetas_kernel<1><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, tiles, d_st, d_ct, n, part);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        po_thetas_sum_kernel<<<(n + 127) / 128, 128, 0, st>>>(part, (int)chunks, n, d_m11);
+        po_thetas_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(part, rows, n, d_m11);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m11_out, d_m11, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
-    cudaFree(buf);
+    cudaFreeAsync(buf, st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "theta scan");
     return MBS_PO_OK;

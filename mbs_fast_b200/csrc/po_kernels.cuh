@@ -1014,10 +1014,14 @@ __device__ __forceinline__ float rcp_t(float x) { return rcp32(x); }
 // (x branch) and (A, B, slope_xy) otherwise (y branch).  All vertex phasors
 // are independent, so the NV*DPT chains interleave.  mn[d] receives the
 // smallest |C_e| (nearly singular edges go to the FP64 pass).
-template <typename T, int DPT, int NV>
+// With kDrop an edge with |C_e| <= eps is left out instead (its coefficient
+// becomes kDropped, its term 1e-100 of the others).
+constexpr double kDropped = 1e100;
+
+template <typename T, int DPT, int NV, bool kDrop>
 __device__ __forceinline__ void edge_sums_fixed(const SVertRaw<T> *v, const double *st, const double *ct,
                                                 const T *X1, const T *X2, const bool *useX,
-                                                T *sr, T *si, T *mn, const double2 *tab)
+                                                T *sr, T *si, T *mn, const double2 *tab, double eps)
 {
     T c[DPT][NV], s[DPT][NV], syx[NV], sxy[NV];
 #pragma unroll
@@ -1042,10 +1046,14 @@ __device__ __forceinline__ void edge_sums_fixed(const SVertRaw<T> *v, const doub
     for (int e = 0; e < NV; e += 2) {
 #pragma unroll
         for (int d = 0; d < DPT; ++d) {
-            const T ca = fma(useX[d] ? syx[e] : sxy[e], X1[d], X2[d]);
+            T ca = fma(useX[d] ? syx[e] : sxy[e], X1[d], X2[d]);
+            if (kDrop && fabs(ca) <= eps)
+                ca = kDropped;
             const int e1 = (e + 1 < NV) ? e + 1 : 0;
             if (e + 1 < NV) {
-                const T cb = fma(useX[d] ? syx[e1] : sxy[e1], X1[d], X2[d]);
+                T cb = fma(useX[d] ? syx[e1] : sxy[e1], X1[d], X2[d]);
+                if (kDrop && fabs(cb) <= eps)
+                    cb = kDropped;
                 const T r = rcp_t(ca * cb);
                 const T ia = cb * r, ib = ca * r;
                 const int e2 = (e + 2 < NV) ? e + 2 : 0;
@@ -1212,11 +1220,11 @@ __device__ __forceinline__ void edge_tail_loop_f32(const SVertRaw<float> *v, int
     }
 }
 
-template <typename T, int DPT>
+template <typename T, int DPT, bool kDrop>
 __device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, const double *st,
                                                const double *ct, const T *X1, const T *X2,
                                                const bool *useX, T *sr, T *si, T *mn,
-                                               const double2 *tab)
+                                               const double2 *tab, double eps)
 {
     T c0[DPT], s0[DPT], cp_[DPT], sp_[DPT];
     T syx, sxy;
@@ -1241,7 +1249,9 @@ __device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, con
             T cn = c0[d], sn = s0[d];
             if (!last)
                 vertex_phasor_t(st[d], ct[d], w, tab, sn, cn);
-            const T coef = fma(useX[d] ? syx_e : sxy_e, X1[d], X2[d]);
+            T coef = fma(useX[d] ? syx_e : sxy_e, X1[d], X2[d]);
+            if (kDrop && fabs(coef) <= eps)
+                coef = kDropped;
             const T inv = rcp_t(coef);
             mn[d] = fmin(mn[d], fabs(coef));
             sr[d] = fma(cn - cp_[d], inv, sr[d]);
@@ -1254,19 +1264,19 @@ __device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, con
 
 // FP64 edge sums of one beam (the FP32C path uses edge_head_f32 and the
 // tails above): fixed vertex counts unrolled, longer apertures in a loop.
-template <typename T, int DPT>
+template <typename T, int DPT, bool kDrop = false>
 __device__ __forceinline__ void edge_sums(const SVertRaw<T> *v, int nv, const double *st,
                                           const double *ct, const T *X1, const T *X2,
                                           const bool *useX, T *sr, T *si, T *mn,
-                                          const double2 *tab)
+                                          const double2 *tab, double eps = 0.0)
 {
     static_assert(sizeof(T) == 8, "FP64 path");
     switch (nv) {   // warp-uniform: every lane evaluates the same beam
-    case 3: edge_sums_fixed<T, DPT, 3>(v, st, ct, X1, X2, useX, sr, si, mn, tab); break;
-    case 4: edge_sums_fixed<T, DPT, 4>(v, st, ct, X1, X2, useX, sr, si, mn, tab); break;
-    case 5: edge_sums_fixed<T, DPT, 5>(v, st, ct, X1, X2, useX, sr, si, mn, tab); break;
-    case 6: edge_sums_fixed<T, DPT, 6>(v, st, ct, X1, X2, useX, sr, si, mn, tab); break;
-    default: edge_sums_loop<T, DPT>(v, nv, st, ct, X1, X2, useX, sr, si, mn, tab); break;
+    case 3: edge_sums_fixed<T, DPT, 3, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 4: edge_sums_fixed<T, DPT, 4, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 5: edge_sums_fixed<T, DPT, 5, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 6: edge_sums_fixed<T, DPT, 6, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    default: edge_sums_loop<T, DPT, kDrop>(v, nv, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
     }
 }
 
@@ -2107,74 +2117,196 @@ __global__ void __launch_bounds__(256) po_csca_kernel(const double *__restrict__
 // ------------------------------------------------------------ theta scan
 // Incoherent, azimuth-summed M11 on a list of zenith angles (reference
 // theta_m11_kernel, GpuDiffraction.cu:1909-1956, called by DiffractThetasGpu
-// :4780-4970).  Grid: x = zenith point, y = beam chunk; the CTA strides over
-// (beam, azimuth bin) pairs of its chunk and sums in a fixed-order tree, so
-// out_partial[chunk][t] is deterministic.
-__global__ void __launch_bounds__(256) po_thetas_kernel(
-    const DevBeam *beams, const DevVert *verts, const int32_t *beam_off, const double *weight,
-    int n_orient, int64_t n_beams, int beams_per_chunk, const double *st, const double *ct,
-    const double *sphi, const double *cphi, int n_az, int n_points, WaveConst wc,
-    double *out_partial)
+// :4780-4970).  Grid: x = (azimuth bin, tile of TPB * DPT zenith points),
+// y = beam chunk.  As in po_diffract_kernel the CTA folds its azimuth into
+// per-beam and per-vertex records in shared memory once and every thread
+// evaluates its points' edge sums from them; per pair only |s|^2 |R|^2 is
+// needed, and |P0 + cos t Pc + sin t Ps|^2 is a quadratic form in
+// (cos t, sin t) whose six coefficients are part of the record.  Small-phase
+// candidates are marked and evaluated in general form after the stage.
+// Bound by the FP64 pipe.  One thread per (point, beam, azimuth) with the
+// general evaluation took 1,225 us for 2,088 beams x 48 x 181 points, now
+// 266 us.
+struct __align__(16) ThetaBeam {
+    double a[6];        // A, B coefficients (see BeamRegs)
+    double q[6];        // |P0|^2 2P0.Pc 2P0.Ps |Pc|^2 |Ps|^2 2Pc.Ps, times 0.5 weight / (n_az + 1)
+    double slab[4];
+    double w;           // 0.5 weight / (n_az + 1)
+    int nv, vs;
+};
+constexpr int kThetaTpb = 64;
+constexpr int kThetaBeams = 64;                // beams and vertices of a stage
+constexpr int kThetaVerts = 4 * kThetaBeams;
+
+template <int DPT>
+__global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
+    KParams P, int64_t n_beams, int beams_per_chunk, int tiles, const double *st_tab, const double *ct_tab,
+    int n_points, double *out_partial)
 {
-    __shared__ double red[256];
-    const int t = blockIdx.x;
+    constexpr int TPB = kThetaTpb;
+    __shared__ ThetaBeam sb[kThetaBeams];
+    __shared__ SVertRaw<double> sv[kThetaVerts];
+    __shared__ double2 s_sincos[128];
+    for (int i = threadIdx.x; i < 128; i += TPB) {
+        double sn, cs;
+        sincos_turns(i * 0.0078125, sn, cs);
+        s_sincos[i] = make_double2(sn, cs);
+    }
+    const int p = blockIdx.x / tiles, tile = blockIdx.x - p * tiles;
+    const double cp = P.cphi[p], sp = P.sphi[p];
     const int64_t b0 = (int64_t)blockIdx.y * beams_per_chunk;
     const int64_t b1 = min(n_beams, b0 + beams_per_chunk);
-    const int64_t pairs = (b1 - b0) * n_az;
-    double acc = 0.0;
-    for (int64_t i = threadIdx.x; i < pairs; i += blockDim.x) {
-        const int64_t b = b0 + i / n_az;
-        const int p = (int)(i - (b - b0) * n_az);
-        // orientation of beam b: last o with beam_off[o] <= b
-        int lo = 0, hi = n_orient;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (beam_off[mid] <= b) lo = mid; else hi = mid;
-        }
-        DirFull dc;
-        dc.st = st[t];
-        dc.ct = ct[t];
-        dc.cp = cphi[p];
-        dc.sp = sphi[p];
-        dc.dir[0] = dc.st * dc.cp;
-        dc.dir[1] = dc.st * dc.sp;
-        dc.dir[2] = -dc.ct;
-        dc.vf[0] = -dc.sp; dc.vf[1] = dc.cp; dc.vf[2] = 0.0;
-        cross3(dc.vf, dc.dir, dc.u);
-        const double l2 = dc.u[0] * dc.u[0] + dc.u[1] * dc.u[1] + dc.u[2] * dc.u[2];
-        const double il = (l2 > 1e-30) ? rsqrt(l2) : 1.0;
-        dc.vt[0] = dc.u[0] * il; dc.vt[1] = dc.u[1] * il; dc.vt[2] = dc.u[2] * il;
-        cross3(dc.vt, dc.dir, dc.w);
-        double d[8];
-        if (beam_general(beams[b], verts, dc, wc, d, false)) {
-            double e = 0.0;
+    const int t0 = tile * TPB * DPT + threadIdx.x;
+    double st[DPT], ct[DPT], acc[DPT];
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                e = fma(d[q], d[q], e);
-            acc += 0.5 * e * weight[lo] / (double)(n_az + 1);
+    for (int d = 0; d < DPT; ++d) {
+        const int t = min(t0 + d * TPB, n_points - 1);
+        st[d] = st_tab[t];
+        ct[d] = ct_tab[t];
+        acc[d] = 0.0;
+    }
+    for (int64_t bs = b0; bs < b1;) {
+        // stage [bs, be): at most kThetaBeams beams and kThetaVerts vertices
+        const int vb0 = P.vbeg[bs];
+        int64_t be = min(b1, bs + kThetaBeams);
+        if (P.vbeg[be] - vb0 > kThetaVerts) {
+            int64_t lo = bs + 1, hi = be;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi + 1) >> 1;
+                if (P.vbeg[mid] - vb0 <= kThetaVerts) lo = mid; else hi = mid - 1;
+            }
+            be = lo;
         }
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-            red[threadIdx.x] += red[threadIdx.x + s];
+        const int nb = (int)(be - bs), nvs = P.vbeg[be] - vb0;
+        __syncthreads();   // the previous stage is consumed
+        for (int i = threadIdx.x; i < nb; i += TPB) {
+            const BrecRef r{P.brec + bs + i, P.brec_stride};
+            ThetaBeam &s = sb[i];
+            s.a[0] = -(cp * r.ab(0) + sp * r.ab(1)); s.a[1] = r.ab(2); s.a[2] = r.ab(3);
+            s.a[3] = -(cp * r.ab(4) + sp * r.ab(5)); s.a[4] = r.ab(6); s.a[5] = r.ab(7);
+            // orientation of the beam: last o with beam_off[o] <= b
+            int lo = 0, hi = P.n_orient;
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (P.beam_off[mid] <= bs + i) lo = mid; else hi = mid;
+            }
+            const double w = 0.5 * P.weight[lo] / (double)(P.n_az + 1);
+            double q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const double x = sp * r.Q(e) + cp * r.Q(8 + e);
+                const double y = -(cp * r.Q(16 + e) + sp * r.Q(24 + e));
+                const double z = r.Q(32 + e);
+                q[0] = fma(x, x, q[0]); q[1] = fma(2.0 * x, y, q[1]); q[2] = fma(2.0 * x, z, q[2]);
+                q[3] = fma(y, y, q[3]); q[4] = fma(z, z, q[4]); q[5] = fma(2.0 * y, z, q[5]);
+            }
+#pragma unroll
+            for (int e = 0; e < 6; ++e)
+                s.q[e] = w * q[e];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                s.slab[e] = r.slab(e);
+            s.w = w;
+            s.nv = r.nv();
+            s.vs = P.vbeg[bs + i] - vb0;
+        }
+        for (int i = threadIdx.x; i < nvs; i += TPB)
+            fill_vert(VrecRef{P.vrec + vb0 + i, P.vrec_stride}, cp, sp, sv[i]);
         __syncthreads();
+        uint64_t marked[DPT];
+#pragma unroll
+        for (int d = 0; d < DPT; ++d)
+            marked[d] = 0;
+        for (int j = 0; j < nb; ++j) {
+            const ThetaBeam &b = sb[j];
+            double X1[DPT], X2[DPT], sr[DPT], si[DPT], mn[DPT], m[DPT];
+            bool useX[DPT], cand[DPT];
+#pragma unroll
+            for (int d = 0; d < DPT; ++d) {
+                const double A = fma(st[d], b.a[0], fma(ct[d], b.a[1], b.a[2]));
+                const double B = fma(st[d], b.a[3], fma(ct[d], b.a[4], b.a[5]));
+                useX[d] = fabs(B) > fabs(A);
+                X1[d] = useX[d] ? B : A;
+                X2[d] = useX[d] ? A : B;
+                m[d] = X1[d];                       // |s|^2 takes 1 / X1^2
+                cand[d] = fabs(fma(A, b.slab[0], B * b.slab[1])) <= 1.0
+                       && fabs(fma(A, b.slab[2], B * b.slab[3])) <= 1.0;
+            }
+            edge_sums<double, DPT, true>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos, P.wc.eps1);
+#pragma unroll
+            for (int d = 0; d < DPT; ++d) {
+                const double q = fma(ct[d], fma(ct[d], b.q[3], b.q[1]),
+                                     fma(st[d], fma(st[d], b.q[4], fma(ct[d], b.q[5], b.q[2])), b.q[0]));
+                const double r = rcp64(m[d]);
+                const double xr = sr[d] * r, xi = si[d] * r;
+                const double e = fma(xr, xr, xi * xi) * q;
+                // a candidate's sums may be inf or NaN: select
+                acc[d] += cand[d] || isnan(e) ? 0.0 : e;
+                if (cand[d])
+                    marked[d] |= 1ull << j;
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < DPT; ++d) {
+            if (marked[d] == 0)
+                continue;
+            DirFull dc;
+            dc.st = st[d];
+            dc.ct = ct[d];
+            dc.cp = cp;
+            dc.sp = sp;
+            dc.dir[0] = dc.st * dc.cp;
+            dc.dir[1] = dc.st * dc.sp;
+            dc.dir[2] = -dc.ct;
+            dc.vf[0] = -dc.sp; dc.vf[1] = dc.cp; dc.vf[2] = 0.0;
+            cross3(dc.vf, dc.dir, dc.u);
+            const double l2 = dc.u[0] * dc.u[0] + dc.u[1] * dc.u[1] + dc.u[2] * dc.u[2];
+            const double il = (l2 > 1e-30) ? rsqrt(l2) : 1.0;
+            dc.vt[0] = dc.u[0] * il; dc.vt[1] = dc.u[1] * il; dc.vt[2] = dc.u[2] * il;
+            cross3(dc.vt, dc.dir, dc.w);
+            while (marked[d]) {
+                const int j = __ffsll((long long)marked[d]) - 1;
+                marked[d] &= marked[d] - 1;
+                double x[8];
+                if (beam_general(P.beams[bs + j], P.verts, dc, P.wc, x, false)) {
+                    double e = 0.0;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        e = fma(x[q], x[q], e);
+                    acc[d] = fma(e, sb[j].w, acc[d]);
+                }
+            }
+        }
+        bs = be;
     }
-    if (threadIdx.x == 0)
-        out_partial[(size_t)blockIdx.y * n_points + t] = red[0];
+    double *out = out_partial + ((size_t)blockIdx.y * P.n_az + p) * n_points;
+#pragma unroll
+    for (int d = 0; d < DPT; ++d)
+        if (t0 + d * TPB < n_points)
+            out[t0 + d * TPB] = acc[d];
 }
 
-// m11[t] = sum over chunks of partial[c][t], chunk order.
-__global__ void po_thetas_sum_kernel(const double *partial, int n_chunks, int n_points, double *m11)
+// m11[t] = sum over rows r of partial[r][t]: 32 points per CTA, the 32 warps
+// take rows in turn and their sums meet in warp order (deterministic).
+__global__ void __launch_bounds__(1024) po_thetas_sum_kernel(const double *partial, int64_t n_rows, int n_points,
+                                                            double *m11)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_points)
-        return;
+    __shared__ double red[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int c = 0; c < n_chunks; ++c)
-        s += partial[(size_t)c * n_points + t];
-    m11[t] = s;
+    if (t < n_points) {
+#pragma unroll 4
+        for (int64_t r = warp; r < n_rows; r += 32)
+            s += partial[r * n_points + t];
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && t < n_points) {
+        for (int w = 1; w < 32; ++w)
+            s += red[w][lane];
+        m11[t] = s;
+    }
 }
 
 // --------------------------------------------------------- extinction

@@ -138,3 +138,20 @@ def test_extinction_splits(n_orient, beams, phase_average):
     got = h.extinction(b)
     h.close()
     assert np.max(np.abs(got - want)) <= 1e-9 * np.max(np.abs(want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_points,n_az,n_orient,beams,nv", [
+    (1, 1, 1, 2, 0), (64, 3, 2, 63, 0), (65, 2, 3, 65, 0), (129, 5, 2, 40, 0), (200, 1, 40, 12, 0), (130, 2, 1, 20, 9)])
+def test_theta_scan_splits(n_points, n_az, n_orient, beams, nv):
+    """Zenith scan at the edges of its tiles (64 and 192 points), stages (64
+    beams, 256 vertices) and vertex-count cases, poles included.  Sums of
+    squares of the FP64 path's terms: its gate per point."""
+    b = _with_nv(beams, nv, 15.0, 3) if nv else S.ragged(n_orient, beams, 15.0, 9 + n_points)
+    g, w = S.grid(n_az, 2), S.wave()
+    th = np.deg2rad(np.linspace(0.0, 180.0, n_points)) if n_points > 1 else np.array([0.7])
+    want = oracle.thetas_m11(b, n_az, g.az_step, th, w)
+    h = GpuHandlerPO(g, w)
+    got = h.diffract_thetas_gpu(b, th)
+    h.close()
+    assert np.max(np.abs(got / want - 1.0)) < FP64_L2
