@@ -768,9 +768,21 @@ Variant shape_of(int pi, int variant, bool ns)
     return pi == 0 ? kVariantsF64[variant] : kVariantsF32[variant];
 }
 
+cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, int n_sets, bool add,
+                          double *out, cudaStream_t st)
+{
+    const dim3 g((unsigned)((G + 31) / 32), (unsigned)n_sets);
+    po_reduce_kernel<<<g, 256, 0, st>>>(partial, chunks_per_set, G, add, out);
+    return cudaGetLastError();
+}
+
+// How the chunk partials reach the caller: added into its accumulators,
+// stored there, or left in ctx->partial.
+enum class Sums { kAdd, kStore, kLeave };
+
 int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double *M_dev,
                  double *Mns_dev, cudaStream_t st, mbs_po_stats *stats, int variant = -1,
-                 int orient_limit = -1)
+                 int orient_limit = -1, Sums sums = Sums::kAdd)
 {
     if (!ctx->has_grid || !ctx->has_wave)
         return fail(ctx, MBS_PO_ESTATE, "grid and wave constants must be set first");
@@ -848,15 +860,13 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
     if (ctx->grid.n_pole > 0)
         CK(cudaStreamWaitEvent(st, ctx->ev[6], 0), "join side stream");
     CK(cudaEventRecord(ctx->ev[1], st), "event");
-    const int rb = 256;
-    const dim3 rg((unsigned)((G * 16 + rb - 1) / rb), (unsigned)n_sets);
-    po_reduce_kernel<<<rg, rb, 0, st>>>(ctx->partial, L.chunks_per_set, G, M_dev);
-    CK(cudaGetLastError(), "reduce launch");
-    ++launches;
-    if (ns) {
-        po_reduce_kernel<<<rg, rb, 0, st>>>(P.partial_ns, L.chunks_per_set, G, Mns_dev);
-        CK(cudaGetLastError(), "reduce launch");
+    if (sums != Sums::kLeave) {
+        CK(launch_reduce(ctx->partial, L.chunks_per_set, G, n_sets, sums == Sums::kAdd, M_dev, st), "reduce launch");
         ++launches;
+        if (ns) {
+            CK(launch_reduce(P.partial_ns, L.chunks_per_set, G, n_sets, sums == Sums::kAdd, Mns_dev, st), "reduce launch");
+            ++launches;
+        }
     }
     CK(cudaEventRecord(ctx->partial_done, st), "event");
     CK(cudaEventRecord(ctx->ev[2], st), "event");
@@ -1202,9 +1212,8 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
         return rc;
     const double td0 = host_ms();
     CK(cudaEventRecord(ctx->ev[4], st), "event");
-    CK(cudaMemsetAsync(ctx->macc, 0, n * (ns ? 2 : 1) * sizeof(double), st), "memset acc");
     rc = run_diffract(ctx, pre ? pre : &ctx->host_staged, precision, ctx->macc, ns ? ctx->macc + n : nullptr,
-                      st, stats);
+                      st, stats, -1, -1, Sums::kStore);
     if (rc)
         return rc;
     const double *dev_out = ctx->macc;
@@ -1529,23 +1538,18 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
     std::memset(rows_out, 0, sizeof(double) * nrow * nO);
     if (nO == 0 || beams->n_beams == 0)
         return MBS_PO_OK;
-    // orientation groups: one Mueller grid per orientation, at most 256 MiB
-    // of grids per group, from the context's pool (stream-ordered: a later
-    // call reuses the blocks without mapping new pages or synchronising)
+    // orientation groups: one Mueller grid per orientation (the chunk
+    // partials), at most 256 MiB of grids per group; the rows from the
+    // context's pool (stream-ordered: a later call reuses the blocks without
+    // mapping new pages or synchronising)
     const int group = (int)std::max<size_t>(
         1, std::min<size_t>(std::min<size_t>(nO, 16384), ((size_t)1 << 25) / plane));
-    double *grids = nullptr, *drows = nullptr;
+    double *drows = nullptr;
     cudaStream_t st = ctx->stream;
     {
-        cudaError_t e = cudaMallocFromPoolAsync((void **)&grids, plane * group * sizeof(double),
-                                                ctx->pool, st);
-        if (e == cudaSuccess)
-            e = cudaMallocFromPoolAsync((void **)&drows, nrow * group * sizeof(double), ctx->pool, st);
-        if (e != cudaSuccess) {
-            if (grids)
-                cudaFreeAsync(grids, st);
-            return fail(ctx, MBS_PO_ENOMEM, std::string("orientation grids: ") + cudaGetErrorString(e));
-        }
+        const cudaError_t e = cudaMallocFromPoolAsync((void **)&drows, nrow * group * sizeof(double), ctx->pool, st);
+        if (e != cudaSuccess)
+            return fail(ctx, MBS_PO_ENOMEM, std::string("orientation rows: ") + cudaGetErrorString(e));
     }
     std::vector<int64_t> boff, voff;
     for (int o0 = 0; o0 < nO && rc == 0; o0 += group) {
@@ -1583,16 +1587,13 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
         // every orientation its own output set
         ctx->host_staged.n_sets = n;
         ctx->host_staged.orient_per_set = 1;
-        cudaError_t e = cudaMemsetAsync(grids, 0, plane * n * sizeof(double), st);
-        if (e != cudaSuccess) {
-            rc = cuda_fail(ctx, e, "memset grids");
+        // one chunk per set: the partial planes are the orientations' grids
+        if ((rc = run_diffract(ctx, &ctx->host_staged, precision, nullptr, nullptr, st, nullptr, -1, -1,
+                               Sums::kLeave)))
             break;
-        }
-        if ((rc = run_diffract(ctx, &ctx->host_staged, precision, grids, nullptr, st, nullptr)))
-            break;
-        po_phi_average_kernel<<<dim3((unsigned)nT, (unsigned)n), 128, 0, st>>>(grids, nAz, nT,
-                                                                               ctx->grid.theta, drows);
-        e = cudaGetLastError();
+        po_phi_rows_kernel<<<dim3((unsigned)((nT + 31) / 32), (unsigned)n), 256, 0, st>>>(
+            ctx->partial, nAz, nT, ctx->grid.theta, drows);
+        cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(rows_out + nrow * o0, drows, nrow * n * sizeof(double),
                                 cudaMemcpyDeviceToHost, st);
@@ -1602,7 +1603,6 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
             rc = cuda_fail(ctx, e, "orientation rows");
     }
     ctx->host_staged.n_sets = 1;
-    cudaFreeAsync(grids, st);
     cudaFreeAsync(drows, st);
     return rc;
 }
@@ -1947,13 +1947,8 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
         return cuda_fail(ctx, e, "diffraction kernel launch");
     if (ctx->grid.n_pole > 0)
         CK(cudaStreamWaitEvent(st, ctx->ev[6], 0), "join side stream");
-    const int rb = 256;
-    const int rg = (int)((G * 16 + rb - 1) / rb);
-    po_reduce_kernel<<<rg, rb, 0, st>>>(P.partial, L.n_chunks, G, M_dev);
-    CK(cudaGetLastError(), "reduce launch");
-    if (ns) {
-        po_reduce_kernel<<<rg, rb, 0, st>>>(P.partial_ns, L.n_chunks, G, Mns_dev);
-        CK(cudaGetLastError(), "reduce launch");
-    }
+    CK(launch_reduce(P.partial, L.n_chunks, G, 1, true, M_dev, st), "reduce launch");
+    if (ns)
+        CK(launch_reduce(P.partial_ns, L.n_chunks, G, 1, true, Mns_dev, st), "reduce launch");
     return MBS_PO_OK;
 }

@@ -155,3 +155,29 @@ def test_theta_scan_splits(n_points, n_az, n_orient, beams, nv):
     got = h.diffract_thetas_gpu(b, th)
     h.close()
     assert np.max(np.abs(got / want - 1.0)) < FP64_L2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_az,n_zen,n_orient", [(1, 1, 1), (7, 31, 2), (9, 32, 3), (16, 70, 5)])
+def test_reduced_planes_and_rows(n_az, n_zen, n_orient):
+    """Plane sums by tiles of 32 directions and per-orientation rows by tiles
+    of 32 zenith rows: direction and row counts around the tiles; the staged
+    call adds to what the accumulator holds, the host call returns its sums."""
+    import torch
+    b = S.ragged(n_orient, 6, 10.0, n_az + n_zen)
+    g, w = S.grid(n_az, n_zen), S.wave()
+    h = GpuHandlerPO(g, w)
+    M = h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, precision=abi.FP64)
+    assert _l2(M, oracle.po_diffract(b, g, w)) < FP64_L2
+    acc = torch.full((M.size,), 2.0, dtype=torch.float64, device="cuda:0")
+    st = h.stage(b)
+    h.diffract_staged(st, acc.data_ptr(), precision=abi.FP64)
+    torch.cuda.synchronize()
+    np.testing.assert_allclose(acc.cpu().numpy(), M.ravel() + 2.0, rtol=1e-15, atol=0)
+    st.free()
+    rows = h.orientation_rows(b, precision=abi.FP64)
+    h.close()
+    for o in range(n_orient):
+        want = oracle.phi_average(oracle.po_diffract(b.select(o, 1), g, w), g)[0]
+        assert np.linalg.norm(rows[o] - want) <= FP64_L2 * np.linalg.norm(want)
