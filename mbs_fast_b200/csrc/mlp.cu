@@ -2,15 +2,24 @@
 //
 // 4 -> 128 -> 128 -> 128 -> 1 with erf GELU.  Every layer product runs on
 // the 5th-generation tensor cores as BF16 x BF16 -> FP32: tcgen05.mma
-// (M = 128, N <= 128, K = 16 per instruction) issued by one thread per CTA,
-// both operands in shared memory in the K-major no-swizzle layout (8 x 16-byte
-// core matrices), the accumulator in tensor memory, read back with
-// tcgen05.ld for the epilogue.  Operands are staged from global memory with
-// arbitrary strides, so the transposed operands of the backward pass need no
-// copies.  The 128 -> 1 head is a per-sample dot product in FP32.  Master parameters,
-// gradients and Adam moments are FP32; the BF16 weight copies are refreshed
-// after every update.  All reductions (bias gradients, loss) run in a fixed
-// order, so training is bitwise repeatable for a given seed.
+// (M = 128, K = 16 per instruction) issued by one thread per CTA, both
+// operands in shared memory in the K-major no-swizzle layout (8 x 16-byte
+// core matrices), the accumulator in tensor memory, read back with tcgen05.ld.
+//
+// A training step is two kernels.  k_chain takes 32 samples per CTA through
+// the whole forward and backward chain (activations stay in shared memory and
+// registers; one MMA chain per layer); k_update forms the weight gradients,
+// which sum over all samples, 16 columns per CTA, and applies Adam to them
+// in the epilogue.  Operands cross between the two as images of the shared-
+// memory tiles, so both kernels stage them with plain bulk copies.  The
+// 128 -> 1 head is a per-sample dot product in FP32.  Master parameters,
+// gradients and Adam moments are FP32.  All reductions run in a fixed order,
+// so training is bitwise repeatable for a given seed.
+//
+// The step's operations are small (59 MFLOP at 256 samples); what bounds it is
+// the chain of dependent passes.  As twenty launches (nine GEMMs and the
+// element-wise and reduction kernels between them) a step of 256 samples took
+// 134 us; now 21 us, of which the chain's kernel is 12.8 and the update's 7.7.
 #include "mbs_mlp.h"
 
 #include <cuda_bf16.h>
@@ -30,9 +39,6 @@ constexpr int kH = MBS_MLP_HIDDEN;   // 128
 constexpr int kIn = MBS_MLP_IN;      // 4
 constexpr int kInPad = 16;           // K of the first layer, padded for the MMA
 constexpr int kTile = 128;           // M of one tcgen05.mma tile (batch rows padded to it)
-constexpr int kTileN = 32;           // N of one CTA's tile: four CTAs share a 128-wide layer
-constexpr int kTileK = 128;          // K staged per round
-constexpr int kGemmSmem = 2 * kTile * kTileK * 2 + 1024;   // A, B tiles (BF16) + barrier
 
 // Flat parameter offsets (include/mbs_mlp.h)
 constexpr int oW1 = 0, ob1 = oW1 + kH * kIn, oW2 = ob1 + kH, ob2 = oW2 + kH * kH;
@@ -52,23 +58,6 @@ __device__ __forceinline__ float gelu_grad(float z)
     return 0.5f * (1.0f + erff(z * 0.70710678118654752f))
          + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
-
-// Logical matrix view: X[r][c] = p[r * sr + c * sc].
-struct Mat {
-    const bf16 *p;
-    long sr, sc;
-};
-
-enum { kModeFwd = 0, kModeBwd = 1, kModeF32 = 2 };
-
-struct GemmOut {
-    const float *bias;   // kModeFwd: [N]
-    const float *zin;    // kModeBwd: pre-activation of the layer below [M][ldo]
-    float *z;            // kModeFwd: pre-activation out
-    bf16 *h;             // kModeFwd: activation out; kModeBwd: gradient out
-    float *f;            // kModeF32: plain product out
-    int ldo;
-};
 
 // ---- tcgen05 helpers --------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
@@ -117,61 +106,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int limi
     return false;
 }
 
-// C[M][N] = A[M][K] B[K][N] with the epilogue of MODE.  M a multiple of 128,
-// N a multiple of 16 (at most 128 per CTA), K a multiple of 16.  Grid: x over
-// N tiles, y over M tiles; 128 threads, thread i owns accumulator row i
-// (tensor-memory lane i).  On a barrier timeout *err is set and the CTA
-// frees its tensor memory and returns without storing.
-// Stages the rows x kt operand tile whose element (r, k) is
-// p[(row0 + r) * rs + (k0 + k) * ks] into shared memory in the K-major core-
-// matrix layout (kmajor_off); rows at or beyond row_limit read as zero.
-// Operands contiguous along K move in 16-byte vectors (one core-matrix row
-// each); operands contiguous along the rows move in 16-byte vectors of 8 rows
-// at one k; anything else element by element.  Every path is unrolled so a
-// thread keeps several global loads in flight.
-__device__ __forceinline__ void stage_operand(unsigned char *dst, const bf16 *p, long rs, long ks,
-                                              int row0, int rows, int row_limit, int k0, int kt)
-{
-    const bool aligned = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
-    if (ks == 1 && (rs & 7) == 0 && aligned) {
-        const int kc = kt >> 3;
-        const int n = rows * kc;
-#pragma unroll 4
-        for (int v = threadIdx.x; v < n; v += blockDim.x) {
-            const int r = v / kc, c = v - r * kc;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (row0 + r < row_limit)
-                val = *reinterpret_cast<const uint4 *>(p + (long)(row0 + r) * rs + k0 + c * 8);
-            *reinterpret_cast<uint4 *>(dst + kmajor_off(r, c * 8, kt)) = val;
-        }
-    } else if (rs == 1 && (ks & 7) == 0 && aligned && (rows & 7) == 0 && (row0 & 7) == 0
-               && (row_limit & 7) == 0) {
-        const int rc = rows >> 3;
-        const int n = kt * rc;
-#pragma unroll 4
-        for (int v = threadIdx.x; v < n; v += blockDim.x) {
-            const int k = v / rc, r = (v - k * rc) * 8;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (row0 + r < row_limit)
-                val = *reinterpret_cast<const uint4 *>(p + (long)(row0 + r) + (long)(k0 + k) * ks);
-            const bf16 *e = reinterpret_cast<const bf16 *>(&val);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<bf16 *>(dst + kmajor_off(r + j, k, kt)) = e[j];
-        }
-    } else {
-        const bf16 zero = __float2bfloat16(0.f);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < rows * kt; i += blockDim.x) {
-            const int r = i / kt, k = i - r * kt;
-            *reinterpret_cast<bf16 *>(dst + kmajor_off(r, k, kt)) =
-                row0 + r < row_limit ? p[(long)(row0 + r) * rs + (long)(k0 + k) * ks] : zero;
-        }
-    }
-}
-
-constexpr int kGemmThreads = 256;   // 8 warps: all stage, two warpgroups read TMEM
-
 // Watchdog of the tensor-core barrier waits: the device error flag, the
 // poll limit, and (test hook) whether to leave out the MMAs and their
 // commit, so that the wait runs out with no asynchronous operation pending.
@@ -181,215 +115,592 @@ struct Watch {
     int skip_mma;
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm(int M, int N, int K, Mat A, Mat B, GemmOut o, Watch w)
+// ---- operand images ----------------------------------------------------
+// A K-major tile of R rows and 128 k in its shared-memory layout (kmajor_off
+// with kt = 128): 2,048 bytes per 8 rows.  Weights: the forward operand of
+// layer l holds (row = output, k = input), the backward one (row = input,
+// k = output).  Activations and gradients, transposed for the weight
+// gradients: one image per 128 samples, (row = column of the layer, k = sample).
+constexpr int kImg = kH * kTile;           // elements of a 128-row image
+constexpr int kImgX = kInPad * kTile;      // of the input's 16-row image
+struct Weights {
+    bf16 *w1f;          // (output, input) with kt = 16
+    bf16 *w2f, *w3f;    // forward
+    bf16 *w2b, *w3b;    // backward
+};
+struct Images {
+    bf16 *x0, *h1, *h2, *h3, *dz1, *dz2, *dz3;
+};
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
-    extern __shared__ __align__(1024) unsigned char gsm[];
-    bf16 *sA = reinterpret_cast<bf16 *>(gsm);
-    bf16 *sB = reinterpret_cast<bf16 *>(gsm + kTile * kTileK * 2);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(gsm + 2 * kTile * kTileK * 2);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
-    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTileN;
-    const int nt = min(kTileN, N - n0);                  // multiple of 16
-    const int ncols = nt <= 32 ? 32 : (nt <= 64 ? 64 : 128);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(1));
+}
+
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+}
+
+// kt / 16 MMAs over a staged tile pair (M = 128, N columns), then the commit;
+// one thread.
+__device__ __forceinline__ void mma_chain(uint32_t tmem, uint32_t a, uint32_t b, int kt, int N, bool accumulate,
+                                          uint32_t bar)
+{
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t idesc = umma_idesc(kTile, N), sbo = (uint32_t)kt * 16;
+    for (int s = 0; s < kt / 16; ++s) {
+        const uint64_t da = umma_desc(a + 256 * s, 128, sbo);
+        const uint64_t db = umma_desc(b + 256 * s, 128, sbo);
+        const uint32_t acc = (accumulate || s > 0) ? 1u : 0u;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "setp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc));
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                 :: "r"(bar) : "memory");
+}
+
+// 32 (or 8) accumulator columns of the warp's 32 tensor-memory lanes.
+__device__ __forceinline__ void tmem_ld32(uint32_t ta, uint32_t *v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                   "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+                   "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+                   "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                 : "r"(ta));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t *v)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(ta));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// ---- forward and backward chain of 32 samples ---------------------------
+constexpr int kRows = 32;            // samples per CTA
+constexpr int kChainThreads = 512;   // thread = (row, 8 consecutive columns)
+constexpr int kAccStride = kH + 4;   // floats: 16-byte rows without bank conflicts
+// shared memory: A tile (rows 32..127 zero), input tile, weight operands,
+// FP32 accumulator tile, small arrays
+constexpr int cA = 0, cX = cA + 2 * kImg, cW1 = cX + kTile * kInPad * 2, cW2f = cW1 + kH * kInPad * 2;
+constexpr int cW3f = cW2f + 2 * kImg, cS = cW3f + 2 * kImg, cVec = cS + kRows * kAccStride * 4;
+constexpr int cBar = cVec + (4 * kH + 3 * kRows) * 4, cFwdEnd = cBar + 64;
+constexpr int cW3b = (cFwdEnd + 127) / 128 * 128, cW2b = cW3b + 2 * kImg;
+constexpr int kChainSmemFwd = cFwdEnd, kChainSmem = cW2b + 2 * kImg;
+static_assert(kChainSmem <= 227 * 1024, "shared memory of one CTA");
+
+struct ChainArgs {
+    const float *q, *t;      // samples [..][4] and targets
+    const int *idx, *epoch;  // null, or the shuffled order [epoch][n_set] and the epoch counter
+    int n_set, b0;           // samples of the set, offset of this batch in the epoch
+    int n;                   // samples of this batch; the rows beyond are padding
+    const float *params;
+    Weights w;
+    Images img;              // training only
+    float *y, *dy;
+    Watch watch;
+};
+
+// The A tile's transpose (row = column of the layer, k = sample) into the
+// samples' 32 k of an image: thread = (column, 8 samples).
+__device__ __forceinline__ void store_image(const unsigned char *sA, bf16 *img, int r0)
+{
+    const int col = threadIdx.x & (kH - 1), rg = threadIdx.x >> 7;
+    const int k = (r0 & (kTile - 1)) + rg * 8;
+    __align__(16) bf16 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        v[i] = *reinterpret_cast<const bf16 *>(sA + kmajor_off(rg * 8 + i, col, kTile));
+    unsigned char *dst = reinterpret_cast<unsigned char *>(img + (size_t)(r0 / kTile) * kImg);
+    *reinterpret_cast<uint4 *>(dst + kmajor_off(col, k, kTile)) = *reinterpret_cast<const uint4 *>(v);
+}
+
+template <bool kTrain>
+__global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const uint32_t sbase = smem_u32(sm);
+    float *S = reinterpret_cast<float *>(sm + cS);
+    float *sb = reinterpret_cast<float *>(sm + cVec);      // b1, b2, b3, w4
+    float *sy = sb + 4 * kH, *st = sy + kRows, *sdy = st + kRows;
+    const uint32_t bars = sbase + cBar;                    // [0] MMA, [1] w1f, w2f, [2] w3f, [3] w3b, w2b
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + cBar + 48);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r0 = blockIdx.x * kRows;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(tslot)), "r"(ncols));
+                     :: "r"(smem_u32(tslot)), "r"(kH));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (threadIdx.x == 0)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(bar)), "r"(1));
+    if (tid == 0) {
+        for (int i = 0; i < 4; ++i)
+            mbar_init(bars + 8 * i);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect(bars + 8, kH * kInPad * 2 + 2 * kImg);
+        bulk_load(sbase + cW1, a.w.w1f, kH * kInPad * 2, bars + 8);
+        bulk_load(sbase + cW2f, a.w.w2f, 2 * kImg, bars + 8);
+        mbar_expect(bars + 16, 2 * kImg);
+        bulk_load(sbase + cW3f, a.w.w3f, 2 * kImg, bars + 16);
+        if (kTrain) {
+            mbar_expect(bars + 24, 4 * kImg);
+            bulk_load(sbase + cW3b, a.w.w3b, 2 * kImg, bars + 24);
+            bulk_load(sbase + cW2b, a.w.w2b, 2 * kImg, bars + 24);
+        }
+    }
+    // zero the tiles' rows beyond the samples and the input's padding columns
+    for (int i = tid; i < 2 * kImg / 16; i += kChainThreads)
+        reinterpret_cast<uint4 *>(sm + cA)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < kTile * kInPad * 2 / 16; i += kChainThreads)
+        reinterpret_cast<uint4 *>(sm + cX)[i] = make_uint4(0u, 0u, 0u, 0u);
+    sb[tid] = a.params[tid < kH ? ob1 + tid : tid < 2 * kH ? ob2 + tid - kH
+                       : tid < 3 * kH ? ob3 + tid - 2 * kH : ow4 + tid - 3 * kH];
+    __syncthreads();
+    if (tid < kRows) {
+        const int r = r0 + tid;
+        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
+        float tv = 0.f;
+        if (r < a.n) {
+            const int s = a.idx ? a.idx[(size_t)(*a.epoch) * a.n_set + a.b0 + r] : r;
+            qv = make_float4(a.q[s * kIn], a.q[s * kIn + 1], a.q[s * kIn + 2], a.q[s * kIn + 3]);
+            if (kTrain)
+                tv = a.t[s];
+        }
+        st[tid] = tv;
+        const bf16 v[4] = {__float2bfloat16(qv.x), __float2bfloat16(qv.y), __float2bfloat16(qv.z),
+                           __float2bfloat16(qv.w)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<bf16 *>(sm + cX + kmajor_off(tid, c, kInPad)) = v[c];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
-    const uint32_t idesc = umma_idesc(kTile, nt);
-    uint32_t phase = 0;
+    if (kTrain && tid < kInPad * (kRows / 8)) {   // the input's image: (column, 8 samples)
+        const int col = tid & (kInPad - 1), rg = tid / kInPad;
+        __align__(16) bf16 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = *reinterpret_cast<const bf16 *>(sm + cX + kmajor_off(rg * 8 + i, col, kInPad));
+        unsigned char *dst = reinterpret_cast<unsigned char *>(a.img.x0 + (size_t)(r0 / kTile) * kImgX);
+        *reinterpret_cast<uint4 *>(dst + kmajor_off(col, (r0 & (kTile - 1)) + rg * 8, kTile)) =
+            *reinterpret_cast<const uint4 *>(v);
+    }
     bool ok = true;
-    for (int k0 = 0; k0 < K && ok; k0 += kTileK) {
-        const int kt = min(kTileK, K - k0);              // multiple of 16
-        // stage A (kTile x kt: element (m, k) = A.p[m sr + k sc]) and B
-        // (nt x kt: element (n, k) = B.p[k sr + n sc]) in the K-major layout
-        stage_operand(reinterpret_cast<unsigned char *>(sA), A.p, A.sr, A.sc, m0, kTile, M, k0, kt);
-        stage_operand(reinterpret_cast<unsigned char *>(sB), B.p, B.sc, B.sr, n0, nt, n0 + nt, k0, kt);
+    uint32_t phase = 0;
+    int loaded = 0;            // weight barriers waited for so far
+    // One layer product on the staged A tile, its accumulators as FP32 rows
+    // in S.  `wbar`: the barrier of the weight operand.
+    auto layer = [&](int aoff, int boff, int kt, int wbar) {
+        if (tid == 0 && ok) {
+            while (loaded < wbar && ok) {
+                ++loaded;
+                ok = mbar_wait(bars + 8 * loaded, 0, kDefaultPollLimit);
+            }
+            if (ok && !a.watch.skip_mma)
+                mma_chain(tmem, sbase + aoff, sbase + boff, kt, kH, false, bars);
+        }
+        const bool done = mbar_wait(bars, phase, a.watch.poll_limit);
+        phase ^= 1u;
+        ok = __syncthreads_and(ok && done);
+        if (!ok)
+            return;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if ((warp & 3) == 0) {   // rows 0..31: the lane quarter of warps 0, 4, 8 and 12
+            uint32_t v[32];
+            const int c0 = (warp >> 2) * 32;
+            tmem_ld32(tmem + (uint32_t)c0, v);
+            float4 *dst = reinterpret_cast<float4 *>(S + lane * kAccStride + c0);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                     __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+    };
+    // this thread's 8 accumulators of S, and the next layer's operand
+    const int row = lane, c0 = warp * 8;
+    auto acc8 = [&](float *v) {
+        const float4 *p = reinterpret_cast<const float4 *>(S + row * kAccStride + c0);
+        const float4 x = p[0], y = p[1];
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    };
+    auto put8 = [&](const float *v) {
+        __align__(16) bf16 h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            h[i] = __float2bfloat16(v[i]);
+        *reinterpret_cast<uint4 *>(sm + cA + kmajor_off(row, c0, kTile)) = *reinterpret_cast<const uint4 *>(h);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (threadIdx.x == 0 && !w.skip_mma) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sbo = (uint32_t)kt * 16;
-            for (int s = 0; s < kt / 16; ++s) {
-                const uint64_t da = umma_desc(a0 + 256 * s, 128, sbo);
-                const uint64_t db = umma_desc(b0 + 256 * s, 128, sbo);
-                const uint32_t acc = (k0 > 0 || s > 0) ? 1u : 0u;
-                asm volatile("{\n\t.reg .pred p;\n\t"
-                             "setp.ne.b32 p, %4, 0;\n\t"
-                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                             :: "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         :: "r"(smem_u32(bar)) : "memory");
+    };
+    float z1[8], z2[8], z3[8], v[8];
+    auto forward = [&](float *z, int layer_no) {
+        acc8(v);
+        float h[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            z[i] = v[i] + sb[layer_no * kH + c0 + i];
+            h[i] = gelu(z[i]);
         }
-        // the tiles may be overwritten once the MMAs that read them are done
-        ok = mbar_wait(smem_u32(bar), phase, w.poll_limit);
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;");
+        put8(h);
+    };
+    layer(cX, cW1, kInPad, 1);
+    if (ok) {
+        forward(z1, 0);
+        if (kTrain)
+            store_image(sm + cA, a.img.h1, r0);
+        layer(cA, cW2f, kH, 1);
+    }
+    if (ok) {
+        forward(z2, 1);
+        if (kTrain)
+            store_image(sm + cA, a.img.h2, r0);
+        layer(cA, cW3f, kH, 2);
+    }
+    if (ok) {
+        forward(z3, 2);
+        if (kTrain)
+            store_image(sm + cA, a.img.h3, r0);
+        // y = sum_j H3[j] w4[j] + b4: a warp per sample, fixed lane order
+        const float b4 = a.params[ob4];
+        for (int r = warp; r < kRows; r += kChainThreads / 32) {
+            float s = 0.f;
+            for (int j = lane; j < kH; j += 32)
+                s = fmaf(__bfloat162float(*reinterpret_cast<const bf16 *>(sm + cA + kmajor_off(r, j, kTile))),
+                         sb[3 * kH + j], s);
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1)
+                s += __shfl_xor_sync(0xffffffffu, s, w);
+            if (lane == 0) {
+                const float yv = s + b4;
+                sy[r] = yv;
+                if (r0 + r < a.n)
+                    a.y[r0 + r] = yv;
+                // dy = 2 (y - t) / n (0 on padding rows)
+                const float d = r0 + r < a.n ? 2.f * (yv - st[r]) / (float)a.n : 0.f;
+                sdy[r] = d;
+                if (kTrain)
+                    a.dy[r0 + r] = d;
+            }
+        }
         __syncthreads();
     }
-    if (!ok) {
-        if (threadIdx.x == 0)
-            atomicExch(w.err, 1);
-        mbar_wait(smem_u32(bar), phase ^ 1u, w.poll_limit);   // let any MMA in flight finish, bounded
-    } else {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its lane quarter); the
-        // two warpgroups take alternate 16-column chunks
-        const int wq = warp & 3, wg = warp >> 2;
-        const int r = m0 + wq * 32 + lane;
-        for (int c0 = wg * 16; c0 < nt; c0 += 32) {
-            uint32_t v[16];
-            const uint32_t ta = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)c0;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                           "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                           "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                         : "r"(ta));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (r < M) {
+    if (kTrain && ok) {
+        // dZ3 = dy w4 gelu'(Z3), dZ2 = (dZ3 W3) gelu'(Z2), dZ1 = (dZ2 W2) gelu'(Z1)
+        const float d = sdy[row];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int c = n0 + c0 + i;
-                    const long idx = (long)r * o.ldo + c;
-                    const float val = __uint_as_float(v[i]);
-                    if (MODE == kModeFwd) {
-                        const float z = val + o.bias[c];
-                        o.z[idx] = z;
-                        o.h[idx] = __float2bfloat16(gelu(z));
-                    } else if (MODE == kModeBwd) {
-                        o.h[idx] = __float2bfloat16(val * gelu_grad(o.zin[idx]));
-                    } else {
-                        o.f[idx] = val;
-                    }
+        for (int i = 0; i < 8; ++i)
+            v[i] = d * sb[3 * kH + c0 + i] * gelu_grad(z3[i]);
+        put8(v);
+        store_image(sm + cA, a.img.dz3, r0);
+        layer(cA, cW3b, kH, 3);
+        if (ok) {
+            acc8(v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = v[i] * gelu_grad(z2[i]);
+            put8(v);
+            store_image(sm + cA, a.img.dz2, r0);
+            layer(cA, cW2b, kH, 3);
+        }
+        if (ok) {
+            acc8(v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = v[i] * gelu_grad(z1[i]);
+            put8(v);
+            store_image(sm + cA, a.img.dz1, r0);
+        }
+    }
+    if (!ok && tid == 0) {
+        atomicExch(a.watch.err, 1);
+        mbar_wait(bars, phase ^ 1u, a.watch.poll_limit);   // any MMA in flight, bounded
+        for (int i = loaded + 1; i <= (kTrain ? 3 : 2); ++i)
+            mbar_wait(bars + 8 * i, 0, kDefaultPollLimit);  // copies in flight, bounded
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kH));
+}
+
+// ---- weight gradients and Adam -------------------------------------------
+struct UpdateArgs {
+    Images img;
+    const float *dy;
+    int bp;                  // padded samples (a multiple of 128)
+    float *grad;             // plain gradients out (null: Adam)
+    float *p, *m, *v;        // parameters and Adam moments
+    float lr;
+    const float *bc;         // bias corrections of step j at [2 j], [2 j + 1]
+    const int *epoch;
+    int steps_per_epoch, k;  // this step: epoch * steps_per_epoch + k
+    Weights w;
+    Watch watch;
+};
+
+// Adam on N consecutive parameters (N = 4 or 8: vector loads, all issued
+// before the first store) with the step's bias corrections; p receives the
+// updated parameters.
+template <int N>
+__device__ __forceinline__ void adam(const UpdateArgs &a, int i, const float *g, float bc1, float bc2, float *p)
+{
+    __align__(16) float m[N], v[N];
+    if (N % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+            *reinterpret_cast<float4 *>(m + k) = *reinterpret_cast<const float4 *>(a.m + i + k);
+            *reinterpret_cast<float4 *>(v + k) = *reinterpret_cast<const float4 *>(a.v + i + k);
+            *reinterpret_cast<float4 *>(p + k) = *reinterpret_cast<const float4 *>(a.p + i + k);
+        }
+    } else {
+        m[0] = a.m[i];
+        v[0] = a.v[i];
+        p[0] = a.p[i];
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float gi = g[k];
+        const float mi = 0.9f * m[k] + 0.1f * gi;
+        const float vi = 0.999f * v[k] + 0.001f * gi * gi;
+        m[k] = mi;
+        v[k] = vi;
+        p[k] = p[k] - a.lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
+    }
+    if (N % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+            *reinterpret_cast<float4 *>(a.m + i + k) = *reinterpret_cast<const float4 *>(m + k);
+            *reinterpret_cast<float4 *>(a.v + i + k) = *reinterpret_cast<const float4 *>(v + k);
+            *reinterpret_cast<float4 *>(a.p + i + k) = *reinterpret_cast<const float4 *>(p + k);
+        }
+    } else {
+        a.m[i] = m[0];
+        a.v[i] = v[0];
+        a.p[i] = p[0];
+    }
+}
+
+// CTAs: 8 of 16 columns each for dW3 = dZ3^T H2 and dW2 = dZ2^T H1, one for
+// dW1 = dZ1^T X0, then the vectors, 32 entries a CTA: db3, db2, db1 (column
+// sums of dZ) and the head's dw4, db4.  Both operands of a product are
+// contiguous pieces of the images, copied 128 samples at a time into two
+// stages; thread 0 copies and issues the MMAs.
+constexpr int kUpThreads = 256;
+constexpr int kUpN = 16;
+constexpr int kUpStage = 2 * kImg + kUpN * kTile * 2;
+constexpr int kUpSmem = 2 * kUpStage + 64;
+constexpr int kJobsW = kH / kUpN, kJobW1 = 2 * kJobsW, kJobBias = kJobW1 + 1, kJobHead = kJobBias + 3 * (kH / 32);
+constexpr int kUpJobs = kJobHead + kH / 32 + 1;
+
+__device__ __forceinline__ float image_at(const bf16 *img, int c, int row)
+{
+    return __bfloat162float(*reinterpret_cast<const bf16 *>(
+        reinterpret_cast<const unsigned char *>(img + (size_t)(row / kTile) * kImg)
+        + kmajor_off(c, row & (kTile - 1), kTile)));
+}
+
+template <bool kAdam>
+__global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ float part[8][32];
+    __shared__ int s_ok;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int job = blockIdx.x;
+    float bc1 = 0.f, bc2 = 0.f;
+    if (kAdam) {
+        const int j = (*a.epoch) * a.steps_per_epoch + a.k;
+        bc1 = a.bc[2 * j];
+        bc2 = a.bc[2 * j + 1];
+    }
+    if (job >= kJobBias) {
+        // vectors: 8 row groups g take rows g, g + 8, ... in turn, the group
+        // sums are added in group order
+        const int g = warp;
+        float s = 0.f;
+        int idx = -1;
+        if (job < kJobHead) {
+            const int l = (job - kJobBias) / (kH / 32), c = (job - kJobBias) % (kH / 32) * 32 + lane;
+            const bf16 *x = l == 0 ? a.img.dz3 : l == 1 ? a.img.dz2 : a.img.dz1;
+            idx = (l == 0 ? ob3 : l == 1 ? ob2 : ob1) + c;
+#pragma unroll 8
+            for (int r = g; r < a.bp; r += 8)
+                s += image_at(x, c, r);
+        } else {
+            const int j = (job - kJobHead) * 32 + lane;
+            if (j <= kH) {
+                idx = j < kH ? ow4 + j : ob4;
+#pragma unroll 8
+                for (int b = g; b < a.bp; b += 8)
+                    s += j < kH ? a.dy[b] * image_at(a.img.h3, j, b) : a.dy[b];
+            }
+        }
+        part[g][lane] = s;
+        __syncthreads();
+        if (g == 0 && idx >= 0) {
+            float t = part[0][lane];
+            for (int k = 1; k < 8; ++k)
+                t += part[k][lane];
+            float p[1];
+            if (kAdam)
+                adam<1>(a, idx, &t, bc1, bc2, p);
+            else
+                a.grad[idx] = t;
+        }
+        return;
+    }
+    const int l = job < kJobsW ? 3 : job < kJobW1 ? 2 : 1;
+    const int n0 = l == 1 ? 0 : (job % kJobsW) * kUpN;
+    const bf16 *A = l == 3 ? a.img.dz3 : l == 2 ? a.img.dz2 : a.img.dz1;
+    const bf16 *B = l == 3 ? a.img.h2 : l == 2 ? a.img.h1 : a.img.x0;
+    const size_t bstep = l == 1 ? kImgX : kImg;
+    B += n0 * kTile;         // 8 rows of an image are 8 * 128 consecutive elements
+    const uint32_t sbase = smem_u32(sm), bars = sbase + 2 * kUpStage;   // full[2], MMA[2]
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + 2 * kUpStage + 48);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     :: "r"(smem_u32(tslot)), "r"(32));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int i = 0; i < 4; ++i)
+            mbar_init(bars + 8 * i);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = *tslot;
+    if (tid == 0) {
+        const int nblk = a.bp / kTile;
+        int issued = 0, waited = 0, committed = 0;
+        auto load = [&]() {
+            const uint32_t d = sbase + (issued & 1) * kUpStage, bar = bars + 8 * (issued & 1);
+            mbar_expect(bar, kUpStage);
+            bulk_load(d, A + (size_t)issued * kImg, 2 * kImg, bar);
+            bulk_load(d + 2 * kImg, B + (size_t)issued * bstep, kUpN * kTile * 2, bar);
+            ++issued;
+        };
+        load();
+        if (nblk > 1)
+            load();
+        bool ok = true;
+        for (int i = 0; i < nblk && ok; ++i) {
+            ok = mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, kDefaultPollLimit);
+            waited = i + 1;
+            if (!ok)
+                break;
+            if (!a.watch.skip_mma) {
+                const uint32_t d = sbase + (i & 1) * kUpStage;
+                mma_chain(tmem, d, d + 2 * kImg, kTile, kUpN, i > 0, bars + 16 + 8 * (i & 1));
+                committed = i + 1;
+            }
+            if (issued < nblk) {   // the stage is free once its MMAs are done
+                ok = mbar_wait(bars + 16 + 8 * (i & 1), (i >> 1) & 1, a.watch.poll_limit);
+                if (ok)
+                    load();
+            }
+        }
+        if (ok)
+            ok = mbar_wait(bars + 16 + 8 * ((nblk - 1) & 1), ((nblk - 1) >> 1) & 1, a.watch.poll_limit);
+        if (!ok) {
+            atomicExch(a.watch.err, 1);
+            for (int i = waited; i < issued; ++i)       // copies in flight, bounded
+                mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, kDefaultPollLimit);
+            if (committed > 0)                          // and MMAs
+                mbar_wait(bars + 16 + 8 * ((committed - 1) & 1), ((committed - 1) >> 1) & 1, a.watch.poll_limit);
+        }
+        s_ok = ok;
+    }
+    __syncthreads();
+    if (s_ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        // warp w: accumulator rows 32 (w % 4) .. + 31 (its lane quarter),
+        // columns 8 (w / 4) .. + 7
+        const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 8;
+        uint32_t u[8];
+        tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cl, u);
+        __align__(16) float gv[8], pv[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            gv[i] = __uint_as_float(u[i]);
+        if (l == 1) {
+            if (cl == 0) {
+                const int i0 = oW1 + r * kIn;
+                if (kAdam) {
+                    adam<kIn>(a, i0, gv, bc1, bc2, pv);
+#pragma unroll
+                    for (int c = 0; c < kIn; ++c)
+                        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(a.w.w1f)
+                                                  + kmajor_off(r, c, kInPad)) = __float2bfloat16(pv[c]);
+                } else {
+                    *reinterpret_cast<float4 *>(a.grad + i0) = *reinterpret_cast<const float4 *>(gv);
                 }
+            }
+        } else {
+            const int c = n0 + cl, i0 = (l == 3 ? oW3 : oW2) + r * kH + c;
+            if (kAdam) {
+                unsigned char *wf = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3f : a.w.w2f);
+                unsigned char *wb = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3b : a.w.w2b);
+                __align__(16) bf16 h[8];
+                adam<8>(a, i0, gv, bc1, bc2, pv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    h[i] = __float2bfloat16(pv[i]);
+                *reinterpret_cast<uint4 *>(wf + kmajor_off(r, c, kTile)) = *reinterpret_cast<const uint4 *>(h);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    *reinterpret_cast<bf16 *>(wb + kmajor_off(c + i, r, kTile)) = h[i];
+            } else {
+                float4 *dst = reinterpret_cast<float4 *>(a.grad + i0);
+                dst[0] = *reinterpret_cast<const float4 *>(gv);
+                dst[1] = *reinterpret_cast<const float4 *>(gv + 4);
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(32));
 }
 
-// X0[b][0..15] (BF16): the quaternion in columns 0..3, zeros elsewhere and
-// on padding rows.
-__global__ void k_input(const float *q, int n, int bpad, bf16 *x0)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bpad * kInPad)
-        return;
-    const int b = i / kInPad, c = i - b * kInPad;
-    x0[i] = __float2bfloat16((b < n && c < kIn) ? q[b * kIn + c] : 0.f);
-}
-
-// y[b] = sum_j H3[b][j] w4[j] + b4: one warp per sample, fixed lane order.
-__global__ void k_head_fwd(const bf16 *h3, const float *params, int n, float *y)
-{
-    const int b = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (b >= n)
-        return;
-    float s = 0.f;
-    for (int j = lane; j < kH; j += 32)
-        s = fmaf(__bfloat162float(h3[(long)b * kH + j]), params[ow4 + j], s);
-#pragma unroll
-    for (int w = 16; w > 0; w >>= 1)
-        s += __shfl_xor_sync(0xffffffffu, s, w);
-    if (lane == 0)
-        y[b] = s + params[ob4];
-}
-
-// dy[b] = 2 (y_b - t_b) / n (0 on padding rows);
-// dZ3[b][j] = dy_b w4[j] gelu'(Z3[b][j]).
-__global__ void k_head_bwd(const float *y, const float *t, int n, int bpad, const float *params,
-                           const float *z3, float *dy, bf16 *dz3)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bpad * kH)
-        return;
-    const int b = i / kH, j = i - b * kH;
-    const float d = b < n ? 2.f * (y[b] - t[b]) / (float)n : 0.f;
-    if (j == 0)
-        dy[b] = d;
-    dz3[i] = __float2bfloat16(d * params[ow4 + j] * gelu_grad(z3[i]));
-}
-
-// Column sums of a [rows][cols] BF16 matrix, fixed row order: out[c].
-// Column sums in fixed order: block b sums columns 32 b .. 32 b + 31, its 8
-// row groups g (threadIdx.x / 32) take rows g, g + 8, ... in turn, and the
-// group sums are added in group order.  Launch with 256 threads and
-// ceil(cols / 32) blocks.
-__global__ void __launch_bounds__(256) k_colsum_bf16(const bf16 *x, int rows, int cols, float *out)
-{
-    __shared__ float part[8][32];
-    const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int c = blockIdx.x * 32 + cl;
-    float s = 0.f;
-    if (c < cols)
-        for (int r = g; r < rows; r += 8)
-            s += __bfloat162float(x[(long)r * cols + c]);
-    part[g][cl] = s;
-    __syncthreads();
-    if (g == 0 && c < cols) {
-        float t = part[0][cl];
-        for (int k = 1; k < 8; ++k)
-            t += part[k][cl];
-        out[c] = t;
-    }
-}
-
-// Head gradients: gw4[j] = sum_b dy_b H3[b][j] (j < 128), gb4 = sum_b dy_b.
-// (fixed order as k_colsum_bf16: block b covers outputs j = 32 b .. 32 b + 31,
-// output kH is gb4; launch with 256 threads and kH / 32 + 1 blocks)
-__global__ void __launch_bounds__(256) k_head_grad(const float *dy, const bf16 *h3, int bpad, float *grad)
-{
-    __shared__ float part[8][32];
-    const int jl = threadIdx.x & 31, g = threadIdx.x >> 5;
-    const int j = blockIdx.x * 32 + jl;
-    float s = 0.f;
-    if (j <= kH)
-        for (int b = g; b < bpad; b += 8)
-            s += j < kH ? dy[b] * __bfloat162float(h3[(long)b * kH + j]) : dy[b];
-    part[g][jl] = s;
-    __syncthreads();
-    if (g == 0 && j <= kH) {
-        float t = part[0][jl];
-        for (int k = 1; k < 8; ++k)
-            t += part[k][jl];
-        grad[j < kH ? ow4 + j : ob4] = t;
-    }
-}
-
-// W1 gradient: the first kIn columns of the padded [128][16] product.
-__global__ void k_pack_w1_grad(const float *gw1p, float *grad)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kH * kIn)
-        return;
-    const int r = i / kIn, c = i - r * kIn;
-    grad[oW1 + i] = gw1p[r * kInPad + c];
-}
-
-// BF16 copies of the weights (W1 padded to [128][16]).
-__global__ void k_refresh(const float *params, bf16 *w1p, bf16 *w2, bf16 *w3)
+// Weight operand images of the master parameters (W1's padding columns zero).
+__global__ void k_refresh(const float *params, Weights w)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kH * kInPad) {
         const int r = i / kInPad, c = i - r * kInPad;
-        w1p[i] = __float2bfloat16(c < kIn ? params[oW1 + r * kIn + c] : 0.f);
+        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(w.w1f) + kmajor_off(r, c, kInPad)) =
+            __float2bfloat16(c < kIn ? params[oW1 + r * kIn + c] : 0.f);
     }
     if (i < kH * kH) {
-        w2[i] = __float2bfloat16(params[oW2 + i]);
-        w3[i] = __float2bfloat16(params[oW3 + i]);
+        const int r = i / kH, c = i - r * kH;
+        const bf16 v2 = __float2bfloat16(params[oW2 + i]), v3 = __float2bfloat16(params[oW3 + i]);
+        const uint32_t f = kmajor_off(r, c, kTile), b = kmajor_off(c, r, kTile);
+        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(w.w2f) + f) = v2;
+        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(w.w3f) + f) = v3;
+        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(w.w2b) + b) = v2;
+        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(w.w3b) + b) = v3;
     }
 }
 
@@ -413,60 +724,6 @@ __global__ void __launch_bounds__(256) k_loss(const float *y, const float *t, in
         *out = red[0] / (float)max(n, 1);
 }
 
-// The training step's minibatch at offset b0 of the epoch the device counter
-// holds (so one captured epoch replays over every epoch's shuffled order):
-// t_b[i] = t[s], X0[i] = the BF16 quaternion of s padded to kInPad columns,
-// s = idx[epoch n + b0 + i]; rows n_b .. bpad-1 of X0 are zeros (k_input's
-// layout, without the FP32 copy of the quaternions).
-__global__ void k_gather_input(const float *q, const float *t, const int *idx, const int *epoch,
-                               int n, int b0, int nb, int bpad, bf16 *x0, float *tb)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bpad)
-        return;
-    if (i < nb) {
-        const int s = idx[(size_t)(*epoch) * n + b0 + i];
-#pragma unroll
-        for (int c = 0; c < kInPad; ++c)
-            x0[i * kInPad + c] = __float2bfloat16(c < kIn ? q[s * kIn + c] : 0.f);
-        tb[i] = t[s];
-    } else {
-#pragma unroll
-        for (int c = 0; c < kInPad; ++c)
-            x0[i * kInPad + c] = __float2bfloat16(0.f);
-    }
-}
-
-// Adam with the bias corrections of step epoch * steps_per_epoch + k (bc[2 j],
-// bc[2 j + 1] for the call's j-th step), and the BF16 copies of the updated
-// weights (k_refresh's layout; W1's padding columns stay the zeros that
-// k_refresh wrote).
-__global__ void k_adam_refresh(float *p, const float *g, float *m, float *v, int n, float lr,
-                               const float *bc, const int *epoch, int steps_per_epoch, int k,
-                               bf16 *w1p, bf16 *w2, bf16 *w3)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const int j = (*epoch) * steps_per_epoch + k;
-    const float bc1 = bc[2 * j], bc2 = bc[2 * j + 1];
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
-    p[i] = pi;
-    if (i < ob1) {
-        const int r = (i - oW1) / kIn, c = (i - oW1) - r * kIn;
-        w1p[r * kInPad + c] = __float2bfloat16(pi);
-    } else if (i >= oW2 && i < ob2) {
-        w2[i - oW2] = __float2bfloat16(pi);
-    } else if (i >= oW3 && i < ob3) {
-        w3[i - oW3] = __float2bfloat16(pi);
-    }
-}
-
 // End of a captured epoch: the epoch counter moves on.
 __global__ void k_next_epoch(int *epoch)
 {
@@ -484,15 +741,15 @@ struct mbs_mlp {
     cudaStream_t stream = nullptr;
     std::string err;
     float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
-    bf16 *w1p = nullptr, *w2 = nullptr, *w3 = nullptr;
+    bf16 *wimg = nullptr;                 // weight operand images
+    Weights w{};
     int step = 0;
-    // activations for up to `cap` padded rows
-    int cap = 0;
-    bf16 *x0 = nullptr, *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;
-    bf16 *dz1 = nullptr, *dz2 = nullptr, *dz3 = nullptr;
-    float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr;
+    // samples for up to `cap` padded rows, activation images for `icap`
+    int cap = 0, icap = 0;
+    bf16 *acts = nullptr;
+    Images img{};
     float *y = nullptr, *t = nullptr, *dy = nullptr, *q = nullptr;
-    float *gw1p = nullptr, *scalar = nullptr;
+    float *scalar = nullptr;
     int poll_limit = kDefaultPollLimit;   // mbs_mlp_set_watchdog
     int skip_mma = 0;
 };
@@ -515,12 +772,10 @@ int mfail(mbs_mlp *net, int code, const std::string &msg)
 
 void free_acts(mbs_mlp *net)
 {
-    void *ps[] = {net->x0, net->h1, net->h2, net->h3, net->dz1, net->dz2, net->dz3, net->z1,
-                  net->z2, net->z3, net->y, net->t, net->dy, net->q};
+    void *ps[] = {net->y, net->t, net->dy, net->q};
     for (void *p : ps)
         cudaFree(p);
-    net->x0 = net->h1 = net->h2 = net->h3 = net->dz1 = net->dz2 = net->dz3 = nullptr;
-    net->z1 = net->z2 = net->z3 = net->y = net->t = net->dy = net->q = nullptr;
+    net->y = net->t = net->dy = net->q = nullptr;
     net->cap = 0;
 }
 
@@ -530,17 +785,6 @@ int ensure_acts(mbs_mlp *net, int rows)
     if (need <= net->cap)
         return 0;
     free_acts(net);
-    const size_t hb = (size_t)need * kH;
-    MK(cudaMalloc((void **)&net->x0, (size_t)need * kInPad * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->h1, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->h2, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->h3, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->dz1, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->dz2, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->dz3, hb * sizeof(bf16)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->z1, hb * sizeof(float)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->z2, hb * sizeof(float)), "cudaMalloc mlp");
-    MK(cudaMalloc((void **)&net->z3, hb * sizeof(float)), "cudaMalloc mlp");
     MK(cudaMalloc((void **)&net->y, need * sizeof(float)), "cudaMalloc mlp");
     MK(cudaMalloc((void **)&net->t, need * sizeof(float)), "cudaMalloc mlp");
     MK(cudaMalloc((void **)&net->dy, need * sizeof(float)), "cudaMalloc mlp");
@@ -549,7 +793,28 @@ int ensure_acts(mbs_mlp *net, int rows)
     return 0;
 }
 
-dim3 tiles(int M, int N) { return dim3((N + kTileN - 1) / kTileN, (M + kTile - 1) / kTile); }
+// Activation and gradient images of a batch of `rows` samples.
+int ensure_images(mbs_mlp *net, int rows)
+{
+    const int need = pad_rows(std::max(rows, 1));
+    if (need <= net->icap)
+        return 0;
+    cudaFree(net->acts);
+    net->acts = nullptr;
+    net->icap = 0;
+    const size_t one = (size_t)need * kH;
+    MK(cudaMalloc((void **)&net->acts, (6 * one + (size_t)need * kInPad) * sizeof(bf16)), "cudaMalloc mlp");
+    Images &g = net->img;
+    g.h1 = net->acts;
+    g.h2 = g.h1 + one;
+    g.h3 = g.h2 + one;
+    g.dz1 = g.h3 + one;
+    g.dz2 = g.dz1 + one;
+    g.dz3 = g.dz2 + one;
+    g.x0 = g.dz3 + one;
+    net->icap = need;
+    return 0;
+}
 
 // Device flag set by a GEMM whose tensor-core barrier wait ran out (the
 // third int of the network's scalar scratch).
@@ -569,88 +834,70 @@ int check_err(mbs_mlp *net)
     return 0;
 }
 
-// The GEMM kernels' dynamic shared-memory limit, set once per process
-// (before any graph capture: the training epoch is captured).
-void gemm_attrs()
+// The kernels' dynamic shared-memory limits on this network's device (set
+// before any graph capture: the training epoch is captured).
+int set_attrs(mbs_mlp *net)
 {
-    static bool done = false;
-    if (!done) {
-        cudaFuncSetAttribute(k_gemm<kModeFwd>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-        cudaFuncSetAttribute(k_gemm<kModeBwd>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-        cudaFuncSetAttribute(k_gemm<kModeF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-        done = true;
-    }
+    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    MK(cudaFuncSetAttribute(k_chain<false>, a, kChainSmemFwd), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_chain<true>, a, kChainSmem), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_update<false>, a, kUpSmem), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_update<true>, a, kUpSmem), "kernel attributes");
+    return 0;
 }
 
-template <int MODE>
-void gemm(cudaStream_t s, int M, int N, int K, Mat A, Mat B, GemmOut o, Watch w)
+ChainArgs chain_args(mbs_mlp *net, int n)
 {
-    gemm_attrs();
-    k_gemm<MODE><<<tiles(M, N), kGemmThreads, kGemmSmem, s>>>(M, N, K, A, B, o, w);
+    ChainArgs a{};
+    a.q = net->q;
+    a.t = net->t;
+    a.n = n;
+    a.n_set = n;
+    a.params = net->params;
+    a.w = net->w;
+    a.img = net->img;
+    a.y = net->y;
+    a.dy = net->dy;
+    a.watch = watch(net);
+    return a;
 }
 
-// Forward pass of n samples already in net->q (device); train keeps the
-// pre-activations for the backward pass.
-int forward_dev(mbs_mlp *net, int n, bool x0_ready = false)
+// Forward pass of n samples already in net->q (device).
+int forward_dev(mbs_mlp *net, int n)
 {
-    const int bp = pad_rows(n);
-    cudaStream_t s = net->stream;
-    if (!x0_ready)
-        k_input<<<(bp * kInPad + 255) / 256, 256, 0, s>>>(net->q, n, bp, net->x0);
-    GemmOut o{};
-    o.ldo = kH;
-    o.bias = net->params + ob1; o.z = net->z1; o.h = net->h1;
-    gemm<kModeFwd>(s, bp, kH, kInPad, Mat{net->x0, kInPad, 1},
-                   Mat{net->w1p, 1, kInPad}, o, watch(net));
-    o.bias = net->params + ob2; o.z = net->z2; o.h = net->h2;
-    gemm<kModeFwd>(s, bp, kH, kH, Mat{net->h1, kH, 1},
-                   Mat{net->w2, 1, kH}, o, watch(net));
-    o.bias = net->params + ob3; o.z = net->z3; o.h = net->h3;
-    gemm<kModeFwd>(s, bp, kH, kH, Mat{net->h2, kH, 1},
-                   Mat{net->w3, 1, kH}, o, watch(net));
-    k_head_fwd<<<(n + 7) / 8, 256, 0, s>>>(net->h3, net->params, n, net->y);
+    const ChainArgs a = chain_args(net, n);
+    k_chain<false><<<(n + kRows - 1) / kRows, kChainThreads, kChainSmemFwd, net->stream>>>(a);
     MK(cudaGetLastError(), "mlp forward launch");
     return 0;
 }
 
-// Backward pass after forward_dev (targets in net->t): net->grad (flat).
-int backward_dev(mbs_mlp *net, int n)
+// Forward and backward chain of a.n samples, then the gradients (adam false:
+// into net->grad) or the updated parameters (u holds the step's constants).
+int step_dev(mbs_mlp *net, const ChainArgs &a, UpdateArgs u, bool use_adam)
 {
-    const int bp = pad_rows(n);
-    cudaStream_t s = net->stream;
-    k_head_bwd<<<(bp * kH + 255) / 256, 256, 0, s>>>(net->y, net->t, n, bp, net->params, net->z3,
-                                                     net->dy, net->dz3);
-    k_head_grad<<<kH / 32 + 1, 256, 0, s>>>(net->dy, net->h3, bp, net->grad);
-    GemmOut o{};
-    // layer 3: dW3 = dZ3^T H2, db3 = colsum dZ3, dZ2 = (dZ3 W3) * gelu'(Z2)
-    o.ldo = kH; o.f = net->grad + oW3;
-    gemm<kModeF32>(s, kH, kH, bp, Mat{net->dz3, 1, kH},
-                   Mat{net->h2, kH, 1}, o, watch(net));
-    k_colsum_bf16<<<(kH + 31) / 32, 256, 0, s>>>(net->dz3, bp, kH, net->grad + ob3);
-    o = GemmOut{}; o.ldo = kH; o.zin = net->z2; o.h = net->dz2;
-    gemm<kModeBwd>(s, bp, kH, kH, Mat{net->dz3, kH, 1},
-                   Mat{net->w3, kH, 1}, o, watch(net));
-    // layer 2
-    o = GemmOut{}; o.ldo = kH; o.f = net->grad + oW2;
-    gemm<kModeF32>(s, kH, kH, bp, Mat{net->dz2, 1, kH},
-                   Mat{net->h1, kH, 1}, o, watch(net));
-    k_colsum_bf16<<<(kH + 31) / 32, 256, 0, s>>>(net->dz2, bp, kH, net->grad + ob2);
-    o = GemmOut{}; o.ldo = kH; o.zin = net->z1; o.h = net->dz1;
-    gemm<kModeBwd>(s, bp, kH, kH, Mat{net->dz2, kH, 1},
-                   Mat{net->w2, kH, 1}, o, watch(net));
-    // layer 1
-    o = GemmOut{}; o.ldo = kInPad; o.f = net->gw1p;
-    gemm<kModeF32>(s, kH, kInPad, bp, Mat{net->dz1, 1, kH},
-                   Mat{net->x0, kInPad, 1}, o, watch(net));
-    k_pack_w1_grad<<<(kH * kIn + 127) / 128, 128, 0, s>>>(net->gw1p, net->grad);
-    k_colsum_bf16<<<(kH + 31) / 32, 256, 0, s>>>(net->dz1, bp, kH, net->grad + ob1);
-    MK(cudaGetLastError(), "mlp backward launch");
+    const int bp = pad_rows(a.n);
+    k_chain<true><<<bp / kRows, kChainThreads, kChainSmem, net->stream>>>(a);
+    MK(cudaGetLastError(), "mlp chain launch");
+    u.img = net->img;
+    u.dy = net->dy;
+    u.bp = bp;
+    u.grad = net->grad;
+    u.p = net->params;
+    u.m = net->m;
+    u.v = net->v;
+    u.w = net->w;
+    u.watch = watch(net);
+    if (use_adam)
+        k_update<true><<<kUpJobs, kUpThreads, kUpSmem, net->stream>>>(u);
+    else
+        k_update<false><<<kUpJobs, kUpThreads, kUpSmem, net->stream>>>(u);
+    MK(cudaGetLastError(), "mlp update launch");
     return 0;
 }
 
 int refresh(mbs_mlp *net)
 {
-    k_refresh<<<(kH * kH + 255) / 256, 256, 0, net->stream>>>(net->params, net->w1p, net->w2, net->w3);
+    k_refresh<<<(kH * kH + 255) / 256, 256, 0, net->stream>>>(net->params, net->w);
     MK(cudaGetLastError(), "mlp refresh launch");
     return 0;
 }
@@ -670,12 +917,13 @@ extern "C" int mbs_mlp_create(mbs_mlp **out, int device, uint64_t seed)
     const size_t np = kNParams;
     if (cudaMalloc((void **)&net->params, np * 4) || cudaMalloc((void **)&net->grad, np * 4)
         || cudaMalloc((void **)&net->m, np * 4) || cudaMalloc((void **)&net->v, np * 4)
-        || cudaMalloc((void **)&net->w1p, kH * kInPad * sizeof(bf16))
-        || cudaMalloc((void **)&net->w2, kH * kH * sizeof(bf16))
-        || cudaMalloc((void **)&net->w3, kH * kH * sizeof(bf16))
-        || cudaMalloc((void **)&net->gw1p, kH * kInPad * 4) || cudaMalloc((void **)&net->scalar, 16)
-        || cudaMemset(net->scalar, 0, 16))
+        || cudaMalloc((void **)&net->wimg, (kH * kInPad + 4 * kImg) * sizeof(bf16))
+        || cudaMalloc((void **)&net->scalar, 16) || cudaMemset(net->scalar, 0, 16))
         return bail(-4);
+    net->w = Weights{net->wimg, net->wimg + kH * kInPad, net->wimg + kH * kInPad + kImg,
+                     net->wimg + kH * kInPad + 2 * kImg, net->wimg + kH * kInPad + 3 * kImg};
+    if (set_attrs(net))
+        return bail(-3);
     // uniform +-sqrt(6 / fan_in) weights, zero biases
     std::vector<float> p(np, 0.f);
     std::mt19937_64 rng(seed);
@@ -701,8 +949,7 @@ extern "C" int mbs_mlp_destroy(mbs_mlp *net)
         return -1;
     cudaSetDevice(net->device);
     free_acts(net);
-    void *ps[] = {net->params, net->grad, net->m, net->v, net->w1p, net->w2, net->w3, net->gw1p,
-                  net->scalar};
+    void *ps[] = {net->params, net->grad, net->m, net->v, net->wimg, net->acts, net->scalar};
     for (void *p : ps)
         cudaFree(p);
     if (net->stream)
@@ -776,11 +1023,11 @@ extern "C" int mbs_mlp_loss_grad(mbs_mlp *net, const float *q, const float *t, i
         return mfail(net, -1, "bad arguments");
     MK(cudaSetDevice(net->device), "cudaSetDevice");
     int rc = ensure_acts(net, n);
-    if (rc)
+    if (rc || (rc = ensure_images(net, n)))
         return rc;
     MK(cudaMemcpyAsync(net->q, q, (size_t)n * kIn * 4, cudaMemcpyHostToDevice, net->stream), "H2D q");
     MK(cudaMemcpyAsync(net->t, t, (size_t)n * 4, cudaMemcpyHostToDevice, net->stream), "H2D t");
-    if ((rc = forward_dev(net, n)) || (rc = backward_dev(net, n)))
+    if ((rc = step_dev(net, chain_args(net, n), UpdateArgs{}, false)))
         return rc;
     k_loss<<<1, 256, 0, net->stream>>>(net->y, net->t, n, net->scalar);
     MK(cudaGetLastError(), "loss launch");
@@ -801,8 +1048,8 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
         return mfail(net, -1, "bad arguments");
     MK(cudaSetDevice(net->device), "cudaSetDevice");
     batch = std::min(batch, n);
-    int rc = ensure_acts(net, std::max(batch, n));
-    if (rc)
+    int rc = ensure_acts(net, n);
+    if (rc || (rc = ensure_images(net, batch)))
         return rc;
     cudaStream_t s = net->stream;
     // one epoch's steps: minibatches of `batch`, the last one shorter
@@ -860,24 +1107,28 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
         cleanup();
         return mfail(net, -3, std::string("training upload: ") + cudaGetErrorString(e));
     }
-    // One epoch (every minibatch: gather, forward, backward, Adam, BF16
-    // weight copies, cursor advance) captured once as a graph and replayed
-    // per epoch: about twenty small launches per step would otherwise bound
-    // the training by launch latency.
+    // One epoch (two kernels per minibatch, the epoch counter's advance at the
+    // end) captured once as a graph and replayed per epoch.
     if (epochs > 0) {
-        gemm_attrs();
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             const int spe = (int)sizes.size();
-            for (int k = 0, b0 = 0; k < spe; b0 += sizes[k], ++k) {
-                const int nb = sizes[k], bp = pad_rows(nb);
-                k_gather_input<<<(bp + 127) / 128, 128, 0, s>>>(dq, dt, didx, dstate, n, b0, nb, bp,
-                                                                net->x0, net->t);
-                if ((rc = forward_dev(net, nb, true)) || (rc = backward_dev(net, nb)))
-                    break;
-                k_adam_refresh<<<(kNParams + 255) / 256, 256, 0, s>>>(
-                    net->params, net->grad, net->m, net->v, kNParams, lr, dbc, dstate, spe, k,
-                    net->w1p, net->w2, net->w3);
+            ChainArgs ca = chain_args(net, batch);
+            ca.q = dq;
+            ca.t = dt;
+            ca.idx = didx;
+            ca.epoch = dstate;
+            ca.n_set = n;
+            UpdateArgs ua{};
+            ua.lr = lr;
+            ua.bc = dbc;
+            ua.epoch = dstate;
+            ua.steps_per_epoch = spe;
+            for (int k = 0, b0 = 0; k < spe && rc == 0; b0 += sizes[k], ++k) {
+                ca.b0 = b0;
+                ca.n = sizes[k];
+                ua.k = k;
+                rc = step_dev(net, ca, ua, true);
             }
             if (rc == 0)
                 k_next_epoch<<<1, 1, 0, s>>>(dstate);

@@ -181,3 +181,33 @@ def test_reduced_planes_and_rows(n_az, n_zen, n_orient):
     for o in range(n_orient):
         want = oracle.phi_average(oracle.po_diffract(b.select(o, 1), g, w), g)[0]
         assert np.linalg.norm(rows[o] - want) <= FP64_L2 * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 128, 129, 385])
+def test_proposal_network_step(n):
+    """One training step over the whole set at the edges of the 32-sample CTAs
+    and 128-sample images: gradients against the oracle with BF16 rounding
+    (the gate of tests/test_mlp.py), and the Adam update against the same
+    formula in float64 on the returned gradients (float32 rounding of a
+    handful of operations: 1e-6 of the step size)."""
+    from mbs_fast_b200.mlp import ProposalNet
+    from oracle import mlp_oracle as MO
+    rng = np.random.default_rng(n)
+    q = rng.normal(size=(n, 4))
+    q = (q / np.linalg.norm(q, axis=1, keepdims=True)).astype(np.float32)
+    t = np.sin(3 * q[:, 0]).astype(np.float32)
+    net = ProposalNet(seed=4)
+    p0 = net.params
+    loss, g = net.loss_grad(q, t)
+    loss_bf, g_bf = MO.loss_grad(p0, q, t, bf16_round=True)
+    assert abs(loss - loss_bf) <= 2e-3 * max(loss_bf, 1e-3)
+    assert np.linalg.norm(g - g_bf) <= 1e-2 * np.linalg.norm(g_bf) + 1e-7
+    net.train(q, t, epochs=1, batch=n, lr=1e-3, seed=1)
+    got = net.params
+    net.close()
+    # the shuffled order changes the sums over samples: gradients to 1e-5
+    # of their norm, so entries well above that step by lr sign(g)
+    big = np.abs(g) > 1e-2 * np.linalg.norm(g) / np.sqrt(len(g))
+    step = 1e-3 * g / (np.abs(g) + 1e-8)
+    assert np.max(np.abs((p0 - got - step)[big])) <= 1e-3 * 2e-3
