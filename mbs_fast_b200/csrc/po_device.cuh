@@ -102,29 +102,40 @@ __device__ __forceinline__ void sincos_turns(double u, double &s, double &c)
     c = ((q + 1) & 2) ? -cc : cc;
 }
 
-// sin and cos of 2*pi*u from a table of the 128 angles 2*pi*k/128 (tab[k] =
-// (sin, cos), filled by sincos_turns): u = k/128 + r exactly (|r| <= 1/256
-// turn, the reduction is exact as in sincos_turns), then the angle-addition
-// formulas with the Taylor polynomials of sin(2 pi r) (to r^7) and cos(2 pi r)
-// (to r^6) in r itself (coefficients (2 pi)^n / n!, rounded to double), whose
-// truncation errors are below 1e-20 and 4e-18.  15 FP64 operations and one
-// shared-memory load against about 22 operations and 8 selects of the
-// quadrant form.
+// sin and cos of 2*pi*u from a table of the kSinTab angles 2*pi*k/kSinTab
+// (tab[k] = (sin, cos), filled by fill_sincos_tab): u = k/512 + r exactly (|r| <=
+// 1/1024 turn, the reduction is exact as in sincos_turns), then the angle-
+// addition formulas.  sin(2 pi r) is its Taylor polynomial to r^5 (truncation
+// below 7e-20).  cos(2 pi r) is 1 + r^2 (C2 + C4 r^2) with the r^6 term
+// economised into C2 and C4: its x^3 (x = r^2 on [0, X], X = 2^-20) is replaced
+// by the best lower-degree polynomial 3/2 X x^2 - 9/16 X^2 x + X^3/32, whose
+// constant, 2e-18, is left out; error below 5e-18.  13 FP64 operations and one
+// shared-memory load (15 with a table of 128 and polynomials to r^7 and r^6).
+constexpr int kSinTab = 512;
+constexpr double kCos2 = -19.739208802134996;   // -(2 pi)^2 / 2!, economised
+constexpr double kCos4 = 64.93927177571068;     //  (2 pi)^4 / 4!, economised
+
+__device__ __forceinline__ void fill_sincos_tab(double2 *tab, int threads)
+{
+    for (int i = threadIdx.x; i < kSinTab; i += threads) {
+        double s, c;
+        sincos_turns(i * (1.0 / kSinTab), s, c);
+        tab[i] = make_double2(s, c);
+    }
+}
+
 __device__ __forceinline__ void sincos_turns_tab(double u, const double2 *tab, double &s, double &c)
 {
-    const double t = fma(u, 128.0, kMagic52);
+    const double t = fma(u, (double)kSinTab, kMagic52);
     const double n = t - kMagic52;
-    const int k = __double2loint(t) & 127;
-    const double r = fma(n, -0.0078125, u);          // exact, |r| <= 1/256 turn
+    const int k = __double2loint(t) & (kSinTab - 1);
+    const double r = fma(n, -1.0 / kSinTab, u);      // exact, |r| <= 1/1024 turn
     const double r2 = r * r;
-    double ps = -76.70585975306139;                  // -(2 pi)^7 / 7!
-    ps = fma(ps, r2, 81.60524927607506);             //  (2 pi)^5 / 5!
+    double ps = 81.60524927607506;                   //  (2 pi)^5 / 5!
     ps = fma(ps, r2, -41.34170224039976);            // -(2 pi)^3 / 3!
     ps = fma(ps, r2, 6.283185307179586);             //   2 pi
     const double sx = r * ps;                        // sin(2 pi r)
-    double pc = -85.45681720669373;                  // -(2 pi)^6 / 6!
-    pc = fma(pc, r2, 64.9393940226683);              //  (2 pi)^4 / 4!
-    pc = fma(pc, r2, -19.739208802178716);           // -(2 pi)^2 / 2!
+    const double pc = fma(kCos4, r2, kCos2);
     const double cx = fma(r2, pc, 1.0);              // cos(2 pi r)
     const double2 sc = tab[k];
     s = fma(sc.x, cx, sc.y * sx);
@@ -136,15 +147,15 @@ __device__ __forceinline__ void sincos_rad(double x, double &s, double &c)
     sincos_turns(x * kInvTwoPi, s, c);
 }
 
-// Reciprocal: hardware approximation refined by one Newton step.
+// Reciprocal: the hardware approximation r (about 20 bits) refined by the
+// third-order iteration r (1 + e + e^2), e = 1 - x r (error e^3, below 2^-58):
+// three FP64 operations where two Newton steps take four.
 __device__ __forceinline__ double rcp64(double x)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    const double e2 = fma(-x, r, 1.0);
-    return fma(r, e2, r);
+    return fma(r, fma(e, e, e), r);
 }
 
 __device__ __forceinline__ float rcp32(float x)

@@ -771,10 +771,13 @@ struct __align__(16) SVertRaw<double> {
     double2 q[3];   // (ps, pc) (p0, syx) (sxy, unused)
 };
 
+// FP64: 64 beams a stage whatever the CTA (a record is 288 bytes, and the sine
+// table takes 8 KB).  FP32C: the stage ends set where the FP32 block sums are
+// folded.
 template <typename T, int TPB>
 struct StageCfg {
-    static constexpr int kBeams = TPB;
-    static constexpr int kVerts = 4 * TPB;
+    static constexpr int kBeams = sizeof(T) == 8 ? 64 : TPB;
+    static constexpr int kVerts = 4 * kBeams;
     static constexpr size_t kBytes = kBeams * sizeof(SBeamRaw<T>) + kVerts * sizeof(SVertRaw<T>);
 };
 
@@ -1008,22 +1011,31 @@ __device__ __forceinline__ void vertex_phasors(const double *st, const double *c
 __device__ __forceinline__ double rcp_t(double x) { return rcp64(x); }
 __device__ __forceinline__ float rcp_t(float x) { return rcp32(x); }
 
-// Edge sums S_d = sum_e (P(e+1) - P(e)) / C_e of one beam for the DPT
+// FP64 edge sums S_d = sum_e (P(e+1) - P(e)) / C_e of one beam for the DPT
 // directions of a thread.  The reference's two branches share one form,
 // C_e = X2 + slope_e X1 with (X1, X2, slope) = (B, A, slope_yx) when |B| > |A|
 // (x branch) and (A, B, slope_xy) otherwise (y branch).  All vertex phasors
 // are independent, so the NV*DPT chains interleave.  mn[d] receives the
-// smallest |C_e| (nearly singular edges go to the FP64 pass).
+// smallest high word of |C_e| (nearly singular edges go to the FP64 pass): the
+// comparison runs on the integer pipe, the FP64 pipe is what bounds the kernel
+// (96 orientations of 87 beams on 48 x 1801 directions: 10.8 ms with edge
+// differences, FP64 minima, two Newton steps and the table of 128; 9.5 ms so).
+__device__ __forceinline__ uint32_t abs_hi(double x)
+{
+    return (uint32_t)__double2hiint(x) & 0x7fffffffu;
+}
+
 // With kDrop an edge with |C_e| <= eps is left out instead (its coefficient
 // becomes kDropped, its term 1e-100 of the others).
 constexpr double kDropped = 1e100;
 
-template <typename T, int DPT, int NV, bool kDrop>
-__device__ __forceinline__ void edge_sums_fixed(const SVertRaw<T> *v, const double *st, const double *ct,
-                                                const T *X1, const T *X2, const bool *useX,
-                                                T *sr, T *si, T *mn, const double2 *tab, double eps)
+template <int DPT, int NV, bool kDrop>
+__device__ __forceinline__ void edge_sums_fixed(const SVertRaw<double> *v, const double *st, const double *ct,
+                                                const double *X1, const double *X2, const bool *useX,
+                                                double *sr, double *si, uint32_t *mn, const double2 *tab,
+                                                double eps)
 {
-    T c[DPT][NV], s[DPT][NV], syx[NV], sxy[NV];
+    double c[DPT][NV], s[DPT][NV], syx[NV], sxy[NV];
 #pragma unroll
     for (int e = 0; e < NV; ++e) {
         VertRegs w;
@@ -1034,40 +1046,39 @@ __device__ __forceinline__ void edge_sums_fixed(const SVertRaw<T> *v, const doub
     }
 #pragma unroll
     for (int d = 0; d < DPT; ++d) {
-        mn[d] = T(1e30);
-        sr[d] = T(0);
-        si[d] = T(0);
-    }
-    // consecutive edges share one reciprocal: 1/a = b/(ab), 1/b = a/(ab)
-    // (FP64 here: coefficients between eps1 and about 1e30 |X1| keep the
-    // product far from overflow and underflow; a pair with a smaller one is
-    // marked and its sums discarded)
+        mn[d] = 0xffffffffu;
+        // 1 / C_e; consecutive edges share one reciprocal: 1/a = b/(ab),
+        // 1/b = a/(ab) (coefficients between eps1 and about 1e30 |X1| keep the
+        // product far from overflow and underflow; a pair with a smaller one
+        // is marked and its sums discarded)
+        double inv[NV];
 #pragma unroll
-    for (int e = 0; e < NV; e += 2) {
-#pragma unroll
-        for (int d = 0; d < DPT; ++d) {
-            T ca = fma(useX[d] ? syx[e] : sxy[e], X1[d], X2[d]);
+        for (int e = 0; e < NV; e += 2) {
+            double ca = fma(useX[d] ? syx[e] : sxy[e], X1[d], X2[d]);
+            mn[d] = min(mn[d], abs_hi(ca));
             if (kDrop && fabs(ca) <= eps)
                 ca = kDropped;
-            const int e1 = (e + 1 < NV) ? e + 1 : 0;
             if (e + 1 < NV) {
-                T cb = fma(useX[d] ? syx[e1] : sxy[e1], X1[d], X2[d]);
+                double cb = fma(useX[d] ? syx[e + 1] : sxy[e + 1], X1[d], X2[d]);
+                mn[d] = min(mn[d], abs_hi(cb));
                 if (kDrop && fabs(cb) <= eps)
                     cb = kDropped;
-                const T r = rcp_t(ca * cb);
-                const T ia = cb * r, ib = ca * r;
-                const int e2 = (e + 2 < NV) ? e + 2 : 0;
-                mn[d] = fmin(mn[d], fmin(fabs(ca), fabs(cb)));
-                sr[d] = fma(c[d][e1] - c[d][e], ia, sr[d]);
-                si[d] = fma(s[d][e1] - s[d][e], ia, si[d]);
-                sr[d] = fma(c[d][e2] - c[d][e1], ib, sr[d]);
-                si[d] = fma(s[d][e2] - s[d][e1], ib, si[d]);
+                const double r = rcp64(ca * cb);
+                inv[e] = cb * r;
+                inv[e + 1] = ca * r;
             } else {
-                const T inv = rcp_t(ca);
-                mn[d] = fmin(mn[d], fabs(ca));
-                sr[d] = fma(c[d][0] - c[d][e], inv, sr[d]);
-                si[d] = fma(s[d][0] - s[d][e], inv, si[d]);
+                inv[e] = rcp64(ca);
             }
+        }
+        // the sum regrouped by vertices: sum_v P(v) (1/C_{v-1} - 1/C_v)
+        const double w0 = inv[NV - 1] - inv[0];
+        sr[d] = c[d][0] * w0;
+        si[d] = s[d][0] * w0;
+#pragma unroll
+        for (int e = 1; e < NV; ++e) {
+            const double we = inv[e - 1] - inv[e];
+            sr[d] = fma(c[d][e], we, sr[d]);
+            si[d] = fma(s[d][e], we, si[d]);
         }
     }
 }
@@ -1220,14 +1231,14 @@ __device__ __forceinline__ void edge_tail_loop_f32(const SVertRaw<float> *v, int
     }
 }
 
-template <typename T, int DPT, bool kDrop>
-__device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, const double *st,
-                                               const double *ct, const T *X1, const T *X2,
-                                               const bool *useX, T *sr, T *si, T *mn,
+template <int DPT, bool kDrop>
+__device__ __forceinline__ void edge_sums_loop(const SVertRaw<double> *v, int nv, const double *st,
+                                               const double *ct, const double *X1, const double *X2,
+                                               const bool *useX, double *sr, double *si, uint32_t *mn,
                                                const double2 *tab, double eps)
 {
-    T c0[DPT], s0[DPT], cp_[DPT], sp_[DPT];
-    T syx, sxy;
+    double c0[DPT], s0[DPT], cp_[DPT], sp_[DPT];
+    double syx, sxy;
     VertRegs w;
     load_vert(v[0], w, syx, sxy);
 #pragma unroll
@@ -1235,25 +1246,25 @@ __device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, con
         vertex_phasor_t(st[d], ct[d], w, tab, s0[d], c0[d]);
         cp_[d] = c0[d];
         sp_[d] = s0[d];
-        mn[d] = T(1e30);
-        sr[d] = T(0);
-        si[d] = T(0);
+        mn[d] = 0xffffffffu;
+        sr[d] = 0.0;
+        si[d] = 0.0;
     }
     for (int e = 0; e < nv; ++e) {
         const bool last = e + 1 == nv;
-        const T syx_e = syx, sxy_e = sxy;
+        const double syx_e = syx, sxy_e = sxy;
         if (!last)
             load_vert(v[e + 1], w, syx, sxy);
 #pragma unroll
         for (int d = 0; d < DPT; ++d) {
-            T cn = c0[d], sn = s0[d];
+            double cn = c0[d], sn = s0[d];
             if (!last)
                 vertex_phasor_t(st[d], ct[d], w, tab, sn, cn);
-            T coef = fma(useX[d] ? syx_e : sxy_e, X1[d], X2[d]);
+            double coef = fma(useX[d] ? syx_e : sxy_e, X1[d], X2[d]);
+            mn[d] = min(mn[d], abs_hi(coef));
             if (kDrop && fabs(coef) <= eps)
                 coef = kDropped;
-            const T inv = rcp_t(coef);
-            mn[d] = fmin(mn[d], fabs(coef));
+            const double inv = rcp64(coef);
             sr[d] = fma(cn - cp_[d], inv, sr[d]);
             si[d] = fma(sn - sp_[d], inv, si[d]);
             cp_[d] = cn;
@@ -1264,19 +1275,18 @@ __device__ __forceinline__ void edge_sums_loop(const SVertRaw<T> *v, int nv, con
 
 // FP64 edge sums of one beam (the FP32C path uses edge_head_f32 and the
 // tails above): fixed vertex counts unrolled, longer apertures in a loop.
-template <typename T, int DPT, bool kDrop = false>
-__device__ __forceinline__ void edge_sums(const SVertRaw<T> *v, int nv, const double *st,
-                                          const double *ct, const T *X1, const T *X2,
-                                          const bool *useX, T *sr, T *si, T *mn,
+template <int DPT, bool kDrop = false>
+__device__ __forceinline__ void edge_sums(const SVertRaw<double> *v, int nv, const double *st,
+                                          const double *ct, const double *X1, const double *X2,
+                                          const bool *useX, double *sr, double *si, uint32_t *mn,
                                           const double2 *tab, double eps = 0.0)
 {
-    static_assert(sizeof(T) == 8, "FP64 path");
     switch (nv) {   // warp-uniform: every lane evaluates the same beam
-    case 3: edge_sums_fixed<T, DPT, 3, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
-    case 4: edge_sums_fixed<T, DPT, 4, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
-    case 5: edge_sums_fixed<T, DPT, 5, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
-    case 6: edge_sums_fixed<T, DPT, 6, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
-    default: edge_sums_loop<T, DPT, kDrop>(v, nv, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 3: edge_sums_fixed<DPT, 3, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 4: edge_sums_fixed<DPT, 4, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 5: edge_sums_fixed<DPT, 5, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    case 6: edge_sums_fixed<DPT, 6, kDrop>(v, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
+    default: edge_sums_loop<DPT, kDrop>(v, nv, st, ct, X1, X2, useX, sr, si, mn, tab, eps); break;
     }
 }
 
@@ -1447,15 +1457,10 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
     __shared__ int s_item;
     __shared__ double s_zdel[TPB / 32];
     __shared__ int s_rwarp[TPB / 32], s_rbase[TPB], s_rok[TPB];   // the spread FP64 pass
-    // FP64: sin and cos of the 128 angles 2 pi k / 128 for the vertex phasors
-    __shared__ double2 s_sincos[kF32 ? 1 : 128];
-    if constexpr (!kF32) {
-        for (int i = threadIdx.x; i < 128; i += TPB) {
-            double sv_, cv_;
-            sincos_turns(i * 0.0078125, sv_, cv_);
-            s_sincos[i] = make_double2(sv_, cv_);
-        }
-    }
+    // FP64: the sine table of the vertex phasors
+    __shared__ double2 s_sincos[kF32 ? 1 : kSinTab];
+    if constexpr (!kF32)
+        fill_sincos_tab(s_sincos, TPB);
 
     // Persistent: take work items until none are left, so CTAs of uneven
     // cost (rare FP64 pairs, ragged beam counts) balance across the SMs.
@@ -1574,8 +1579,8 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
             for (int j = j0; j < j1; ++j) {
                 BeamRegs<T> b;
                 load_beam(sb[j], b);
-                T X1[DPT], X2[DPT], sr[DPT], si[DPT], mn[DPT], mden[DPT], Av[DPT], Bv[DPT];
-                bool useX[DPT], rare[DPT];
+                T X1[DPT], X2[DPT], sr[DPT], si[DPT], mden[DPT], Av[DPT], Bv[DPT];
+                bool useX[DPT], rare[DPT], sing[DPT];   // sing: a nearly singular edge
 #pragma unroll
                 for (int d = 0; d < DPT; ++d) {
                     T A, B;
@@ -1610,6 +1615,7 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
                     }
                 }
                 if constexpr (kF32) {
+                    float mn[DPT];
                     EdgeHead<DPT> eh;
                     const SVertRaw<float> *vb = sv + b.vs;
                     edge_head_f32<DPT>(vb, st, ct, X1, X2, useX, eh, sr, si, mn);
@@ -1620,13 +1626,22 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
                     case 6: edge_tail_fixed_f32<DPT, 6>(vb, st, ct, X1, X2, useX, eh, sr, si, mn); break;
                     default: edge_tail_loop_f32<DPT>(vb, b.nv, st, ct, X1, X2, useX, eh, sr, si, mn); break;
                     }
+#pragma unroll
+                    for (int d = 0; d < DPT; ++d)
+                        sing[d] = mn[d] <= eps;
                 } else {
-                    edge_sums<T, DPT>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos);
+                    // high words: a coefficient within 2^-20 above eps is marked
+                    // too (the pass takes its plain quotient)
+                    uint32_t mn[DPT];
+                    edge_sums<DPT>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos);
+#pragma unroll
+                    for (int d = 0; d < DPT; ++d)
+                        sing[d] = mn[d] <= abs_hi(eps);
                 }
                 T s_r[DPT], s_i[DPT];
 #pragma unroll
                 for (int d = 0; d < DPT; ++d) {
-                    rare[d] = (rare[d] || mn[d] <= eps) && active[d];
+                    rare[d] = (rare[d] || sing[d]) && active[d];
                     bits[d] |= (rare[d] ? 1u : 0u) << (j & 31);
                     // select, not multiply: a marked pair may hold inf or NaN sums
                     const T m = rcp_t(mden[d]);
@@ -2233,12 +2248,8 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
     constexpr int TPB = kThetaTpb;
     __shared__ ThetaBeam sb[kThetaBeams];
     __shared__ SVertRaw<double> sv[kThetaVerts];
-    __shared__ double2 s_sincos[128];
-    for (int i = threadIdx.x; i < 128; i += TPB) {
-        double sn, cs;
-        sincos_turns(i * 0.0078125, sn, cs);
-        s_sincos[i] = make_double2(sn, cs);
-    }
+    __shared__ double2 s_sincos[kSinTab];
+    fill_sincos_tab(s_sincos, TPB);
     const int p = blockIdx.x / tiles, tile = blockIdx.x - p * tiles;
     const double cp = P.cphi[p], sp = P.sphi[p];
     const int64_t b0 = (int64_t)blockIdx.y * beams_per_chunk;
@@ -2306,7 +2317,8 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
             marked[d] = 0;
         for (int j = 0; j < nb; ++j) {
             const ThetaBeam &b = sb[j];
-            double X1[DPT], X2[DPT], sr[DPT], si[DPT], mn[DPT], m[DPT];
+            double X1[DPT], X2[DPT], sr[DPT], si[DPT], m[DPT];
+            uint32_t mn[DPT];
             bool useX[DPT], cand[DPT];
 #pragma unroll
             for (int d = 0; d < DPT; ++d) {
@@ -2319,7 +2331,7 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
                 cand[d] = fabs(fma(A, b.slab[0], B * b.slab[1])) <= 1.0
                        && fabs(fma(A, b.slab[2], B * b.slab[3])) <= 1.0;
             }
-            edge_sums<double, DPT, true>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos, P.wc.eps1);
+            edge_sums<DPT, true>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos, P.wc.eps1);
 #pragma unroll
             for (int d = 0; d < DPT; ++d) {
                 const double q = fma(ct[d], fma(ct[d], b.q[3], b.q[1]),
