@@ -57,6 +57,9 @@ constexpr Variant kVariantsF64[] = {{64, 3, 4}, {128, 1, 3}, {96, 2, 4}, {128, 1
 // 128x1x3 / 64x2x4 / 64x1x6 for FP64 on the column).
 constexpr Variant kNoShadowF32 = {128, 3, 3};
 constexpr Variant kNoShadowF64 = {128, 1, 3};
+// Shapes for the rows past the last whole tile (see row_tail).
+constexpr Variant kTailF32[] = {{128, 1, 4}, {128, 2, 4}};
+constexpr Variant kTailF64[] = {{64, 1, 6}, {128, 1, 4}};
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
 
@@ -114,7 +117,7 @@ struct mbs_po_ctx {
     size_t phiW_cap = 0;
     int phiW_low = 0, phiW_full = 0;
     Arena raw;                   // raw upload area for staging
-    int *d_status = nullptr;      // [0] pack status, [1] work counter of the diffraction kernel
+    int *d_status = nullptr;      // [0] pack status, [1], [2] work counters of the diffraction kernel
     mbs_po_staged host_staged;   // reused by mbs_po_diffract
     cudaEvent_t ev[8] = {};
     cudaEvent_t partial_done = nullptr;   // recorded after each launch that used `partial`
@@ -776,6 +779,77 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
     return cudaGetLastError();
 }
 
+// The zenith rows past the last whole tile of the default shape (kVariants[0]:
+// 384 rows FP32C, 192 FP64) run as a second launch with fewer directions per
+// thread, on the side stream beside the main one, when a narrower shape
+// holds them: index into kTail*, or -1.  A thread whose slots lie past the
+// last row still evaluates them.  Time of a tail tile against a whole one
+// (64 orientations of 87 beams, 48 azimuths): FP32C 128 rows 0.50, 256 rows
+// 0.81; FP64 64 rows 0.45, 128 rows 0.76.  The tail shapes stage the same
+// beams at a time as the default ones, so a direction's sums are the same
+// bit for bit whichever launch holds it.
+int row_tail(int pi, int n_t)
+{
+    const Variant *tails = pi == 0 ? kTailF64 : kTailF32;
+    const Variant full = pi == 0 ? kVariantsF64[0] : kVariantsF32[0];
+    const int rest = n_t % (full.tpb * full.dpt);
+    for (int i = 0; i < 2 && rest > 0; ++i)
+        if (rest <= tails[i].tpb * tails[i].dpt)
+            return i;
+    return -1;
+}
+
+cudaError_t launch_tail(int pi, int tail, const KParams &P, cudaStream_t st)
+{
+    if (pi == 0)
+        return tail == 0 ? launch_one<double, 64, 1, false, 6>(P, st) : launch_one<double, 128, 1, false, 4>(P, st);
+    return tail == 0 ? launch_one<float, 128, 1, false, 4>(P, st) : launch_one<float, 128, 2, false, 4>(P, st);
+}
+
+// The rows of a call: [0, main_rows) in the chosen shape, the rest (`tail` >= 0)
+// in kTail*[tail].
+struct RowPlan {
+    int main_rows, tail;
+    bool beside() const { return tail >= 0 && main_rows > 0; }   // two launches
+};
+
+RowPlan plan_rows(int precision, int variant, bool ns, const Variant &V, int n_t)
+{
+    const int tail = variant == 0 && !ns ? row_tail(precision == MBS_PO_FP64 ? 0 : 1, n_t) : -1;
+    const int rows = V.tpb * V.dpt;
+    return {tail < 0 ? n_t : n_t / rows * rows, tail};
+}
+
+// The diffraction launches: the main rows on `st`, a tail beside them on
+// `side` (which already waits for the start of the call), or alone on `st`.
+// P.work: two counters.
+cudaError_t launch_rows(int precision, int variant, bool ns, KParams P, const Variant &V, const RowPlan &R,
+                        int n_chunks, cudaStream_t st, cudaStream_t side)
+{
+    cudaError_t e = cudaSuccess;
+    if (R.main_rows > 0) {
+        P.row0 = 0;
+        P.row1 = R.main_rows;
+        P.tiles_per_row = (R.main_rows + V.tpb * V.dpt - 1) / (V.tpb * V.dpt);
+        P.n_items = n_chunks * P.n_az * P.tiles_per_row;
+        e = cudaMemsetAsync(P.work, 0, sizeof(int), st);
+        if (e == cudaSuccess)
+            e = launch_diffract(precision, variant, ns, P, st);
+    }
+    if (e == cudaSuccess && R.tail >= 0) {
+        P.row0 = R.main_rows;
+        P.row1 = P.n_t;
+        P.tiles_per_row = 1;
+        P.n_items = n_chunks * P.n_az;
+        ++P.work;
+        cudaStream_t ts = R.beside() ? side : st;
+        e = cudaMemsetAsync(P.work, 0, sizeof(int), ts);
+        if (e == cudaSuccess)
+            e = launch_tail(precision == MBS_PO_FP64 ? 0 : 1, R.tail, P, ts);
+    }
+    return e;
+}
+
 // How the chunk partials reach the caller: added into its accumulators,
 // stored there, or left in ctx->partial.
 enum class Sums { kAdd, kStore, kLeave };
@@ -834,31 +908,33 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
     P.n_t = nT;
     P.n_orient = n_orient;
     P.orient_per_chunk = L.orient_per_chunk;
-    P.tiles_per_row = L.tiles_per_row;
     P.orient_per_set = per_set;
     P.chunks_per_set = L.chunks_per_set;
     P.wc = ctx->wc;
     P.partial = ctx->partial;
     P.partial_ns = ns ? ctx->partial + plane * L.n_chunks : nullptr;
     P.work = ctx->d_status + 1;
-    P.n_items = L.n_chunks * nAz * L.tiles_per_row;
     int launches = 0;
     CK(cudaEventRecord(ctx->ev[0], st), "event");
-    // polar rows on the side stream, concurrently with the main kernel
-    if (ctx->grid.n_pole > 0) {
+    // polar rows and a row tail on the side stream, concurrently with the
+    // main kernel
+    const RowPlan R = plan_rows(precision, variant, ns, V, nT);
+    const bool on_side = ctx->grid.n_pole > 0 || R.beside();
+    if (on_side)
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
+    if (ctx->grid.n_pole > 0) {
         CK(launch_pole(P, L, s->n_beams, s->n_orient, ctx->grid.pole_rows, ctx->grid.n_pole, ns, ctx->side),
            "pole kernel launch");
-        CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
         ++launches;
     }
-    CK(cudaMemsetAsync(P.work, 0, sizeof(int), st), "memset work counter");
-    const cudaError_t e = launch_diffract(precision, variant, ns, P, st);
+    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, ctx->side);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "diffraction kernel launch");
-    ++launches;
-    if (ctx->grid.n_pole > 0)
+    launches += R.beside() ? 2 : 1;
+    if (on_side) {
+        CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
         CK(cudaStreamWaitEvent(st, ctx->ev[6], 0), "join side stream");
+    }
     CK(cudaEventRecord(ctx->ev[1], st), "event");
     if (sums != Sums::kLeave) {
         CK(launch_reduce(ctx->partial, L.chunks_per_set, G, n_sets, sums == Sums::kAdd, M_dev, st), "reduce launch");
@@ -1925,28 +2001,29 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     P.n_t = nT;
     P.n_orient = s->n_orient;
     P.orient_per_chunk = L.orient_per_chunk;
-    P.tiles_per_row = L.tiles_per_row;
     P.orient_per_set = s->n_orient;
     P.chunks_per_set = L.n_chunks;
     P.wc = ctx->wc;
     P.partial = scratch;
     P.partial_ns = ns ? scratch + plane * L.n_chunks : nullptr;
     P.work = work;
-    P.n_items = L.n_chunks * nAz * L.tiles_per_row;
     cudaStream_t st = (cudaStream_t)stream;
-    if (ctx->grid.n_pole > 0) {
+    const RowPlan R = plan_rows(precision, variant, ns, V, nT);
+    const bool on_side = ctx->grid.n_pole > 0 || R.beside();
+    if (on_side) {
         CK(cudaEventRecord(ctx->ev[0], st), "event");
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
+    }
+    if (ctx->grid.n_pole > 0)
         CK(launch_pole(P, L, s->n_beams, s->n_orient, ctx->grid.pole_rows, ctx->grid.n_pole, ns, ctx->side),
            "pole kernel launch");
-        CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
-    }
-    CK(cudaMemsetAsync(work, 0, sizeof(int), st), "memset work counter");
-    const cudaError_t e = launch_diffract(precision, variant, ns, P, st);
+    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, ctx->side);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "diffraction kernel launch");
-    if (ctx->grid.n_pole > 0)
+    if (on_side) {
+        CK(cudaEventRecord(ctx->ev[6], ctx->side), "event");
         CK(cudaStreamWaitEvent(st, ctx->ev[6], 0), "join side stream");
+    }
     CK(launch_reduce(P.partial, L.n_chunks, G, 1, true, M_dev, st), "reduce launch");
     if (ns)
         CK(launch_reduce(P.partial_ns, L.n_chunks, G, 1, true, Mns_dev, st), "reduce launch");

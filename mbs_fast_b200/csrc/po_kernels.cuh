@@ -125,6 +125,7 @@ struct KParams {
     const double *st, *ct, *sphi, *cphi, *vf;
     const int8_t *row_kind;    // [n_t] 0 regular, 1 polar (po_pole_kernel), 2 general
     int n_az, n_t;             // n_t = n_zen+1
+    int row0, row1;            // zenith rows of this launch
     int n_orient;
     int orient_per_chunk;
     int tiles_per_row;
@@ -1017,9 +1018,7 @@ __device__ __forceinline__ float rcp_t(float x) { return rcp32(x); }
 // (x branch) and (A, B, slope_xy) otherwise (y branch).  All vertex phasors
 // are independent, so the NV*DPT chains interleave.  mn[d] receives the
 // smallest high word of |C_e| (nearly singular edges go to the FP64 pass): the
-// comparison runs on the integer pipe, the FP64 pipe is what bounds the kernel
-// (96 orientations of 87 beams on 48 x 1801 directions: 10.8 ms with edge
-// differences, FP64 minima, two Newton steps and the table of 128; 9.5 ms so).
+// comparison runs on the integer pipe, the FP64 pipe is what bounds the kernel.
 __device__ __forceinline__ uint32_t abs_hi(double x)
 {
     return (uint32_t)__double2hiint(x) & 0x7fffffffu;
@@ -1431,7 +1430,7 @@ struct JonesAcc {
 
 // Fused diffraction kernel, persistent: each CTA takes work items
 // (orientation chunk, azimuth bin, zenith tile) from a global counter.  Each
-// thread owns DPT directions of an item (zenith rows t0 + d*TPB of the
+// thread owns DPT directions of an item (rows trow + d*TPB + thread of the
 // item's azimuth).  T = float selects FP32C.
 template <typename T, int TPB, int DPT, bool NS, int MINB>
 __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
@@ -1476,6 +1475,7 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
     const int pt = item - chunk * items_per_chunk;
     const int p = pt / P.tiles_per_row;
     const int tile = pt - p * P.tiles_per_row;
+    const int trow = P.row0 + tile * kDirs;   // the tile's first zenith row
     int o0, o1;
     chunk_range(P, chunk, o0, o1);
     const double cp = P.cphi[p], sp = P.sphi[p];
@@ -1486,10 +1486,10 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
     T stT[DPT], ctT[DPT];
 #pragma unroll
     for (int d = 0; d < DPT; ++d) {
-        const int tr = tile * kDirs + d * TPB + threadIdx.x;
-        t[d] = tr < P.n_t ? tr : P.n_t - 1;
+        const int tr = trow + d * TPB + threadIdx.x;
+        t[d] = tr < P.row1 ? tr : P.row1 - 1;
         const int kind = P.row_kind[t[d]];
-        active[d] = tr < P.n_t && kind != 1;
+        active[d] = tr < P.row1 && kind != 1;
         general[d] = kind == 2;
         st[d] = P.st[t[d]];
         ct[d] = P.ct[t[d]];
@@ -1506,7 +1506,7 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
     // spread of the tile's directions around its middle row, for the zone
     // flags of the stage fill (read there after the fill's first barrier)
     {
-        const int tm = min(tile * kDirs + kDirs / 2, P.n_t - 1);
+        const int tm = min(trow + kDirs / 2, P.row1 - 1);
         const double stc = P.st[tm], ctc = P.ct[tm];
         double dd = 0.0;
 #pragma unroll
@@ -1548,7 +1548,7 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
             __syncthreads();   // previous stage fully consumed
             TileZone tz;
             {
-                const int tm = min(tile * kDirs + kDirs / 2, P.n_t - 1);
+                const int tm = min(trow + kDirs / 2, P.row1 - 1);
                 double dd = 0.0;
 #pragma unroll
                 for (int w = 0; w < TPB / 32; ++w)
@@ -1780,7 +1780,7 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
                                     k -= c;
                                 }
                             }
-                        const int to = tile * kDirs + od * TPB + o;   // < n_t: marked pairs are active
+                        const int to = trow + od * TPB + o;   // < row1: marked pairs are active
                         const double sto = P.st[to], cto = P.ct[to];
                         const bool gen = P.row_kind[to] == 2;
                         const T stTo = (T)sto, ctTo = (T)cto;

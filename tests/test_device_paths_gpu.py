@@ -211,3 +211,39 @@ def test_proposal_network_step(n):
     big = np.abs(g) > 1e-2 * np.linalg.norm(g) / np.sqrt(len(g))
     step = 1e-3 * g / (np.abs(g) + 1e-8)
     assert np.max(np.abs((p0 - got - step)[big])) <= 1e-3 * 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tile,rest", [
+    (p, n, r) for p, n, rs in ((abi.FP64, 192, (1, 64, 65, 128, 129)), (abi.FP32C, 384, (1, 128, 129, 256, 257)))
+    for r in rs])
+@pytest.mark.parametrize("whole", [0, 1])
+def test_row_tails(precision, tile, rest, whole):
+    """Zenith rows past the last whole tile (alone, and after a whole tile):
+    against the oracle, and bit for bit against the same directions evaluated
+    inside a whole tile of the main shape (FP32C sums included: the tail
+    shapes stage the same beams)."""
+    b, w = S.ragged(3, 70, 12.0, 17), S.wave()
+    g = S.grid(2, whole * tile + rest - 1)
+    h = GpuHandlerPO(g, w)
+    M = h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, precision=precision)
+    h.close()
+    assert _l2(M, oracle.po_diffract(b, g, w)) < (FP64_L2 if precision == abi.FP64 else 2e-5)
+    # the last `tile` rows (polar row left out) as a grid of their own, padded
+    # with rows between the first ones when there are fewer
+    th, vf = g.theta[1:-1][-tile:], g.vf[:, 1:-1][:, -tile:]
+    n = len(th)
+    fill = tile - n
+    extra = np.linspace(0.01, 0.02, fill)
+    th2 = np.concatenate([extra, th])
+    phi = np.arange(2) * g.az_step
+    reg = np.stack([-np.sin(phi), np.cos(phi), np.zeros(2)], -1)
+    g2 = type(g)(2, tile - 1, g.az_step, np.ascontiguousarray(th2),
+                 np.ascontiguousarray(np.concatenate([np.repeat(reg[:, None], fill, 1), vf], 1)), None)
+    h2 = GpuHandlerPO(g2, w)
+    M2 = h2.new_mueller()
+    assert h2.handle_orientations_to_local_gpu(b, M2, precision=precision)
+    h2.close()
+    if n:
+        assert np.array_equal(M[:, 1:-1][:, -n:], M2[:, fill:])
