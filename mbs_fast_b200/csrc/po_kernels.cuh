@@ -1018,7 +1018,9 @@ __device__ __forceinline__ float rcp_t(float x) { return rcp32(x); }
 // (x branch) and (A, B, slope_xy) otherwise (y branch).  All vertex phasors
 // are independent, so the NV*DPT chains interleave.  mn[d] receives the
 // smallest high word of |C_e| (nearly singular edges go to the FP64 pass): the
-// comparison runs on the integer pipe, the FP64 pipe is what bounds the kernel.
+// comparison runs on the integer pipe, the FP64 pipe is what bounds the kernel
+// (96 orientations of 87 beams on 48 x 1801 directions: 10.8 ms with edge
+// differences, FP64 minima, two Newton steps and the table of 128; 9.5 ms so).
 __device__ __forceinline__ uint32_t abs_hi(double x)
 {
     return (uint32_t)__double2hiint(x) & 0x7fffffffu;
