@@ -169,16 +169,43 @@ int ensure(mbs_po_ctx *ctx, T *&ptr, size_t &cap, size_t n, const char *what)
     return MBS_PO_OK;
 }
 
+// Unused memory that a context's pool may keep after a staged batch is freed.
+constexpr size_t kPoolKeep = (size_t)512 << 20;
+
+// Memory from the context's pool, in stream order on `st`; what the pool keeps
+// unused is given back to the device before the request is refused.
+cudaError_t pool_alloc(mbs_po_ctx *ctx, void **p, size_t bytes, cudaStream_t st)
+{
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    }
+    if (e != cudaSuccess)
+        *p = nullptr;
+    return e;
+}
+
+// A staged batch's arena: from the context's pool (mapping and unmapping
+// device memory per batch took 0.5 ms of cudaMalloc and 1 to 4 ms of cudaFree
+// on a batch that diffracts in 5), ready for every stream on return.
 int ensure_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what)
 {
     if (bytes <= a.cap && a.base)
         return MBS_PO_OK;
-    cudaFree(a.base);
+    if (a.base) {
+        CK(cudaDeviceSynchronize(), "releasing an arena");
+        cudaFree(a.base);
+    }
     a.base = nullptr;
     a.cap = 0;
-    cudaError_t e = cudaMalloc(&a.base, std::max<size_t>(bytes, 256));
+    cudaError_t e = pool_alloc(ctx, &a.base, std::max<size_t>(bytes, 256), ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess)
-        return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMalloc ") + what + ": " + cudaGetErrorString(e));
+        return fail(ctx, MBS_PO_ENOMEM, std::string("device memory for the ") + what + ": " + cudaGetErrorString(e));
     a.cap = std::max<size_t>(bytes, 256);
     return MBS_PO_OK;
 }
@@ -211,7 +238,7 @@ int grow_partial(mbs_po_ctx *ctx, size_t n, cudaStream_t st, size_t min_doubles 
     ctx->partial = nullptr;
     const size_t want = std::max<size_t>(std::max<size_t>(n, 2 * ctx->partial_cap), min_doubles);
     ctx->partial_cap = 0;
-    e = cudaMallocFromPoolAsync((void **)&ctx->partial, want * sizeof(double), ctx->pool, st);
+    e = pool_alloc(ctx, (void **)&ctx->partial, want * sizeof(double), st);
     if (e != cudaSuccess) {
         ctx->partial = nullptr;
         return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMallocAsync partials: ") + cudaGetErrorString(e));
@@ -244,7 +271,7 @@ int grow_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what, cudaSt
     const size_t want = std::max<size_t>({(size_t)2 * bytes, (size_t)4 * a.cap, (size_t)32 << 20});
     const size_t cap = (want + ((size_t)1 << 21) - 1) & ~(((size_t)1 << 21) - 1);
     a.cap = 0;
-    cudaError_t e = cudaMallocFromPoolAsync(&a.base, cap, ctx->pool, st);
+    cudaError_t e = pool_alloc(ctx, &a.base, cap, st);
     if (e != cudaSuccess) {
         a.base = nullptr;
         return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMallocAsync ") + what + ": " + cudaGetErrorString(e));
@@ -253,10 +280,30 @@ int grow_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what, cudaSt
     return MBS_PO_OK;
 }
 
-void staged_release(mbs_po_staged *s)
+// Waits for all work on the device (a diffraction may still read the batch on
+// any stream) and gives the arena back to the context's pool (`ctx` null: the
+// context is gone, its pool goes with the last arena).
+void staged_release(mbs_po_ctx *ctx, mbs_po_staged *s)
 {
-    cudaFree(s->arena.base);
+    if (s->arena.base && cudaDeviceSynchronize() == cudaSuccess) {
+        if (ctx)
+            cudaFreeAsync(s->arena.base, ctx->stream);
+        else
+            cudaFree(s->arena.base);
+    }
     *s = mbs_po_staged();
+}
+
+// More than kPoolKeep unused in the pool: all of it goes back to the device
+// (the pool releases whole blocks, a large batch's at once or not at all).
+void pool_trim(mbs_po_ctx *ctx)
+{
+    uint64_t held = 0, used = 0;
+    if (cudaStreamSynchronize(ctx->stream) == cudaSuccess   // the frees have completed
+        && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess
+        && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess
+        && held > used + kPoolKeep)
+        cudaMemPoolTrimTo(ctx->pool, 0);
 }
 
 int validate(mbs_po_ctx *ctx, const mbs_po_beams *b)
@@ -358,7 +405,7 @@ extern "C" int mbs_po_destroy(mbs_po_ctx *ctx)
     cudaFreeHost(ctx->hres);
     cudaFree(ctx->raw.base);
     cudaFree(ctx->d_status);
-    staged_release(&ctx->host_staged);
+    staged_release(ctx, &ctx->host_staged);
     for (int i = 0; i < 8; ++i)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->partial_done)
@@ -1019,13 +1066,13 @@ extern "C" int mbs_po_stage(mbs_po_ctx *ctx, const mbs_po_beams *beams, mbs_po_s
     mbs_po_staged *s = new mbs_po_staged();
     int rc = stage_into(ctx, beams, s, ctx->stream);
     if (rc) {
-        staged_release(s);
+        staged_release(ctx, s);
         delete s;
         return rc;
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        staged_release(s);
+        staged_release(ctx, s);
         delete s;
         return cuda_fail(ctx, e, "stage sync");
     }
@@ -1061,7 +1108,9 @@ extern "C" int mbs_po_staged_free(mbs_po_ctx *ctx, mbs_po_staged *s)
         return MBS_PO_EINVAL;
     if (ctx)
         cudaSetDevice(ctx->device);
-    staged_release(s);
+    staged_release(ctx, s);
+    if (ctx)
+        pool_trim(ctx);
     delete s;
     return MBS_PO_OK;
 }
@@ -1132,7 +1181,7 @@ extern "C" int mbs_po_stage_repeat(mbs_po_ctx *ctx, const mbs_po_staged *src, in
     if (e == cudaSuccess && !w.empty())
         e = cudaMemcpy(v->weight, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
-        staged_release(v);
+        staged_release(ctx, v);
         delete v;
         return cuda_fail(ctx, e, "H2D repeated batch");
     }
@@ -1269,16 +1318,17 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
     // planes handed back: the grid's, or the interpolated ones
     const size_t n_out = n_full > 0 ? (size_t)n_full * n_rows * 16 : n;
     int rc;
-    if ((rc = ensure(ctx, ctx->macc, ctx->macc_cap, n * 2, "accumulators")))
+    const size_t two = ns ? 2 : 1;
+    if ((rc = ensure(ctx, ctx->macc, ctx->macc_cap, n * two, "accumulators")))
         return rc;
-    if (n_full > 0 && (rc = ensure(ctx, ctx->mfull, ctx->mfull_cap, n_out * 2, "interpolated planes")))
+    if (n_full > 0 && (rc = ensure(ctx, ctx->mfull, ctx->mfull_cap, n_out * two, "interpolated planes")))
         return rc;
-    if (ctx->hres_cap < n_out * 2 || !ctx->hres) {
+    if (ctx->hres_cap < n_out * two || !ctx->hres) {
         cudaFreeHost(ctx->hres);
         ctx->hres = nullptr;
         ctx->hres_cap = 0;
-        CK(cudaMallocHost((void **)&ctx->hres, n_out * 2 * sizeof(double)), "cudaMallocHost");
-        ctx->hres_cap = n_out * 2;
+        CK(cudaMallocHost((void **)&ctx->hres, n_out * two * sizeof(double)), "cudaMallocHost");
+        ctx->hres_cap = n_out * two;
     }
     for (double &v : ctx->prof)
         v = 0.0;
@@ -1534,13 +1584,13 @@ extern "C" int mbs_po_stage_multisize(mbs_po_ctx *ctx, const mbs_po_beams *beams
     mbs_po_staged *s = new mbs_po_staged();
     int rc = stage_into(ctx, beams, s, ctx->stream, scales, n_scales, wave_index);
     if (rc) {
-        staged_release(s);
+        staged_release(ctx, s);
         delete s;
         return rc;
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        staged_release(s);
+        staged_release(ctx, s);
         delete s;
         return cuda_fail(ctx, e, "stage sync");
     }
@@ -1564,14 +1614,13 @@ extern "C" int mbs_po_phi_average(mbs_po_ctx *ctx, const double *M_dev, const do
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     const int nT = ctx->grid.n_zen + 1, nAz = ctx->grid.n_az;
     cudaStream_t st = (cudaStream_t)stream;
-    double *buf = nullptr;
-    size_t cap = 0;
-    int rc;
     // [dcos2pi nT][rows nT*16][C_sca, g]
-    if ((rc = ensure(ctx, buf, cap, (size_t)nT * 17 + 2, "azimuth average")))
-        return rc;
+    double *buf = nullptr;
+    cudaError_t e = pool_alloc(ctx, (void **)&buf, ((size_t)nT * 17 + 2) * sizeof(double), st);
+    if (e != cudaSuccess)
+        return fail(ctx, MBS_PO_ENOMEM, std::string("azimuth average: ") + cudaGetErrorString(e));
     double *d_dc = buf, *d_rows = buf + nT, *d_out = d_rows + (size_t)nT * 16;
-    cudaError_t e = cudaMemcpyAsync(d_dc, dcos2pi, nT * sizeof(double), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(d_dc, dcos2pi, nT * sizeof(double), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
         po_phi_average_kernel<<<nT, 128, 0, st>>>(M_dev, nAz, nT, ctx->grid.theta, d_rows);
         e = cudaGetLastError();
@@ -1587,7 +1636,7 @@ extern "C" int mbs_po_phi_average(mbs_po_ctx *ctx, const double *M_dev, const do
         e = cudaMemcpyAsync(res, d_out, 2 * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
-    cudaFree(buf);
+    cudaFreeAsync(buf, st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "azimuth average");
     if (csca_out)
@@ -1623,7 +1672,7 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
     double *drows = nullptr;
     cudaStream_t st = ctx->stream;
     {
-        const cudaError_t e = cudaMallocFromPoolAsync((void **)&drows, nrow * group * sizeof(double), ctx->pool, st);
+        const cudaError_t e = pool_alloc(ctx, (void **)&drows, nrow * group * sizeof(double), st);
         if (e != cudaSuccess)
             return fail(ctx, MBS_PO_ENOMEM, std::string("orientation rows: ") + cudaGetErrorString(e));
     }
@@ -1729,7 +1778,7 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
     // cudaMalloc and cudaFree of that size per call took longer than the kernel
     double *buf = nullptr;
     const size_t need = 2 * (size_t)n + (size_t)rows * n + n;
-    cudaError_t e = cudaMallocFromPoolAsync((void **)&buf, need * sizeof(double), ctx->pool, st);
+    cudaError_t e = pool_alloc(ctx, (void **)&buf, need * sizeof(double), st);
     if (e != cudaSuccess)
         return fail(ctx, MBS_PO_ENOMEM, std::string("theta scan scratch: ") + cudaGetErrorString(e));
     double *d_st = buf, *d_ct = buf + n, *part = buf + 2 * n, *d_m11 = part + (size_t)rows * n;
@@ -1785,9 +1834,9 @@ extern "C" int mbs_po_extinction(mbs_po_ctx *ctx, const mbs_po_beams *beams, dou
     if (rc)
         return rc;
     double *d = nullptr;
-    size_t cap = 0;
-    if ((rc = ensure(ctx, d, cap, (size_t)beams->n_orient, "cext")))
-        return rc;
+    cudaError_t e = pool_alloc(ctx, (void **)&d, (size_t)beams->n_orient * sizeof(double), st);
+    if (e != cudaSuccess)
+        return fail(ctx, MBS_PO_ENOMEM, std::string("extinction: ") + cudaGetErrorString(e));
     // a warp per orientation, more where that leaves a lane over four beams
     int slices = 1;
     while (slices < kExtThreads / 32 && (int64_t)slices * 128 * beams->n_orient < beams->n_beams)
@@ -1796,12 +1845,12 @@ extern "C" int mbs_po_extinction(mbs_po_ctx *ctx, const mbs_po_beams *beams, dou
     po_extinction_kernel<<<(beams->n_orient + per_cta - 1) / per_cta, kExtThreads, 0, st>>>(
         ctx->host_staged.beams, ctx->host_staged.verts, ctx->host_staged.beam_off,
         ctx->host_staged.weight, beams->n_orient, slices, ctx->wc, d);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(cext_out, d, beams->n_orient * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
-    cudaFree(d);
+    cudaFreeAsync(d, st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "extinction");
     return MBS_PO_OK;

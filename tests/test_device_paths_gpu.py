@@ -247,3 +247,50 @@ def test_row_tails(precision, tile, rest, whole):
     h2.close()
     if n:
         assert np.array_equal(M[:, 1:-1][:, -n:], M2[:, fill:])
+
+
+@pytest.mark.gpu
+def test_staged_memory_is_reused_and_given_back():
+    """A staged batch freed while a diffraction that reads it is in flight on
+    another stream; its memory staged again at once; a batch larger than the
+    pool keeps goes back in part when it is freed, does not pile up over
+    stage and free cycles, and leaves nothing behind the context (64 MiB for
+    the driver's own blocks)."""
+    import torch
+    b, w = S.batch(40, 60, 12.0, 5), S.wave()
+    g = S.grid(16, 200)
+    h = GpuHandlerPO(g, w)
+    n = g.n_dirs * 16
+    ref = torch.zeros(n, dtype=torch.float64, device="cuda:0")
+    st = h.stage(b)
+    h.diffract_staged(st, ref.data_ptr(), precision=abi.FP64)
+    torch.cuda.synchronize()
+    st.free()
+    side = torch.cuda.Stream()
+    other = S.batch(40, 60, 12.0, 6)
+    for _ in range(3):
+        st = h.stage(b)
+        acc = torch.zeros(n, dtype=torch.float64, device="cuda:0")
+        torch.cuda.synchronize()
+        h.diffract_staged(st, acc.data_ptr(), precision=abi.FP64, stream=side.cuda_stream, stats=False)
+        st.free()
+        st2 = h.stage(other)          # takes the freed memory
+        torch.cuda.synchronize()
+        assert torch.equal(acc, ref)
+        st2.free()
+    h.close()
+    one = _with_nv(99, 31, 6.0, 2)
+    many = one.concat([one] * 2200)   # about 750 MB of records
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    h = GpuHandlerPO(g, w)
+    left = []
+    for _ in range(3):
+        st = h.stage(many)
+        held = torch.cuda.mem_get_info()[0]
+        st.free()
+        left.append(torch.cuda.mem_get_info()[0])
+        assert left[-1] > held             # part of it at once
+    assert left[0] == left[1] == left[2]   # nothing piles up
+    h.close()
+    assert torch.cuda.mem_get_info()[0] > before - (64 << 20)   # the rest with the context
