@@ -55,7 +55,7 @@ struct __align__(16) VertRec {
 // at base[w * stride + i], so the lanes of a warp that fill consecutive
 // records read consecutive words (full 32-byte sectors) instead of one
 // scattered sector per lane.
-constexpr int kBrecWords = 54;   // ab[8] Q[40] slab[4] (nearr2 | vbeg) (nv | 0)
+constexpr int kBrecWords = 54;   // ab[8] Q[40] slab[4] (nearr2 | vbeg) (nv | beam flags)
 constexpr int kVrecWords = 6;    // X Y pc p0 syx sxy
 
 struct BrecRef {
@@ -66,6 +66,10 @@ struct BrecRef {
     __device__ __forceinline__ double slab(int i) const { return p[(48 + i) * s]; }
     __device__ __forceinline__ float nearr2() const { return __int_as_float(__double2loint(p[52 * s])); }
     __device__ __forceinline__ int nv() const { return __double2loint(p[53 * s]); }
+    __device__ __forceinline__ bool external() const
+    {
+        return (__double2hiint(p[53 * s]) & MBS_PO_BEAM_EXTERNAL) != 0;
+    }
 };
 
 struct VrecRef {
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(kPackThreads) po_pack_kernel(PackParams P)
             } else if (w == 32) {
                 out[52 * P.brec_stride] = __hiloint2double(__double2loint(d[34]), __double2hiint(d[35]));
             } else {
-                out[53 * P.brec_stride] = __hiloint2double(0, __double2hiint(d[34]));
+                out[53 * P.brec_stride] = __hiloint2double(__double2loint(d[35]), __double2hiint(d[34]));
             }
         }
     }
@@ -699,6 +703,7 @@ struct BeamRegs {
     T slab[4];
     float nearr2;
     int nv, vs, gbeam, zone;
+    bool external;
 };
 
 template <typename T>
@@ -706,7 +711,7 @@ struct SBeamRaw;
 
 template <>
 struct __align__(16) SBeamRaw<float> {
-    float4 q[10];   // a0 a3 a1 a4 | a2 a5 slab0 slab1 | slab2 slab3 nearr2 nv | P[24] | gbeam vs zone
+    float4 q[10];   // a0 a3 a1 a4 | a2 a5 slab0 slab1 | slab2 slab3 nearr2 nv | P[24] | gbeam vs zone external
                     // ((a0, a3), (a1, a4), (a2, a5): operand pairs of the packed A, B;
                     // P entries 2h, 2h+1 of P0, Pc, Ps as (re, re, im, im): the
                     // real and the imaginary operand pairs of the packed Jones update)
@@ -714,8 +719,8 @@ struct __align__(16) SBeamRaw<float> {
 
 template <>
 struct __align__(16) SBeamRaw<double> {
-    double2 q[18];  // a0a1 a2a3 a4a5 | slab | slab | P[24] | (zone,nv) (gbeam,vs)
-                    // (FP64 has no near-forward zone: the nearr2 word holds the zone flag)
+    double2 q[18];  // a0a1 a2a3 a4a5 | slab | slab | P[24] | (zone + 2 external,nv) (gbeam,vs)
+                    // (FP64 has no near-forward zone: the nearr2 word holds the flags)
 };
 
 // The zenith tile of a work item seen from the stage fill: every direction
@@ -805,7 +810,8 @@ __device__ __forceinline__ void fill_beam(const BrecRef &r, double cp, double sp
 #pragma unroll
     for (int i = 0; i < 6; ++i)
         s.q[3 + i] = make_float4(P[4 * i], P[4 * i + 2], P[4 * i + 1], P[4 * i + 3]);
-    s.q[9] = make_float4(__int_as_float(gbeam), __int_as_float(vs), __int_as_float(zone), 0.f);
+    s.q[9] = make_float4(__int_as_float(gbeam), __int_as_float(vs), __int_as_float(zone),
+                         __int_as_float(r.external() ? 1 : 0));
 }
 
 __device__ __forceinline__ void fill_beam(const BrecRef &r, double cp, double sp, int vs, int gbeam,
@@ -827,7 +833,7 @@ __device__ __forceinline__ void fill_beam(const BrecRef &r, double cp, double sp
                                       -(cp * r.Q(17 + e) + sp * r.Q(25 + e)));
         s.q[13 + e / 2] = make_double2(r.Q(32 + e), r.Q(33 + e));
     }
-    s.q[17] = make_double2(__hiloint2double(r.nv(), zone), __hiloint2double(vs, gbeam));
+    s.q[17] = make_double2(__hiloint2double(r.nv(), zone + (r.external() ? 2 : 0)), __hiloint2double(vs, gbeam));
 }
 
 // FP32C: p0 carries the range-reduction constant 1.5*2^29 + 1/2, so the
@@ -857,6 +863,7 @@ __device__ __forceinline__ void load_beam(const SBeamRaw<float> &s, BeamRegs<flo
     b.gbeam = __float_as_int(q9.x);
     b.vs = __float_as_int(q9.y);
     b.zone = __float_as_int(q9.z);
+    b.external = __float_as_int(q9.w) != 0;
 }
 
 __device__ __forceinline__ void load_beam(const SBeamRaw<double> &s, BeamRegs<double> &b)
@@ -865,7 +872,8 @@ __device__ __forceinline__ void load_beam(const SBeamRaw<double> &s, BeamRegs<do
     b.a[0] = q0.x; b.a[1] = q0.y; b.a[2] = q1.x; b.a[3] = q1.y; b.a[4] = q2.x; b.a[5] = q2.y;
     b.slab[0] = q3.x; b.slab[1] = q3.y; b.slab[2] = q4.x; b.slab[3] = q4.y;
     b.nearr2 = 0.f;
-    b.zone = __double2loint(q17.x);
+    b.zone = __double2loint(q17.x) & 1;
+    b.external = (__double2loint(q17.x) & 2) != 0;
     b.nv = __double2hiint(q17.x);
     b.vs = __double2hiint(q17.y);
     b.gbeam = __double2loint(q17.y);
@@ -889,18 +897,8 @@ __device__ __forceinline__ void load_P(const SBeamRaw<double> &s, double *P)
     }
 }
 
-// P0, Pc, Ps entries 2h and 2h+1 (re, im each) of a beam record.
-__device__ __forceinline__ void load_P_pair(const SBeamRaw<float> &s, int h, float *p0, float *pc,
-                                            float *ps)
-{
-    const float4 a = s.q[3 + h], b = s.q[5 + h], c = s.q[7 + h];
-    p0[0] = a.x; p0[1] = a.z; p0[2] = a.y; p0[3] = a.w;
-    pc[0] = b.x; pc[1] = b.z; pc[2] = b.y; pc[3] = b.w;
-    ps[0] = c.x; ps[1] = c.z; ps[2] = c.y; ps[3] = c.w;
-}
-
-// FP32C packed form of load_P_pair: (re 2h, re 2h+1) and (im 2h, im 2h+1)
-// operand pairs of P0, Pc and Ps, straight from the record's layout.
+// P0, Pc, Ps entries 2h and 2h+1 of an FP32C beam record as (re 2h, re 2h+1)
+// and (im 2h, im 2h+1) operand pairs, straight from the record's layout.
 __device__ __forceinline__ void load_P_packed(const SBeamRaw<float> &s, int h, float2 &p0r, float2 &p0i,
                                               float2 &pcr, float2 &pci, float2 &psr, float2 &psi)
 {
@@ -910,6 +908,7 @@ __device__ __forceinline__ void load_P_packed(const SBeamRaw<float> &s, int h, f
     psr = make_float2(c.x, c.y); psi = make_float2(c.z, c.w);
 }
 
+// The same of an FP64 record, (re, im) each.
 __device__ __forceinline__ void load_P_pair(const SBeamRaw<double> &s, int h, double *p0, double *pc,
                                             double *ps)
 {
@@ -1430,6 +1429,57 @@ struct JonesAcc {
     }
 };
 
+// J += s x (P0 + cos t Pc + sin t Ps) for DPT directions, two complex entries
+// at a time.
+template <typename T, int DPT>
+__device__ __forceinline__ void jones_update(const SBeamRaw<T> &rec, const T *s_r, const T *s_i, const T *stT,
+                                             const T *ctT, const float2 *st2, const float2 *ct2, JonesAcc<T> *J)
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if constexpr (sizeof(T) == 4) {
+            // entries 2h and 2h+1 side by side: R = P0 + cos t Pc + sin t Ps
+            // as (re, re) and (im, im) pairs, then J_re += -s_i R_i + s_r R_r
+            // and J_im += s_i R_r + s_r R_i, the scalar form's operations
+            // lane by lane (no operand pair needs its halves swapped)
+            float2 p0r, p0i, pcr, pci, psr, psi;
+            load_P_packed(rec, h, p0r, p0i, pcr, pci, psr, psi);
+#pragma unroll
+            for (int d = 0; d < DPT; ++d) {
+                const float2 srr = make_float2(s_r[d], s_r[d]);
+                const float2 sii = make_float2(s_i[d], s_i[d]);
+                const float2 nsi = make_float2(-s_i[d], -s_i[d]);
+                const float2 Rr = __ffma2_rn(st2[d], psr, __ffma2_rn(ct2[d], pcr, p0r));
+                const float2 Ri = __ffma2_rn(st2[d], psi, __ffma2_rn(ct2[d], pci, p0i));
+                float2 jr = make_float2(J[d].b[4 * h], J[d].b[4 * h + 2]);
+                float2 ji = make_float2(J[d].b[4 * h + 1], J[d].b[4 * h + 3]);
+                jr = __ffma2_rn(nsi, Ri, jr);
+                jr = __ffma2_rn(srr, Rr, jr);
+                ji = __ffma2_rn(sii, Rr, ji);
+                ji = __ffma2_rn(srr, Ri, ji);
+                J[d].b[4 * h] = jr.x;
+                J[d].b[4 * h + 2] = jr.y;
+                J[d].b[4 * h + 1] = ji.x;
+                J[d].b[4 * h + 3] = ji.y;
+            }
+        } else {
+            T p0[4], pc[4], ps[4];
+            load_P_pair(rec, h, p0, pc, ps);
+#pragma unroll
+            for (int d = 0; d < DPT; ++d) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int q = 4 * h + 2 * e;
+                    const T rr = fma(stT[d], ps[2 * e], fma(ctT[d], pc[2 * e], p0[2 * e]));
+                    const T ri = fma(stT[d], ps[2 * e + 1], fma(ctT[d], pc[2 * e + 1], p0[2 * e + 1]));
+                    J[d].b[q] = fma(s_r[d], rr, fma(-s_i[d], ri, J[d].b[q]));
+                    J[d].b[q + 1] = fma(s_r[d], ri, fma(s_i[d], rr, J[d].b[q + 1]));
+                }
+            }
+        }
+    }
+}
+
 // Fused diffraction kernel, persistent: each CTA takes work items
 // (orientation chunk, azimuth bin, zenith tile) from a global counter.  Each
 // thread owns DPT directions of an item (rows trow + d*TPB + thread of the
@@ -1650,54 +1700,23 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
                     s_r[d] = rare[d] ? T(0) : sr[d] * m;
                     s_i[d] = rare[d] ? T(0) : si[d] * m;
                 }
-                const T fi = (NS && !(P.beams[b.gbeam].flags & MBS_PO_BEAM_EXTERNAL)) ? T(1) : T(0);
-                // J += s x (P0 + cos t Pc + sin t Ps), two complex entries at a time
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if constexpr (kF32 && !NS) {
-                        // entries 2h and 2h+1 side by side: R = P0 + cos t Pc + sin t Ps
-                        // as (re, re) and (im, im) pairs, then J_re += -s_i R_i + s_r R_r
-                        // and J_im += s_i R_r + s_r R_i, the scalar form's operations
-                        // lane by lane (no operand pair needs its halves swapped)
-                        float2 p0r, p0i, pcr, pci, psr, psi;
-                        load_P_packed(sb[j], h, p0r, p0i, pcr, pci, psr, psi);
-#pragma unroll
-                        for (int d = 0; d < DPT; ++d) {
-                            const float2 srr = make_float2(s_r[d], s_r[d]);
-                            const float2 sii = make_float2(s_i[d], s_i[d]);
-                            const float2 nsi = make_float2(-s_i[d], -s_i[d]);
-                            const float2 Rr = __ffma2_rn(st2[d], psr, __ffma2_rn(ct2[d], pcr, p0r));
-                            const float2 Ri = __ffma2_rn(st2[d], psi, __ffma2_rn(ct2[d], pci, p0i));
-                            float2 jr = make_float2(J[d].b[4 * h], J[d].b[4 * h + 2]);
-                            float2 ji = make_float2(J[d].b[4 * h + 1], J[d].b[4 * h + 3]);
-                            jr = __ffma2_rn(nsi, Ri, jr);
-                            jr = __ffma2_rn(srr, Rr, jr);
-                            ji = __ffma2_rn(sii, Rr, ji);
-                            ji = __ffma2_rn(srr, Ri, ji);
-                            J[d].b[4 * h] = jr.x;
-                            J[d].b[4 * h + 2] = jr.y;
-                            J[d].b[4 * h + 1] = ji.x;
-                            J[d].b[4 * h + 3] = ji.y;
-                        }
-                    } else {
-                        T p0[4], pc[4], ps[4];
-                        load_P_pair(sb[j], h, p0, pc, ps);
-#pragma unroll
-                        for (int d = 0; d < DPT; ++d) {
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const int q = 4 * h + 2 * e;
-                                const T rr = fma(stT[d], ps[2 * e], fma(ctT[d], pc[2 * e], p0[2 * e]));
-                                const T ri = fma(stT[d], ps[2 * e + 1], fma(ctT[d], pc[2 * e + 1], p0[2 * e + 1]));
-                                J[d].b[q] = fma(s_r[d], rr, fma(-s_i[d], ri, J[d].b[q]));
-                                J[d].b[q + 1] = fma(s_r[d], ri, fma(s_i[d], rr, J[d].b[q + 1]));
-                                if (NS) {
-                                    Jn[NS ? d : 0].b[q] = fma(fi * s_r[d], rr, fma(-fi * s_i[d], ri, Jn[NS ? d : 0].b[q]));
-                                    Jn[NS ? d : 0].b[q + 1] = fma(fi * s_r[d], ri, fma(fi * s_i[d], rr, Jn[NS ? d : 0].b[q + 1]));
-                                }
-                            }
-                        }
-                    }
+                // J += s x (P0 + cos t Pc + sin t Ps).  With no-shadow sums: FP32C
+                // adds every beam to J and the internal ones to Jn (two sums, each
+                // in beam order); FP64 adds external beams to J and internal ones
+                // to Jn, and the full sum is J + Jn.  The branches are warp-uniform
+                // (scalar updates weighted by a flag read per pair from global memory
+                // took 1,157 us on 61 x 93 beams, 47 x 358 directions; now 1,039).
+                if constexpr (!NS) {
+                    jones_update<T, DPT>(sb[j], s_r, s_i, stT, ctT, st2, ct2, J);
+                } else if constexpr (kF32) {
+                    jones_update<T, DPT>(sb[j], s_r, s_i, stT, ctT, st2, ct2, J);
+                    if (!b.external)
+                        jones_update<T, DPT>(sb[j], s_r, s_i, stT, ctT, st2, ct2, Jn);
+                } else {
+                    if (b.external)
+                        jones_update<T, DPT>(sb[j], s_r, s_i, stT, ctT, st2, ct2, J);
+                    else
+                        jones_update<T, DPT>(sb[j], s_r, s_i, stT, ctT, st2, ct2, Jn);
                 }
             }
             if ((j1 & 31) == 0 || j1 == nb) {
@@ -1819,12 +1838,15 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
 #pragma unroll
                             for (int d2 = 0; d2 < DPT; ++d2)
                                 if (d2 == cd) {
-                                    J[d2].add(dj);
                                     if (NS) {
                                         BeamRegs<T> bj;
                                         load_beam(sb[j], bj);
-                                        if (!(P.beams[bj.gbeam].flags & MBS_PO_BEAM_EXTERNAL))
+                                        if (kF32 || bj.external)
+                                            J[d2].add(dj);
+                                        if (!bj.external)
                                             Jn[NS ? d2 : 0].add(dj);
+                                    } else {
+                                        J[d2].add(dj);
                                     }
                                 }
                         }
@@ -1866,7 +1888,8 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
                 } else {
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        j[i] = (double)(set == 0 ? J[d].b[i] : Jn[NS ? d : 0].b[i]);
+                        j[i] = NS ? (double)Jn[NS ? d : 0].b[i] + (set == 0 ? (double)J[d].b[i] : 0.0)
+                                  : (double)J[d].b[i];
                 }
                 double m[16];
 #pragma unroll

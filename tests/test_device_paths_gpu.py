@@ -294,3 +294,32 @@ def test_staged_memory_is_reused_and_given_back():
     assert left[0] == left[1] == left[2]   # nothing piles up
     h.close()
     assert torch.cuda.mem_get_info()[0] > before - (64 << 20)   # the rest with the context
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [abi.FP64, abi.FP32C])
+@pytest.mark.parametrize("external", ["none", "first", "every third", "all"])
+def test_noshadow_sums(precision, external):
+    """The sums over internal beams beside the full sums: no, one, mixed and
+    only external beams, near-forward and polar rows among the directions;
+    the full sums as without the second set (FP32C bit for bit: the same
+    additions; FP64 to the rounding of a different grouping of 150 beams,
+    150 x 1.1e-16 of the largest element's scale times a margin of 10)."""
+    b, w = S.batch(3, 150, 12.0, 31), S.wave()
+    i = np.arange(b.n_beams)
+    if external != "first":
+        b.beam_flags = np.where({"none": i < 0, "every third": i % 3 == 0, "all": i >= 0}[external], 1, 0).astype(np.uint8)
+    g = S.grid(3, 140, plates=True)
+    M0, N0 = oracle.po_diffract(b, g, w, noshadow=True)
+    h = GpuHandlerPO(g, w)
+    M, N, P = h.new_mueller(), h.new_mueller(), h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, N, precision=precision)
+    assert h.handle_orientations_to_local_gpu(b, P, precision=precision)
+    h.close()
+    gate = FP64_L2 if precision == abi.FP64 else 1e-4
+    assert _l2(M, M0) < gate
+    assert _l2(N, N0) < gate if external != "all" else not N.any()
+    if precision == abi.FP32C:
+        assert np.array_equal(M, P)
+    else:
+        assert np.max(np.abs(M - P)) <= 1.7e-13 * np.max(np.abs(P))
