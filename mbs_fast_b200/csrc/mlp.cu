@@ -6,7 +6,7 @@
 // operands in shared memory in the K-major no-swizzle layout (8 x 16-byte
 // core matrices), the accumulator in tensor memory, read back with tcgen05.ld.
 //
-// A training step is two kernels.  k_chain takes 32 samples per CTA through
+// A training step is two kernels.  k_chain takes 16 samples per CTA through
 // the whole forward and backward chain (activations stay in shared memory and
 // registers; one MMA chain per layer); k_update forms the weight gradients,
 // which sum over all samples, 16 columns per CTA, and applies Adam to them
@@ -19,7 +19,9 @@
 // The step's operations are small (59 MFLOP at 256 samples); what bounds it is
 // the chain of dependent passes.  As twenty launches (nine GEMMs and the
 // element-wise and reduction kernels between them) a step of 256 samples took
-// 134 us; now 21 us, of which the chain's kernel is 12.8 and the update's 7.7.
+// 134 us; as two with 32 samples per CTA 21 us; now, with 16, gelu and gelu'
+// from one erf and each kernel's prologue beside the one before
+// (programmatic dependent launch), 18 us.
 #include "mbs_mlp.h"
 
 #include <cuda_bf16.h>
@@ -53,10 +55,25 @@ __device__ __forceinline__ float gelu(float z)
     return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
 }
 
-__device__ __forceinline__ float gelu_grad(float z)
+// GELU and its derivative from one erf.
+__device__ __forceinline__ float gelu_both(float z, float &grad)
 {
-    return 0.5f * (1.0f + erff(z * 0.70710678118654752f))
-         + z * 0.39894228040143268f * expf(-0.5f * z * z);
+    const float e = 1.0f + erff(z * 0.70710678118654752f);
+    grad = 0.5f * e + z * 0.39894228040143268f * expf(-0.5f * z * z);
+    return 0.5f * z * e;
+}
+
+// Programmatic dependent launch: the next kernel of the stream may start its
+// prologue; nothing global is touched before grid_wait (the kernels before
+// have completed and their writes are visible then).
+__device__ __forceinline__ void grid_release()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void grid_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---- tcgen05 helpers --------------------------------------------------
@@ -191,15 +208,17 @@ __device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t *v)
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// ---- forward and backward chain of 32 samples ---------------------------
-constexpr int kRows = 32;            // samples per CTA
-constexpr int kChainThreads = 512;   // thread = (row, 8 consecutive columns)
+// ---- forward and backward chain of a CTA's samples -----------------------
+// Samples per CTA: 16 in training (a step has few samples, and the element-wise
+// work of a CTA is what its chain waits for), 32 in inference (each CTA loads
+// all weights).  Thread = (row, 8 consecutive columns).
+constexpr int kTrainRows = 16, kFwdRows = 32;
 constexpr int kAccStride = kH + 4;   // floats: 16-byte rows without bank conflicts
 // shared memory: A tile (rows 32..127 zero), input tile, weight operands,
 // FP32 accumulator tile, small arrays
 constexpr int cA = 0, cX = cA + 2 * kImg, cW1 = cX + kTile * kInPad * 2, cW2f = cW1 + kH * kInPad * 2;
-constexpr int cW3f = cW2f + 2 * kImg, cS = cW3f + 2 * kImg, cVec = cS + kRows * kAccStride * 4;
-constexpr int cBar = cVec + (4 * kH + 3 * kRows) * 4, cFwdEnd = cBar + 64;
+constexpr int cW3f = cW2f + 2 * kImg, cS = cW3f + 2 * kImg, cVec = cS + kFwdRows * kAccStride * 4;
+constexpr int cBar = cVec + (4 * kH + 3 * kFwdRows) * 4, cFwdEnd = cBar + 64;
 constexpr int cW3b = (cFwdEnd + 127) / 128 * 128, cW2b = cW3b + 2 * kImg;
 constexpr int kChainSmemFwd = cFwdEnd, kChainSmem = cW2b + 2 * kImg;
 static_assert(kChainSmem <= 227 * 1024, "shared memory of one CTA");
@@ -230,14 +249,16 @@ __device__ __forceinline__ void store_image(const unsigned char *sA, bf16 *img, 
     *reinterpret_cast<uint4 *>(dst + kmajor_off(col, k, kTile)) = *reinterpret_cast<const uint4 *>(v);
 }
 
-template <bool kTrain>
-__global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
+template <bool kTrain, int kRows>
+__global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
 {
+    constexpr int kChainThreads = 16 * kRows;
+    constexpr int kLaneRows = kRows < 32 ? kRows : 32;     // rows of a warp: its lanes split into column groups
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t sbase = smem_u32(sm);
     float *S = reinterpret_cast<float *>(sm + cS);
     float *sb = reinterpret_cast<float *>(sm + cVec);      // b1, b2, b3, w4
-    float *sy = sb + 4 * kH, *st = sy + kRows, *sdy = st + kRows;
+    float *sy = sb + 4 * kH, *st = sy + kFwdRows, *sdy = st + kFwdRows;
     const uint32_t bars = sbase + cBar;                    // [0] MMA, [1] w1f, w2f, [2] w3f, [3] w3b, w2b
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + cBar + 48);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -251,6 +272,17 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
         for (int i = 0; i < 4; ++i)
             mbar_init(bars + 8 * i);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    // zero the tiles' rows beyond the samples and the input's padding columns
+    for (int i = tid; i < 2 * kImg / 16; i += kChainThreads)
+        reinterpret_cast<uint4 *>(sm + cA)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < kTile * kInPad * 2 / 16; i += kChainThreads)
+        reinterpret_cast<uint4 *>(sm + cX)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (kTrain) {
+        grid_release();
+        grid_wait();
+    }
+    if (tid == 0) {
         mbar_expect(bars + 8, kH * kInPad * 2 + 2 * kImg);
         bulk_load(sbase + cW1, a.w.w1f, kH * kInPad * 2, bars + 8);
         bulk_load(sbase + cW2f, a.w.w2f, 2 * kImg, bars + 8);
@@ -262,13 +294,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             bulk_load(sbase + cW2b, a.w.w2b, 2 * kImg, bars + 24);
         }
     }
-    // zero the tiles' rows beyond the samples and the input's padding columns
-    for (int i = tid; i < 2 * kImg / 16; i += kChainThreads)
-        reinterpret_cast<uint4 *>(sm + cA)[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = tid; i < kTile * kInPad * 2 / 16; i += kChainThreads)
-        reinterpret_cast<uint4 *>(sm + cX)[i] = make_uint4(0u, 0u, 0u, 0u);
-    sb[tid] = a.params[tid < kH ? ob1 + tid : tid < 2 * kH ? ob2 + tid - kH
-                       : tid < 3 * kH ? ob3 + tid - 2 * kH : ow4 + tid - 3 * kH];
+    for (int i = tid; i < 4 * kH; i += kChainThreads)
+        sb[i] = a.params[i < kH ? ob1 + i : i < 2 * kH ? ob2 + i - kH : i < 3 * kH ? ob3 + i - 2 * kH : ow4 + i - 3 * kH];
     __syncthreads();
     if (tid < kRows) {
         const int r = r0 + tid;
@@ -323,20 +350,24 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             return;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if ((warp & 3) == 0) {   // rows 0..31: the lane quarter of warps 0, 4, 8 and 12
-            uint32_t v[32];
-            const int c0 = (warp >> 2) * 32;
-            tmem_ld32(tmem + (uint32_t)c0, v);
-            float4 *dst = reinterpret_cast<float4 *>(S + lane * kAccStride + c0);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                     __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+            for (int c0 = (warp >> 2) * 32; c0 < kH; c0 += kChainThreads / 4) {
+                uint32_t v[32];
+                tmem_ld32(tmem + (uint32_t)c0, v);
+                if (lane < kRows) {
+                    float4 *dst = reinterpret_cast<float4 *>(S + lane * kAccStride + c0);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+                }
+            }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();
     };
     // this thread's 8 accumulators of S, and the next layer's operand
-    const int row = lane, c0 = warp * 8;
+    const int row = lane & (kLaneRows - 1), c0 = (warp * (32 / kLaneRows) + lane / kLaneRows) * 8;
     auto acc8 = [&](float *v) {
         const float4 *p = reinterpret_cast<const float4 *>(S + row * kAccStride + c0);
         const float4 x = p[0], y = p[1];
@@ -352,32 +383,32 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     };
-    float z1[8], z2[8], z3[8], v[8];
-    auto forward = [&](float *z, int layer_no) {
+    float g1[8], g2[8], g3[8], v[8];   // gelu' of each layer
+    auto forward = [&](float *g, int layer_no) {
         acc8(v);
         float h[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            z[i] = v[i] + sb[layer_no * kH + c0 + i];
-            h[i] = gelu(z[i]);
+            const float z = v[i] + sb[layer_no * kH + c0 + i];
+            h[i] = kTrain ? gelu_both(z, g[i]) : gelu(z);
         }
         put8(h);
     };
     layer(cX, cW1, kInPad, 1);
     if (ok) {
-        forward(z1, 0);
+        forward(g1, 0);
         if (kTrain)
             store_image(sm + cA, a.img.h1, r0);
         layer(cA, cW2f, kH, 1);
     }
     if (ok) {
-        forward(z2, 1);
+        forward(g2, 1);
         if (kTrain)
             store_image(sm + cA, a.img.h2, r0);
         layer(cA, cW3f, kH, 2);
     }
     if (ok) {
-        forward(z3, 2);
+        forward(g3, 2);
         if (kTrain)
             store_image(sm + cA, a.img.h3, r0);
         // y = sum_j H3[j] w4[j] + b4: a warp per sample, fixed lane order
@@ -409,7 +440,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
         const float d = sdy[row];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            v[i] = d * sb[3 * kH + c0 + i] * gelu_grad(z3[i]);
+            v[i] = d * sb[3 * kH + c0 + i] * g3[i];
         put8(v);
         store_image(sm + cA, a.img.dz3, r0);
         layer(cA, cW3b, kH, 3);
@@ -417,7 +448,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             acc8(v);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                v[i] = v[i] * gelu_grad(z2[i]);
+                v[i] = v[i] * g2[i];
             put8(v);
             store_image(sm + cA, a.img.dz2, r0);
             layer(cA, cW2b, kH, 3);
@@ -426,7 +457,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             acc8(v);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                v[i] = v[i] * gelu_grad(z1[i]);
+                v[i] = v[i] * g1[i];
             put8(v);
             store_image(sm + cA, a.img.dz1, r0);
         }
@@ -528,6 +559,22 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int job = blockIdx.x;
     float bc1 = 0.f, bc2 = 0.f;
+    grid_release();
+    const uint32_t sbase = smem_u32(sm), bars = sbase + 2 * kUpStage;   // full[2], MMA[2]
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + 2 * kUpStage + 48);
+    if (job < kJobBias) {
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         :: "r"(smem_u32(tslot)), "r"(32));
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        }
+        if (tid == 0) {
+            for (int i = 0; i < 4; ++i)
+                mbar_init(bars + 8 * i);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+    }
+    grid_wait();
     if (kAdam) {
         const int j = (*a.epoch) * a.steps_per_epoch + a.k;
         bc1 = a.bc[2 * j];
@@ -575,18 +622,6 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     const bf16 *B = l == 3 ? a.img.h2 : l == 2 ? a.img.h1 : a.img.x0;
     const size_t bstep = l == 1 ? kImgX : kImg;
     B += n0 * kTile;         // 8 rows of an image are 8 * 128 consecutive elements
-    const uint32_t sbase = smem_u32(sm), bars = sbase + 2 * kUpStage;   // full[2], MMA[2]
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + 2 * kUpStage + 48);
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(tslot)), "r"(32));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    if (tid == 0) {
-        for (int i = 0; i < 4; ++i)
-            mbar_init(bars + 8 * i);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -839,8 +874,8 @@ int check_err(mbs_mlp *net)
 int set_attrs(mbs_mlp *net)
 {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    MK(cudaFuncSetAttribute(k_chain<false>, a, kChainSmemFwd), "kernel attributes");
-    MK(cudaFuncSetAttribute(k_chain<true>, a, kChainSmem), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_chain<false, kFwdRows>, a, kChainSmemFwd), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_chain<true, kTrainRows>, a, kChainSmem), "kernel attributes");
     MK(cudaFuncSetAttribute(k_update<false>, a, kUpSmem), "kernel attributes");
     MK(cudaFuncSetAttribute(k_update<true>, a, kUpSmem), "kernel attributes");
     return 0;
@@ -866,9 +901,28 @@ ChainArgs chain_args(mbs_mlp *net, int n)
 int forward_dev(mbs_mlp *net, int n)
 {
     const ChainArgs a = chain_args(net, n);
-    k_chain<false><<<(n + kRows - 1) / kRows, kChainThreads, kChainSmemFwd, net->stream>>>(a);
+    k_chain<false, kFwdRows><<<(n + kFwdRows - 1) / kFwdRows, 16 * kFwdRows, kChainSmemFwd, net->stream>>>(a);
     MK(cudaGetLastError(), "mlp forward launch");
     return 0;
+}
+
+// A launch whose prologue may overlap the kernel before it (grid_wait).
+template <typename Args>
+cudaError_t launch_dependent(cudaStream_t s, void (*kern)(Args), int grid, int threads, int smem, Args args)
+{
+    cudaLaunchAttribute at;
+    std::memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args);
 }
 
 // Forward and backward chain of a.n samples, then the gradients (adam false:
@@ -876,8 +930,8 @@ int forward_dev(mbs_mlp *net, int n)
 int step_dev(mbs_mlp *net, const ChainArgs &a, UpdateArgs u, bool use_adam)
 {
     const int bp = pad_rows(a.n);
-    k_chain<true><<<bp / kRows, kChainThreads, kChainSmem, net->stream>>>(a);
-    MK(cudaGetLastError(), "mlp chain launch");
+    MK(launch_dependent(net->stream, k_chain<true, kTrainRows>, bp / kTrainRows, 16 * kTrainRows, kChainSmem, a),
+       "mlp chain launch");
     u.img = net->img;
     u.dy = net->dy;
     u.bp = bp;
@@ -887,11 +941,8 @@ int step_dev(mbs_mlp *net, const ChainArgs &a, UpdateArgs u, bool use_adam)
     u.v = net->v;
     u.w = net->w;
     u.watch = watch(net);
-    if (use_adam)
-        k_update<true><<<kUpJobs, kUpThreads, kUpSmem, net->stream>>>(u);
-    else
-        k_update<false><<<kUpJobs, kUpThreads, kUpSmem, net->stream>>>(u);
-    MK(cudaGetLastError(), "mlp update launch");
+    MK(launch_dependent(net->stream, use_adam ? k_update<true> : k_update<false>, kUpJobs, kUpThreads, kUpSmem, u),
+       "mlp update launch");
     return 0;
 }
 
