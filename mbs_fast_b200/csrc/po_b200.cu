@@ -1764,14 +1764,20 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         tab[n + i] = std::cos(th);
     }
     const int nAz = ctx->grid.n_az;
-    // three points per thread where a tile of 192 is mostly used; beam chunks
-    // for about 16 CTAs per resident one, whole stages each
+    // Three points per thread where a tile of 192 is mostly used.  Beam chunks:
+    // as many equal CTAs as are resident at once (whole multiples of that for
+    // many beams, up to 8 stages a CTA), so that none wait for a second round;
+    // 64 beams a CTA whatever the batch made 2.7 rounds of 2,088 beams x 48
+    // azimuths.
     const int dpt = n > 2 * kThetaTpb ? 3 : 1;
     const int tiles = (n + dpt * kThetaTpb - 1) / (dpt * kThetaTpb);
-    int64_t chunks = std::max<int64_t>(1, (int64_t)148 * 4 * 16 / ((int64_t)tiles * nAz));
-    chunks = std::min<int64_t>(chunks, (s.n_beams + kThetaBeams - 1) / kThetaBeams);
-    int64_t bpc = (s.n_beams + chunks - 1) / chunks;
-    bpc = (bpc + kThetaBeams - 1) / kThetaBeams * kThetaBeams;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    const int64_t resident = (int64_t)sms * 4, columns = (int64_t)tiles * nAz;
+    const int64_t rounds = std::max<int64_t>(1, s.n_beams * columns / (resident * 8 * kThetaBeams));
+    int64_t chunks = std::max<int64_t>(1, resident * rounds / columns);
+    chunks = std::min<int64_t>(std::min<int64_t>(chunks, 65535), (s.n_beams + 15) / 16);
+    const int64_t bpc = (s.n_beams + chunks - 1) / chunks;
     chunks = (s.n_beams + bpc - 1) / bpc;
     const int64_t rows = chunks * nAz;
     // scratch from the context's pool: the partial sums take megabytes, and a

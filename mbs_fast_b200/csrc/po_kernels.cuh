@@ -2253,7 +2253,7 @@ __global__ void __launch_bounds__(256) po_csca_kernel(const double *__restrict__
 // candidates are marked and evaluated in general form after the stage.
 // Bound by the FP64 pipe.  One thread per (point, beam, azimuth) with the
 // general evaluation took 1,225 us for 2,088 beams x 48 x 181 points, now
-// 266 us.
+// 229 us.
 struct __align__(16) ThetaBeam {
     double a[6];        // A, B coefficients (see BeamRegs)
     double q[6];        // |P0|^2 2P0.Pc 2P0.Ps |Pc|^2 |Ps|^2 2Pc.Ps, times 0.5 weight / (n_az + 1)

@@ -323,3 +323,33 @@ def test_noshadow_sums(precision, external):
         assert np.array_equal(M, P)
     else:
         assert np.max(np.abs(M - P)) <= 1.7e-13 * np.max(np.abs(P))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_zen", [95, 383, 500])
+@pytest.mark.parametrize("precision", [abi.FP64, abi.FP32C])
+def test_row_tails_in_a_captured_graph(n_zen, precision):
+    """A tail alone, no FP32C tail, and a tail beside the main launch (side
+    stream forked and joined) in a captured call: its replays add what the
+    direct call adds, bit for bit."""
+    import torch
+    b, w = S.batch(5, 40, 12.0, 8), S.wave()
+    g = S.grid(6, n_zen)
+    h = GpuHandlerPO(g, w)
+    st = h.stage(b)
+    acc = torch.zeros(g.n_dirs * 16, dtype=torch.float64, device="cuda:0")
+    h.diffract_staged(st, acc.data_ptr(), precision=precision)
+    torch.cuda.synchronize()
+    want = acc.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        h.diffract_staged(st, acc.data_ptr(), precision=precision,
+                          stream=torch.cuda.current_stream().cuda_stream, stats=False)
+    for _ in range(2):
+        acc.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(acc, want)
+    del graph
+    st.free()
+    h.close()
