@@ -353,3 +353,33 @@ def test_row_tails_in_a_captured_graph(n_zen, precision):
     del graph
     st.free()
     h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("beams", [3, 700, 2600])
+def test_small_uploads_and_results_in_parts(beams):
+    """Batches below and above the size that goes up as one image (with size
+    instances and absorption paths too), and results of one to eight parts,
+    with the boundary of the two sets inside a part; calls in turn on one
+    context, so each finds the buffers as the last one left them."""
+    b, w = S.batch(2, beams, 8.0, 44, raw=True, absorbing=True), S.wave(True)
+    rng = np.random.default_rng(beams)
+    for n_az, n_zen in ((3, 10), (7, 400), (37, 800)):
+        g = S.grid(n_az, n_zen)
+        h = GpuHandlerPO(g, w)
+        add, add_ns = h.diffract_pinned(b, noshadow=True, precision=abi.FP64)
+        M, N = rng.normal(size=add.shape), rng.normal(size=add.shape)
+        want, want_ns = M + add, N + add_ns
+        assert h.handle_orientations_to_local_gpu(b, M, N, precision=abi.FP64)
+        assert np.array_equal(M, want) and np.array_equal(N, want_ns)
+        if n_az == 3:
+            assert _l2(add, oracle.po_diffract(b, g, w)) < FP64_L2
+            ms = [h.new_mueller(), h.new_mueller()]
+            assert h.handle_orientations_to_local_gpu_multik(b, 0, 2, [0.7, 1.6], w.wave_index, ms)
+            for s, m in zip((0.7, 1.6), ms):
+                assert _l2(m, oracle.po_diffract(oracle.scale_batch(b, s, w.wave_index, w.abs_coeff), g, w)) < FP64_L2
+            one = b.select(1, 1)
+            P = h.new_mueller()
+            assert h.handle_orientations_to_local_gpu(one, P, precision=abi.FP64)
+            assert _l2(P, oracle.po_diffract(one, g, w)) < FP64_L2
+        h.close()
