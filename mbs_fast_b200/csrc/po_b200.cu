@@ -58,7 +58,7 @@ constexpr Variant kVariantsF64[] = {{64, 3, 4}, {128, 1, 3}, {96, 2, 4}, {128, 1
 constexpr Variant kNoShadowF32 = {128, 3, 3};
 constexpr Variant kNoShadowF64 = {128, 1, 3};
 // Shapes for the rows past the last whole tile (see row_tail).
-constexpr Variant kTailF32[] = {{128, 1, 4}, {128, 2, 4}};
+constexpr Variant kTailF32[] = {{128, 1, 4}, {128, 2, 3}};
 constexpr Variant kTailF64[] = {{64, 1, 6}, {128, 1, 4}};
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
@@ -874,7 +874,7 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // holds them: index into kTail*, or -1.  A thread whose slots lie past the
 // last row still evaluates them.  Time of a tail tile against a whole one
 // (64 orientations of 87 beams, 48 azimuths): FP32C 128 rows 0.50, 256 rows
-// 0.81; FP64 64 rows 0.45, 128 rows 0.76.  The tail shapes stage the same
+// 0.77 (0.81 with four CTAs per SM and spills); FP64 64 rows 0.45, 128 rows 0.76.  The tail shapes stage the same
 // beams at a time as the default ones, so a direction's sums are the same
 // bit for bit whichever launch holds it.
 int row_tail(int pi, int n_t)
@@ -892,7 +892,7 @@ cudaError_t launch_tail(int pi, int tail, const KParams &P, cudaStream_t st)
 {
     if (pi == 0)
         return tail == 0 ? launch_one<double, 64, 1, false, 6>(P, st) : launch_one<double, 128, 1, false, 4>(P, st);
-    return tail == 0 ? launch_one<float, 128, 1, false, 4>(P, st) : launch_one<float, 128, 2, false, 4>(P, st);
+    return tail == 0 ? launch_one<float, 128, 1, false, 4>(P, st) : launch_one<float, 128, 2, false, 3>(P, st);
 }
 
 // The rows of a call: [0, main_rows) in the chosen shape, the rest (`tail` >= 0)

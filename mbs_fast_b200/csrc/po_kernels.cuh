@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kPackThreads) po_pack_kernel(PackParams P)
     const double k = wc.k, kt = wc.k * kInvTwoPi;
     const bool has = il < nb;
     const double *g = sg + (has ? il : 0) * MBS_PO_GEOM_STRIDE;
-    const int64_t bl = bl0 + (has ? il : 0), b = ob + bl;
+    const int64_t bl = bl0 + (has ? il : 0);
     const int vo = svo[has ? il : 0], nv = svo[has ? il + 1 : 1] - vo;
     // a0 = bd.hor, b0 = bd.ver (GpuDiffraction.cu:301-302)
     const double a0 = g[MBS_PO_G_BD] * g[MBS_PO_G_HOR] + g[MBS_PO_G_BD + 1] * g[MBS_PO_G_HOR + 1]
