@@ -21,7 +21,8 @@
 // element-wise and reduction kernels between them) a step of 256 samples took
 // 134 us; as two with 32 samples per CTA 21 us; now, with 16, gelu and gelu'
 // from one erf and each kernel's prologue beside the one before
-// (programmatic dependent launch), 18 us.
+// (programmatic dependent launch), 18 us; with the epoch's samples laid out in
+// its shuffled order and the Adam state loaded under the products, 16 us.
 #include "mbs_mlp.h"
 
 #include <cuda_bf16.h>
@@ -185,48 +186,48 @@ __device__ __forceinline__ void mma_chain(uint32_t tmem, uint32_t a, uint32_t b,
                  :: "r"(bar) : "memory");
 }
 
-// 32 (or 8) accumulator columns of the warp's 32 tensor-memory lanes.
-__device__ __forceinline__ void tmem_ld32(uint32_t ta, uint32_t *v)
+// N accumulator columns (4 or 8) of the warp's 32 tensor-memory lanes.
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t ta, float *f)
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                   "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
-                   "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
-                   "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(ta));
+    uint32_t v[N];
+    if constexpr (N == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "r"(ta));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(ta));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t ta, uint32_t *v)
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(ta));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        f[i] = __uint_as_float(v[i]);
 }
 
 // ---- forward and backward chain of a CTA's samples -----------------------
 // Samples per CTA: 16 in training (a step has few samples, and the element-wise
 // work of a CTA is what its chain waits for), 32 in inference (each CTA loads
-// all weights).  Thread = (row, 8 consecutive columns).
+// all weights).  The weights are the M = 128 operand and the samples the N
+// operand, so an accumulator row is a unit of the layer (tensor-memory lane)
+// and its columns are the samples: every warp reads its lane quarter straight
+// into registers, and a unit's consecutive samples are what the images hold.
+// (Samples as the M operand filled 16 of 128 rows, eight times the MMA time,
+// and their accumulators went through shared memory twice per layer.)
 constexpr int kTrainRows = 16, kFwdRows = 32;
-constexpr int kAccStride = kH + 4;   // floats: 16-byte rows without bank conflicts
-// shared memory: A tile (rows 32..127 zero), input tile, weight operands,
-// FP32 accumulator tile, small arrays
-constexpr int cA = 0, cX = cA + 2 * kImg, cW1 = cX + kTile * kInPad * 2, cW2f = cW1 + kH * kInPad * 2;
-constexpr int cW3f = cW2f + 2 * kImg, cS = cW3f + 2 * kImg, cVec = cS + kFwdRows * kAccStride * 4;
-constexpr int cBar = cVec + (4 * kH + 3 * kFwdRows) * 4, cFwdEnd = cBar + 64;
-constexpr int cW3b = (cFwdEnd + 127) / 128 * 128, cW2b = cW3b + 2 * kImg;
-constexpr int kChainSmemFwd = cFwdEnd, kChainSmem = cW2b + 2 * kImg;
-static_assert(kChainSmem <= 227 * 1024, "shared memory of one CTA");
+constexpr int kChainThreads = 512;   // warp = (lane quarter of the units, a quarter of the samples)
+
+// shared memory: weight operands, sample tile, input tile, small arrays
+template <bool kTrain, int kRows>
+struct ChainSmem {
+    static constexpr int W1 = 0, W2f = W1 + kH * kInPad * 2, W3f = W2f + 2 * kImg;
+    static constexpr int W3b = W3f + 2 * kImg, W2b = W3b + (kTrain ? 2 * kImg : 0);
+    static constexpr int H = W2b + (kTrain ? 2 * kImg : 0), X = H + kRows * kH * 2;
+    static constexpr int vec = X + kRows * kInPad * 2, bar = vec + (4 * kH + 3 * kRows) * 4, bytes = bar + 64;
+};
+static_assert(ChainSmem<true, kTrainRows>::bytes <= 227 * 1024, "shared memory of one CTA");
 
 struct ChainArgs {
-    const float *q, *t;      // samples [..][4] and targets
-    const int *idx, *epoch;  // null, or the shuffled order [epoch][n_set] and the epoch counter
-    int n_set, b0;           // samples of the set, offset of this batch in the epoch
+    const float *q, *t;      // samples [n][4] and targets
     int n;                   // samples of this batch; the rows beyond are padding
     const float *params;
     Weights w;
@@ -235,37 +236,23 @@ struct ChainArgs {
     Watch watch;
 };
 
-// The A tile's transpose (row = column of the layer, k = sample) into the
-// samples' 32 k of an image: thread = (column, 8 samples).
-__device__ __forceinline__ void store_image(const unsigned char *sA, bf16 *img, int r0)
-{
-    const int col = threadIdx.x & (kH - 1), rg = threadIdx.x >> 7;
-    const int k = (r0 & (kTile - 1)) + rg * 8;
-    __align__(16) bf16 v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        v[i] = *reinterpret_cast<const bf16 *>(sA + kmajor_off(rg * 8 + i, col, kTile));
-    unsigned char *dst = reinterpret_cast<unsigned char *>(img + (size_t)(r0 / kTile) * kImg);
-    *reinterpret_cast<uint4 *>(dst + kmajor_off(col, k, kTile)) = *reinterpret_cast<const uint4 *>(v);
-}
-
 template <bool kTrain, int kRows>
-__global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
+__global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
 {
-    constexpr int kChainThreads = 16 * kRows;
-    constexpr int kLaneRows = kRows < 32 ? kRows : 32;     // rows of a warp: its lanes split into column groups
+    using L = ChainSmem<kTrain, kRows>;
+    constexpr int kV = kRows / 4;                          // samples of a thread
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t sbase = smem_u32(sm);
-    float *S = reinterpret_cast<float *>(sm + cS);
-    float *sb = reinterpret_cast<float *>(sm + cVec);      // b1, b2, b3, w4
-    float *sy = sb + 4 * kH, *st = sy + kFwdRows, *sdy = st + kFwdRows;
-    const uint32_t bars = sbase + cBar;                    // [0] MMA, [1] w1f, w2f, [2] w3f, [3] w3b, w2b
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + cBar + 48);
+    float *sb = reinterpret_cast<float *>(sm + L::vec);    // b1, b2, b3, w4
+    float *st = sb + 4 * kH, *sdy = st + kRows;
+    const uint32_t bars = sbase + L::bar;                  // [0] MMA, [1] w1f, w2f, [2] w3f, [3] w3b, w2b
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + L::bar + 48);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r0 = blockIdx.x * kRows;
+    const int unit = (warp & 3) * 32 + lane, s0 = (warp >> 2) * kV;   // this thread's accumulators
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(tslot)), "r"(kH));
+                     :: "r"(smem_u32(tslot)), "r"(32));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
@@ -273,75 +260,59 @@ __global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
             mbar_init(bars + 8 * i);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    // zero the tiles' rows beyond the samples and the input's padding columns
-    for (int i = tid; i < 2 * kImg / 16; i += kChainThreads)
-        reinterpret_cast<uint4 *>(sm + cA)[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = tid; i < kTile * kInPad * 2 / 16; i += kChainThreads)
-        reinterpret_cast<uint4 *>(sm + cX)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (kTrain) {
         grid_release();
         grid_wait();
     }
     if (tid == 0) {
         mbar_expect(bars + 8, kH * kInPad * 2 + 2 * kImg);
-        bulk_load(sbase + cW1, a.w.w1f, kH * kInPad * 2, bars + 8);
-        bulk_load(sbase + cW2f, a.w.w2f, 2 * kImg, bars + 8);
+        bulk_load(sbase + L::W1, a.w.w1f, kH * kInPad * 2, bars + 8);
+        bulk_load(sbase + L::W2f, a.w.w2f, 2 * kImg, bars + 8);
         mbar_expect(bars + 16, 2 * kImg);
-        bulk_load(sbase + cW3f, a.w.w3f, 2 * kImg, bars + 16);
+        bulk_load(sbase + L::W3f, a.w.w3f, 2 * kImg, bars + 16);
         if (kTrain) {
             mbar_expect(bars + 24, 4 * kImg);
-            bulk_load(sbase + cW3b, a.w.w3b, 2 * kImg, bars + 24);
-            bulk_load(sbase + cW2b, a.w.w2b, 2 * kImg, bars + 24);
+            bulk_load(sbase + L::W3b, a.w.w3b, 2 * kImg, bars + 24);
+            bulk_load(sbase + L::W2b, a.w.w2b, 2 * kImg, bars + 24);
         }
     }
-    for (int i = tid; i < 4 * kH; i += kChainThreads)
-        sb[i] = a.params[i < kH ? ob1 + i : i < 2 * kH ? ob2 + i - kH : i < 3 * kH ? ob3 + i - 2 * kH : ow4 + i - 3 * kH];
-    __syncthreads();
-    if (tid < kRows) {
+    if (tid < kRows) {   // a sample's input row: the quaternion, zeros to 16 columns
         const int r = r0 + tid;
         float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
         float tv = 0.f;
         if (r < a.n) {
-            const int s = a.idx ? a.idx[(size_t)(*a.epoch) * a.n_set + a.b0 + r] : r;
-            qv = make_float4(a.q[s * kIn], a.q[s * kIn + 1], a.q[s * kIn + 2], a.q[s * kIn + 3]);
+            qv = make_float4(a.q[r * kIn], a.q[r * kIn + 1], a.q[r * kIn + 2], a.q[r * kIn + 3]);
             if (kTrain)
-                tv = a.t[s];
+                tv = a.t[r];
         }
         st[tid] = tv;
-        const bf16 v[4] = {__float2bfloat16(qv.x), __float2bfloat16(qv.y), __float2bfloat16(qv.z),
-                           __float2bfloat16(qv.w)};
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<bf16 *>(sm + cX + kmajor_off(tid, c, kInPad)) = v[c];
+        const bf16 z = __float2bfloat16(0.f);
+        __align__(16) const bf16 v[8] = {__float2bfloat16(qv.x), __float2bfloat16(qv.y), __float2bfloat16(qv.z),
+                                         __float2bfloat16(qv.w), z, z, z, z};
+        *reinterpret_cast<uint4 *>(sm + L::X + kmajor_off(tid, 0, kInPad)) = *reinterpret_cast<const uint4 *>(v);
+        *reinterpret_cast<uint4 *>(sm + L::X + kmajor_off(tid, 8, kInPad)) = make_uint4(0u, 0u, 0u, 0u);
     }
+    for (int i = tid; i < 4 * kH; i += kChainThreads)
+        sb[i] = a.params[i < kH ? ob1 + i : i < 2 * kH ? ob2 + i - kH : i < 3 * kH ? ob3 + i - 2 * kH : ow4 + i - 3 * kH];
+    const float b4 = a.params[ob4];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
-    if (kTrain && tid < kInPad * (kRows / 8)) {   // the input's image: (column, 8 samples)
-        const int col = tid & (kInPad - 1), rg = tid / kInPad;
-        __align__(16) bf16 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            v[i] = *reinterpret_cast<const bf16 *>(sm + cX + kmajor_off(rg * 8 + i, col, kInPad));
-        unsigned char *dst = reinterpret_cast<unsigned char *>(a.img.x0 + (size_t)(r0 / kTile) * kImgX);
-        *reinterpret_cast<uint4 *>(dst + kmajor_off(col, (r0 & (kTile - 1)) + rg * 8, kTile)) =
-            *reinterpret_cast<const uint4 *>(v);
-    }
     bool ok = true;
     uint32_t phase = 0;
     int loaded = 0;            // weight barriers waited for so far
-    // One layer product on the staged A tile, its accumulators as FP32 rows
-    // in S.  `wbar`: the barrier of the weight operand.
-    auto layer = [&](int aoff, int boff, int kt, int wbar) {
+    // One layer product W (128 x kt) times the staged samples: this thread's
+    // accumulators.  `wbar`: the barrier of the weight operand.
+    auto layer = [&](int woff, int soff, int kt, int wbar, float *v) {
         if (tid == 0 && ok) {
             while (loaded < wbar && ok) {
                 ++loaded;
                 ok = mbar_wait(bars + 8 * loaded, 0, kDefaultPollLimit);
             }
             if (ok && !a.watch.skip_mma)
-                mma_chain(tmem, sbase + aoff, sbase + boff, kt, kH, false, bars);
+                mma_chain(tmem, sbase + woff, sbase + soff, kt, kRows, false, bars);
         }
         const bool done = mbar_wait(bars, phase, a.watch.poll_limit);
         phase ^= 1u;
@@ -349,81 +320,71 @@ __global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
         if (!ok)
             return;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        if ((warp & 3) == 0) {   // rows 0..31: the lane quarter of warps 0, 4, 8 and 12
-#pragma unroll
-            for (int c0 = (warp >> 2) * 32; c0 < kH; c0 += kChainThreads / 4) {
-                uint32_t v[32];
-                tmem_ld32(tmem + (uint32_t)c0, v);
-                if (lane < kRows) {
-                    float4 *dst = reinterpret_cast<float4 *>(S + lane * kAccStride + c0);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                             __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-                }
-            }
-        }
+        tmem_ld<kV>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)s0, v);
         asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncthreads();
     };
-    // this thread's 8 accumulators of S, and the next layer's operand
-    const int row = lane & (kLaneRows - 1), c0 = (warp * (32 / kLaneRows) + lane / kLaneRows) * 8;
-    auto acc8 = [&](float *v) {
-        const float4 *p = reinterpret_cast<const float4 *>(S + row * kAccStride + c0);
-        const float4 x = p[0], y = p[1];
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-    };
-    auto put8 = [&](const float *v) {
-        __align__(16) bf16 h[8];
+    // This thread's values of a layer, BF16: into the sample tile (the next
+    // product's operand) and, in training, into an image.
+    auto put = [&](const float *v, bf16 *img, bool tile) {
+        __align__(16) bf16 h[kV];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < kV; ++i) {
             h[i] = __float2bfloat16(v[i]);
-        *reinterpret_cast<uint4 *>(sm + cA + kmajor_off(row, c0, kTile)) = *reinterpret_cast<const uint4 *>(h);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
+            if (tile)
+                *reinterpret_cast<bf16 *>(sm + L::H + kmajor_off(s0 + i, unit, kTile)) = h[i];
+        }
+        if (kTrain) {
+            unsigned char *dst = reinterpret_cast<unsigned char *>(img + (size_t)(r0 / kTile) * kImg)
+                               + kmajor_off(unit, (r0 & (kTile - 1)) + s0, kTile);
+            if constexpr (kV == 4)
+                *reinterpret_cast<uint2 *>(dst) = *reinterpret_cast<const uint2 *>(h);
+            else
+                *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
+        }
+        if (tile) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
     };
-    float g1[8], g2[8], g3[8], v[8];   // gelu' of each layer
-    auto forward = [&](float *g, int layer_no) {
-        acc8(v);
-        float h[8];
+    float g1[kV], g2[kV], g3[kV], v[kV];   // gelu' of each layer
+    auto forward = [&](float *g, int layer_no, bf16 *img) {
+        const float bias = sb[layer_no * kH + unit];
+        float h[kV];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float z = v[i] + sb[layer_no * kH + c0 + i];
+        for (int i = 0; i < kV; ++i) {
+            const float z = v[i] + bias;
             h[i] = kTrain ? gelu_both(z, g[i]) : gelu(z);
         }
-        put8(h);
+        put(h, img, true);
     };
-    layer(cX, cW1, kInPad, 1);
+    auto backward = [&](const float *g, bf16 *img, bool tile) {
+#pragma unroll
+        for (int i = 0; i < kV; ++i)
+            v[i] = v[i] * g[i];
+        put(v, img, tile);
+    };
+    layer(L::W1, L::X, kInPad, 1, v);
     if (ok) {
-        forward(g1, 0);
-        if (kTrain)
-            store_image(sm + cA, a.img.h1, r0);
-        layer(cA, cW2f, kH, 1);
+        forward(g1, 0, a.img.h1);
+        layer(L::W2f, L::H, kH, 1, v);
     }
     if (ok) {
-        forward(g2, 1);
-        if (kTrain)
-            store_image(sm + cA, a.img.h2, r0);
-        layer(cA, cW3f, kH, 2);
+        forward(g2, 1, a.img.h2);
+        layer(L::W3f, L::H, kH, 2, v);
     }
     if (ok) {
-        forward(g3, 2);
-        if (kTrain)
-            store_image(sm + cA, a.img.h3, r0);
+        forward(g3, 2, a.img.h3);
         // y = sum_j H3[j] w4[j] + b4: a warp per sample, fixed lane order
-        const float b4 = a.params[ob4];
         for (int r = warp; r < kRows; r += kChainThreads / 32) {
             float s = 0.f;
             for (int j = lane; j < kH; j += 32)
-                s = fmaf(__bfloat162float(*reinterpret_cast<const bf16 *>(sm + cA + kmajor_off(r, j, kTile))),
+                s = fmaf(__bfloat162float(*reinterpret_cast<const bf16 *>(sm + L::H + kmajor_off(r, j, kTile))),
                          sb[3 * kH + j], s);
 #pragma unroll
             for (int w = 16; w > 0; w >>= 1)
                 s += __shfl_xor_sync(0xffffffffu, s, w);
             if (lane == 0) {
                 const float yv = s + b4;
-                sy[r] = yv;
                 if (r0 + r < a.n)
                     a.y[r0 + r] = yv;
                 // dy = 2 (y - t) / n (0 on padding rows)
@@ -437,29 +398,27 @@ __global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
     }
     if (kTrain && ok) {
         // dZ3 = dy w4 gelu'(Z3), dZ2 = (dZ3 W3) gelu'(Z2), dZ1 = (dZ2 W2) gelu'(Z1)
-        const float d = sdy[row];
+        const float w4 = sb[3 * kH + unit];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            v[i] = d * sb[3 * kH + c0 + i] * g3[i];
-        put8(v);
-        store_image(sm + cA, a.img.dz3, r0);
-        layer(cA, cW3b, kH, 3);
+        for (int i = 0; i < kV; ++i)
+            v[i] = sdy[s0 + i] * w4;
+        backward(g3, a.img.dz3, true);
+        layer(L::W3b, L::H, kH, 3, v);
         if (ok) {
-            acc8(v);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                v[i] = v[i] * g2[i];
-            put8(v);
-            store_image(sm + cA, a.img.dz2, r0);
-            layer(cA, cW2b, kH, 3);
+            backward(g2, a.img.dz2, true);
+            layer(L::W2b, L::H, kH, 3, v);
         }
-        if (ok) {
-            acc8(v);
+        if (ok)
+            backward(g1, a.img.dz1, false);
+        if (tid < kInPad * (kRows / 8)) {   // the input's image: (column, 8 samples)
+            const int col = tid & (kInPad - 1), rg = tid / kInPad;
+            __align__(16) bf16 x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                v[i] = v[i] * g1[i];
-            put8(v);
-            store_image(sm + cA, a.img.dz1, r0);
+                x[i] = *reinterpret_cast<const bf16 *>(sm + L::X + kmajor_off(rg * 8 + i, col, kInPad));
+            unsigned char *dst = reinterpret_cast<unsigned char *>(a.img.x0 + (size_t)(r0 / kTile) * kImgX);
+            *reinterpret_cast<uint4 *>(dst + kmajor_off(col, (r0 & (kTile - 1)) + rg * 8, kTile)) =
+                *reinterpret_cast<const uint4 *>(x);
         }
     }
     if (!ok && tid == 0) {
@@ -471,7 +430,7 @@ __global__ void __launch_bounds__(16 * kRows, 1) k_chain(ChainArgs a)
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kH));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(32));
 }
 
 // ---- weight gradients and Adam -------------------------------------------
@@ -489,47 +448,55 @@ struct UpdateArgs {
     Watch watch;
 };
 
-// Adam on N consecutive parameters (N = 4 or 8: vector loads, all issued
-// before the first store) with the step's bias corrections; p receives the
-// updated parameters.
+// Adam state of N consecutive parameters (N = 4 or 8: vector accesses): loaded
+// while the gradients are still being formed, then updated with the step's
+// bias corrections and stored.
 template <int N>
-__device__ __forceinline__ void adam(const UpdateArgs &a, int i, const float *g, float bc1, float bc2, float *p)
-{
-    __align__(16) float m[N], v[N];
-    if (N % 4 == 0) {
+struct AdamState {
+    float m[N], v[N], p[N];
+    __device__ __forceinline__ void load(const UpdateArgs &a, int i)
+    {
+        if constexpr (N % 4 == 0) {
 #pragma unroll
-        for (int k = 0; k < N; k += 4) {
-            *reinterpret_cast<float4 *>(m + k) = *reinterpret_cast<const float4 *>(a.m + i + k);
-            *reinterpret_cast<float4 *>(v + k) = *reinterpret_cast<const float4 *>(a.v + i + k);
-            *reinterpret_cast<float4 *>(p + k) = *reinterpret_cast<const float4 *>(a.p + i + k);
+            for (int k = 0; k < N; k += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(a.m + i + k);
+                const float4 y = *reinterpret_cast<const float4 *>(a.v + i + k);
+                const float4 z = *reinterpret_cast<const float4 *>(a.p + i + k);
+                m[k] = x.x; m[k + 1] = x.y; m[k + 2] = x.z; m[k + 3] = x.w;
+                v[k] = y.x; v[k + 1] = y.y; v[k + 2] = y.z; v[k + 3] = y.w;
+                p[k] = z.x; p[k + 1] = z.y; p[k + 2] = z.z; p[k + 3] = z.w;
+            }
+        } else {
+            m[0] = a.m[i];
+            v[0] = a.v[i];
+            p[0] = a.p[i];
         }
-    } else {
-        m[0] = a.m[i];
-        v[0] = a.v[i];
-        p[0] = a.p[i];
     }
+    __device__ __forceinline__ void step(const UpdateArgs &a, int i, const float *g, float bc1, float bc2)
+    {
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const float gi = g[k];
-        const float mi = 0.9f * m[k] + 0.1f * gi;
-        const float vi = 0.999f * v[k] + 0.001f * gi * gi;
-        m[k] = mi;
-        v[k] = vi;
-        p[k] = p[k] - a.lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
-    }
-    if (N % 4 == 0) {
-#pragma unroll
-        for (int k = 0; k < N; k += 4) {
-            *reinterpret_cast<float4 *>(a.m + i + k) = *reinterpret_cast<const float4 *>(m + k);
-            *reinterpret_cast<float4 *>(a.v + i + k) = *reinterpret_cast<const float4 *>(v + k);
-            *reinterpret_cast<float4 *>(a.p + i + k) = *reinterpret_cast<const float4 *>(p + k);
+        for (int k = 0; k < N; ++k) {
+            const float gi = g[k];
+            const float mi = 0.9f * m[k] + 0.1f * gi;
+            const float vi = 0.999f * v[k] + 0.001f * gi * gi;
+            m[k] = mi;
+            v[k] = vi;
+            p[k] = p[k] - a.lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
         }
-    } else {
-        a.m[i] = m[0];
-        a.v[i] = v[0];
-        a.p[i] = p[0];
+        if constexpr (N % 4 == 0) {
+#pragma unroll
+            for (int k = 0; k < N; k += 4) {
+                *reinterpret_cast<float4 *>(a.m + i + k) = make_float4(m[k], m[k + 1], m[k + 2], m[k + 3]);
+                *reinterpret_cast<float4 *>(a.v + i + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+                *reinterpret_cast<float4 *>(a.p + i + k) = make_float4(p[k], p[k + 1], p[k + 2], p[k + 3]);
+            }
+        } else {
+            a.m[i] = m[0];
+            a.v[i] = v[0];
+            a.p[i] = p[0];
+        }
     }
-}
+};
 
 // CTAs: 8 of 16 columns each for dW3 = dZ3^T H2 and dW2 = dZ2^T H1, one for
 // dW1 = dZ1^T X0, then the vectors, 32 entries a CTA: db3, db2, db1 (column
@@ -559,6 +526,13 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int job = blockIdx.x;
     float bc1 = 0.f, bc2 = 0.f;
+    auto corrections = [&]() {
+        if (kAdam) {
+            const int j = (*a.epoch) * a.steps_per_epoch + a.k;
+            bc1 = a.bc[2 * j];
+            bc2 = a.bc[2 * j + 1];
+        }
+    };
     grid_release();
     const uint32_t sbase = smem_u32(sm), bars = sbase + 2 * kUpStage;   // full[2], MMA[2]
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + 2 * kUpStage + 48);
@@ -575,11 +549,6 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         }
     }
     grid_wait();
-    if (kAdam) {
-        const int j = (*a.epoch) * a.steps_per_epoch + a.k;
-        bc1 = a.bc[2 * j];
-        bc2 = a.bc[2 * j + 1];
-    }
     if (job >= kJobBias) {
         // vectors: 8 row groups g take rows g, g + 8, ... in turn, the group
         // sums are added in group order
@@ -603,14 +572,18 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
             }
         }
         part[g][lane] = s;
+        AdamState<1> ad;
+        if (g == 0 && idx >= 0 && kAdam) {
+            corrections();
+            ad.load(a, idx);
+        }
         __syncthreads();
         if (g == 0 && idx >= 0) {
             float t = part[0][lane];
             for (int k = 1; k < 8; ++k)
                 t += part[k][lane];
-            float p[1];
             if (kAdam)
-                adam<1>(a, idx, &t, bc1, bc2, p);
+                ad.step(a, idx, &t, bc1, bc2);
             else
                 a.grad[idx] = t;
         }
@@ -626,19 +599,33 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
+    const int nblk = a.bp / kTile;
+    int issued = 0, waited = 0, committed = 0;
+    auto load = [&]() {
+        const uint32_t d = sbase + (issued & 1) * kUpStage, bar = bars + 8 * (issued & 1);
+        mbar_expect(bar, kUpStage);
+        bulk_load(d, A + (size_t)issued * kImg, 2 * kImg, bar);
+        bulk_load(d + 2 * kImg, B + (size_t)issued * bstep, kUpN * kTile * 2, bar);
+        ++issued;
+    };
     if (tid == 0) {
-        const int nblk = a.bp / kTile;
-        int issued = 0, waited = 0, committed = 0;
-        auto load = [&]() {
-            const uint32_t d = sbase + (issued & 1) * kUpStage, bar = bars + 8 * (issued & 1);
-            mbar_expect(bar, kUpStage);
-            bulk_load(d, A + (size_t)issued * kImg, 2 * kImg, bar);
-            bulk_load(d + 2 * kImg, B + (size_t)issued * bstep, kUpN * kTile * 2, bar);
-            ++issued;
-        };
         load();
         if (nblk > 1)
             load();
+    }
+    // accumulator rows 32 (w % 4) .. + 31 (the warp's lane quarter), columns
+    // 8 (w / 4) .. + 7; their Adam state comes while the products run
+    const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 8, c = n0 + cl;
+    AdamState<8> ad;
+    AdamState<4> ad1;
+    if (kAdam) {
+        corrections();
+        if (l != 1)
+            ad.load(a, (l == 3 ? oW3 : oW2) + r * kH + c);
+        else if (cl == 0)
+            ad1.load(a, oW1 + r * kIn);
+    }
+    if (tid == 0) {
         bool ok = true;
         for (int i = 0; i < nblk && ok; ++i) {
             ok = mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, kDefaultPollLimit);
@@ -670,38 +657,31 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     __syncthreads();
     if (s_ok) {
         asm volatile("tcgen05.fence::after_thread_sync;");
-        // warp w: accumulator rows 32 (w % 4) .. + 31 (its lane quarter),
-        // columns 8 (w / 4) .. + 7
-        const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 8;
-        uint32_t u[8];
-        tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cl, u);
-        __align__(16) float gv[8], pv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            gv[i] = __uint_as_float(u[i]);
+        __align__(16) float gv[8];
+        tmem_ld<8>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cl, gv);
         if (l == 1) {
             if (cl == 0) {
                 const int i0 = oW1 + r * kIn;
                 if (kAdam) {
-                    adam<kIn>(a, i0, gv, bc1, bc2, pv);
+                    ad1.step(a, i0, gv, bc1, bc2);
 #pragma unroll
-                    for (int c = 0; c < kIn; ++c)
+                    for (int k = 0; k < kIn; ++k)
                         *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(a.w.w1f)
-                                                  + kmajor_off(r, c, kInPad)) = __float2bfloat16(pv[c]);
+                                                  + kmajor_off(r, k, kInPad)) = __float2bfloat16(ad1.p[k]);
                 } else {
                     *reinterpret_cast<float4 *>(a.grad + i0) = *reinterpret_cast<const float4 *>(gv);
                 }
             }
         } else {
-            const int c = n0 + cl, i0 = (l == 3 ? oW3 : oW2) + r * kH + c;
+            const int i0 = (l == 3 ? oW3 : oW2) + r * kH + c;
             if (kAdam) {
                 unsigned char *wf = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3f : a.w.w2f);
                 unsigned char *wb = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3b : a.w.w2b);
                 __align__(16) bf16 h[8];
-                adam<8>(a, i0, gv, bc1, bc2, pv);
+                ad.step(a, i0, gv, bc1, bc2);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    h[i] = __float2bfloat16(pv[i]);
+                    h[i] = __float2bfloat16(ad.p[i]);
                 *reinterpret_cast<uint4 *>(wf + kmajor_off(r, c, kTile)) = *reinterpret_cast<const uint4 *>(h);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -759,10 +739,21 @@ __global__ void __launch_bounds__(256) k_loss(const float *y, const float *t, in
         *out = red[0] / (float)max(n, 1);
 }
 
-// End of a captured epoch: the epoch counter moves on.
-__global__ void k_next_epoch(int *epoch)
+// Start of a captured epoch: the epoch counter moves on (it starts at -1) and
+// the samples are laid out in the epoch's shuffled order idx[epoch][n], so the
+// steps read theirs without a chain of dependent loads.
+__global__ void __launch_bounds__(1024) k_epoch(const float4 *q, const float *t, const int *idx, int n, int *epoch,
+                                                float4 *sq, float *st)
 {
-    *epoch += 1;
+    const int e = *epoch + 1;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const int k = idx[(size_t)e * n + i];
+        sq[i] = q[k];
+        st[i] = t[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        *epoch = e;
 }
 
 inline int pad_rows(int n) { return (n + kTile - 1) / kTile * kTile; }
@@ -771,14 +762,20 @@ inline int pad_rows(int n) { return (n + kTile - 1) / kTile * kTile; }
 
 using namespace mlp;
 
+// Device memory of a training call that the network keeps for the next one (a
+// cudaMalloc and cudaFree per call took 0.85 ms of a 13 ms fit).
+constexpr size_t kBlockKeep = (size_t)64 << 20;
+
 struct mbs_mlp {
     int device = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, upload = nullptr;   // upload: the training orders
     std::string err;
     float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     bf16 *wimg = nullptr;                 // weight operand images
     Weights w{};
     int step = 0;
+    unsigned char *block = nullptr;       // a training call's device arrays, kept between calls
+    size_t block_cap = 0;
     // samples for up to `cap` padded rows, activation images for `icap`
     int cap = 0, icap = 0;
     bf16 *acts = nullptr;
@@ -874,8 +871,8 @@ int check_err(mbs_mlp *net)
 int set_attrs(mbs_mlp *net)
 {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    MK(cudaFuncSetAttribute(k_chain<false, kFwdRows>, a, kChainSmemFwd), "kernel attributes");
-    MK(cudaFuncSetAttribute(k_chain<true, kTrainRows>, a, kChainSmem), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_chain<false, kFwdRows>, a, ChainSmem<false, kFwdRows>::bytes), "kernel attributes");
+    MK(cudaFuncSetAttribute(k_chain<true, kTrainRows>, a, ChainSmem<true, kTrainRows>::bytes), "kernel attributes");
     MK(cudaFuncSetAttribute(k_update<false>, a, kUpSmem), "kernel attributes");
     MK(cudaFuncSetAttribute(k_update<true>, a, kUpSmem), "kernel attributes");
     return 0;
@@ -887,7 +884,6 @@ ChainArgs chain_args(mbs_mlp *net, int n)
     a.q = net->q;
     a.t = net->t;
     a.n = n;
-    a.n_set = n;
     a.params = net->params;
     a.w = net->w;
     a.img = net->img;
@@ -901,7 +897,8 @@ ChainArgs chain_args(mbs_mlp *net, int n)
 int forward_dev(mbs_mlp *net, int n)
 {
     const ChainArgs a = chain_args(net, n);
-    k_chain<false, kFwdRows><<<(n + kFwdRows - 1) / kFwdRows, 16 * kFwdRows, kChainSmemFwd, net->stream>>>(a);
+    k_chain<false, kFwdRows><<<(n + kFwdRows - 1) / kFwdRows, kChainThreads, ChainSmem<false, kFwdRows>::bytes,
+                               net->stream>>>(a);
     MK(cudaGetLastError(), "mlp forward launch");
     return 0;
 }
@@ -930,7 +927,8 @@ cudaError_t launch_dependent(cudaStream_t s, void (*kern)(Args), int grid, int t
 int step_dev(mbs_mlp *net, const ChainArgs &a, UpdateArgs u, bool use_adam)
 {
     const int bp = pad_rows(a.n);
-    MK(launch_dependent(net->stream, k_chain<true, kTrainRows>, bp / kTrainRows, 16 * kTrainRows, kChainSmem, a),
+    MK(launch_dependent(net->stream, k_chain<true, kTrainRows>, bp / kTrainRows, kChainThreads,
+                        ChainSmem<true, kTrainRows>::bytes, a),
        "mlp chain launch");
     u.img = net->img;
     u.dy = net->dy;
@@ -963,7 +961,8 @@ extern "C" int mbs_mlp_create(mbs_mlp **out, int device, uint64_t seed)
     mbs_mlp *net = new mbs_mlp();
     net->device = device;
     auto bail = [&](int rc) { mbs_mlp_destroy(net); return rc; };
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking) != cudaSuccess
+        || cudaStreamCreateWithFlags(&net->upload, cudaStreamNonBlocking) != cudaSuccess)
         return bail(-3);
     const size_t np = kNParams;
     if (cudaMalloc((void **)&net->params, np * 4) || cudaMalloc((void **)&net->grad, np * 4)
@@ -1000,11 +999,13 @@ extern "C" int mbs_mlp_destroy(mbs_mlp *net)
         return -1;
     cudaSetDevice(net->device);
     free_acts(net);
-    void *ps[] = {net->params, net->grad, net->m, net->v, net->wimg, net->acts, net->scalar};
+    void *ps[] = {net->params, net->grad, net->m, net->v, net->wimg, net->acts, net->scalar, net->block};
     for (void *p : ps)
         cudaFree(p);
     if (net->stream)
         cudaStreamDestroy(net->stream);
+    if (net->upload)
+        cudaStreamDestroy(net->upload);
     delete net;
     return 0;
 }
@@ -1108,8 +1109,14 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
     for (int b0 = 0; b0 < n; b0 += batch)
         sizes.push_back(std::min(batch, n - b0));
     const size_t steps = (size_t)epochs * sizes.size();
-    float *dq = nullptr, *dt = nullptr, *dbc = nullptr;
-    int *didx = nullptr, *dstate = nullptr;
+    // one block (kept by the network up to kBlockKeep): samples, targets, the
+    // same in the epoch's order, the orders, the bias corrections, the epoch
+    // counter
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t bq = up((size_t)n * kIn * 4), bt = up((size_t)n * 4), bi = up((size_t)epochs * n * 4);
+    const size_t bb = up(steps * 2 * 4);
+    const size_t need = 2 * bq + 2 * bt + bi + bb + 256;
+    cudaEvent_t ready = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     auto cleanup = [&]() {
@@ -1117,80 +1124,103 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
             cudaGraphExecDestroy(exec);
         if (graph)
             cudaGraphDestroy(graph);
-        cudaFree(dq); cudaFree(dt); cudaFree(didx); cudaFree(dbc); cudaFree(dstate);
+        if (ready)
+            cudaEventDestroy(ready);
+        cudaStreamSynchronize(net->upload);   // it reads this call's host arrays
+        cudaStreamSynchronize(s);
+        if (net->block_cap > kBlockKeep) {
+            cudaFree(net->block);
+            net->block = nullptr;
+            net->block_cap = 0;
+        }
     };
-    if (cudaMalloc((void **)&dq, (size_t)n * kIn * 4) || cudaMalloc((void **)&dt, (size_t)n * 4)
-        || cudaMalloc((void **)&didx, (size_t)epochs * n * 4 + 4)
-        || cudaMalloc((void **)&dbc, steps * 2 * 4 + 8) || cudaMalloc((void **)&dstate, 8)) {
+    if (net->block_cap < need) {
+        cudaFree(net->block);
+        net->block = nullptr;
+        net->block_cap = 0;
+        if (cudaMalloc((void **)&net->block, need) == cudaSuccess)
+            net->block_cap = need;
+    }
+    unsigned char *block = net->block;
+    if (net->block_cap < need
+        || cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
         cleanup();
         return mfail(net, -4, "cudaMalloc training set");
     }
-    // the shuffled order of every epoch and every step's Adam bias
-    // corrections, uploaded once
-    std::vector<int> order((size_t)epochs * n);
-    std::mt19937_64 rng(seed);
-    std::vector<int> perm(n);
-    for (int e = 0; e < epochs; ++e) {
-        for (int i = 0; i < n; ++i)
-            perm[i] = i;
-        std::shuffle(perm.begin(), perm.end(), rng);
-        std::copy(perm.begin(), perm.end(), order.begin() + (size_t)e * n);
-    }
+    float *dq = (float *)block, *sq = (float *)(block + bq), *dt = (float *)(block + 2 * bq);
+    float *st = (float *)(block + 2 * bq + bt), *dbc = (float *)(block + 2 * bq + 2 * bt + bi);
+    int *didx = (int *)(block + 2 * bq + 2 * bt), *dstate = (int *)(block + 2 * bq + 2 * bt + bi + bb);
+    // every step's Adam bias corrections
     std::vector<float> bc(steps * 2 + 2);
     for (size_t k = 0; k < steps; ++k) {
         const float step = (float)(net->step + 1 + (long long)k);
         bc[2 * k] = 1.f - std::pow(0.9f, step);
         bc[2 * k + 1] = 1.f - std::pow(0.999f, step);
     }
-    const int zero2[2] = {0, 0};
+    const int before = -1;
     cudaError_t e = cudaMemcpyAsync(dq, q, (size_t)n * kIn * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dt, t, (size_t)n * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && epochs > 0)
-        e = cudaMemcpyAsync(didx, order.data(), order.size() * 4, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && epochs > 0)
         e = cudaMemcpyAsync(dbc, bc.data(), steps * 2 * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dstate, zero2, 8, cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(dstate, &before, 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);   // the host arrays are read before they go
     if (e != cudaSuccess) {
         cleanup();
         return mfail(net, -3, std::string("training upload: ") + cudaGetErrorString(e));
     }
-    // One epoch (two kernels per minibatch, the epoch counter's advance at the
-    // end) captured once as a graph and replayed per epoch.
+    std::vector<int> order((size_t)epochs * n);   // outlives the uploads (cleanup waits)
+    // One epoch (its shuffle, then two kernels per minibatch) captured once as a
+    // graph and replayed per epoch.
     if (epochs > 0) {
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             const int spe = (int)sizes.size();
+            k_epoch<<<1, 1024, 0, s>>>((const float4 *)dq, dt, didx, n, dstate, (float4 *)sq, st);
             ChainArgs ca = chain_args(net, batch);
-            ca.q = dq;
-            ca.t = dt;
-            ca.idx = didx;
-            ca.epoch = dstate;
-            ca.n_set = n;
             UpdateArgs ua{};
             ua.lr = lr;
             ua.bc = dbc;
             ua.epoch = dstate;
             ua.steps_per_epoch = spe;
             for (int k = 0, b0 = 0; k < spe && rc == 0; b0 += sizes[k], ++k) {
-                ca.b0 = b0;
+                ca.q = sq + (size_t)b0 * kIn;
+                ca.t = st + b0;
                 ca.n = sizes[k];
                 ua.k = k;
                 rc = step_dev(net, ca, ua, true);
             }
-            if (rc == 0)
-                k_next_epoch<<<1, 1, 0, s>>>(dstate);
             const cudaError_t ec = cudaStreamEndCapture(s, &graph);
             if (e == cudaSuccess)
                 e = ec;
         }
         if (e == cudaSuccess && rc == 0)
             e = cudaGraphInstantiate(&exec, graph, 0);
-        for (int ep = 0; ep < epochs && e == cudaSuccess && rc == 0; ++ep)
-            e = cudaGraphLaunch(exec, s);
+        // the epochs' shuffled orders, some epochs at a time on the upload
+        // stream while the device trains on the ones before
+        std::mt19937_64 rng(seed);
+        std::vector<int> perm(n);
+        const int some = std::max(1, 16384 / n);
+        for (int e0 = 0; e0 < epochs && e == cudaSuccess && rc == 0; e0 += some) {
+            const int e1 = std::min(epochs, e0 + some);
+            for (int ep = e0; ep < e1; ++ep) {
+                for (int i = 0; i < n; ++i)
+                    perm[i] = i;
+                std::shuffle(perm.begin(), perm.end(), rng);
+                std::copy(perm.begin(), perm.end(), order.begin() + (size_t)ep * n);
+            }
+            e = cudaMemcpyAsync(didx + (size_t)e0 * n, order.data() + (size_t)e0 * n, (size_t)(e1 - e0) * n * 4,
+                                cudaMemcpyHostToDevice, net->upload);
+            if (e == cudaSuccess)
+                e = cudaEventRecord(ready, net->upload);
+            if (e == cudaSuccess)
+                e = cudaStreamWaitEvent(s, ready, 0);
+            for (int ep = e0; ep < e1 && e == cudaSuccess; ++ep)
+                e = cudaGraphLaunch(exec, s);
+        }
         if (e != cudaSuccess || rc) {
             cudaGetLastError();
             cleanup();
