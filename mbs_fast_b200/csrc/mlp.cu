@@ -448,24 +448,21 @@ struct UpdateArgs {
     Watch watch;
 };
 
-// Adam state of N consecutive parameters (N = 4 or 8: vector accesses): loaded
-// while the gradients are still being formed, then updated with the step's
-// bias corrections and stored.
+// Adam state of N consecutive parameters (1, or 4 as vectors): loaded while the
+// gradients are still being formed, then updated with the step's bias
+// corrections and stored.
 template <int N>
 struct AdamState {
     float m[N], v[N], p[N];
     __device__ __forceinline__ void load(const UpdateArgs &a, int i)
     {
-        if constexpr (N % 4 == 0) {
-#pragma unroll
-            for (int k = 0; k < N; k += 4) {
-                const float4 x = *reinterpret_cast<const float4 *>(a.m + i + k);
-                const float4 y = *reinterpret_cast<const float4 *>(a.v + i + k);
-                const float4 z = *reinterpret_cast<const float4 *>(a.p + i + k);
-                m[k] = x.x; m[k + 1] = x.y; m[k + 2] = x.z; m[k + 3] = x.w;
-                v[k] = y.x; v[k + 1] = y.y; v[k + 2] = y.z; v[k + 3] = y.w;
-                p[k] = z.x; p[k + 1] = z.y; p[k + 2] = z.z; p[k + 3] = z.w;
-            }
+        if constexpr (N == 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(a.m + i);
+            const float4 y = *reinterpret_cast<const float4 *>(a.v + i);
+            const float4 z = *reinterpret_cast<const float4 *>(a.p + i);
+            m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w;
+            v[0] = y.x; v[1] = y.y; v[2] = y.z; v[3] = y.w;
+            p[0] = z.x; p[1] = z.y; p[2] = z.z; p[3] = z.w;
         } else {
             m[0] = a.m[i];
             v[0] = a.v[i];
@@ -483,13 +480,10 @@ struct AdamState {
             v[k] = vi;
             p[k] = p[k] - a.lr * (mi / bc1) / (sqrtf(vi / bc2) + 1e-8f);
         }
-        if constexpr (N % 4 == 0) {
-#pragma unroll
-            for (int k = 0; k < N; k += 4) {
-                *reinterpret_cast<float4 *>(a.m + i + k) = make_float4(m[k], m[k + 1], m[k + 2], m[k + 3]);
-                *reinterpret_cast<float4 *>(a.v + i + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
-                *reinterpret_cast<float4 *>(a.p + i + k) = make_float4(p[k], p[k + 1], p[k + 2], p[k + 3]);
-            }
+        if constexpr (N == 4) {
+            *reinterpret_cast<float4 *>(a.m + i) = make_float4(m[0], m[1], m[2], m[3]);
+            *reinterpret_cast<float4 *>(a.v + i) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4 *>(a.p + i) = make_float4(p[0], p[1], p[2], p[3]);
         } else {
             a.m[i] = m[0];
             a.v[i] = v[0];
@@ -502,8 +496,11 @@ struct AdamState {
 // dW1 = dZ1^T X0, then the vectors, 32 entries a CTA: db3, db2, db1 (column
 // sums of dZ) and the head's dw4, db4.  Both operands of a product are
 // contiguous pieces of the images, copied 128 samples at a time into two
-// stages; thread 0 copies and issues the MMAs.
-constexpr int kUpThreads = 256;
+// stages; thread 0 copies and issues the MMAs.  The Adam update,
+// a chain of divisions and a square root per parameter, takes half of the
+// kernel's 6.7 us: four parameters per thread (1638 samples, 100 epochs: 11.60
+// ms) rather than eight with 256 threads (11.82) or two with 1024 (12.19).
+constexpr int kUpThreads = 512;
 constexpr int kUpN = 16;
 constexpr int kUpStage = 2 * kImg + kUpN * kTile * 2;
 constexpr int kUpSmem = 2 * kUpStage + 64;
@@ -555,6 +552,8 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         const int g = warp;
         float s = 0.f;
         int idx = -1;
+        if (g >= 8)
+            return;                            // 8 warps work, and wait for each other below
         if (job < kJobHead) {
             const int l = (job - kJobBias) / (kH / 32), c = (job - kJobBias) % (kH / 32) * 32 + lane;
             const bf16 *x = l == 0 ? a.img.dz3 : l == 1 ? a.img.dz2 : a.img.dz1;
@@ -574,10 +573,10 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         part[g][lane] = s;
         AdamState<1> ad;
         if (g == 0 && idx >= 0 && kAdam) {
-            corrections();
             ad.load(a, idx);
+            corrections();
         }
-        __syncthreads();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         if (g == 0 && idx >= 0) {
             float t = part[0][lane];
             for (int k = 1; k < 8; ++k)
@@ -613,17 +612,16 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         if (nblk > 1)
             load();
     }
-    // accumulator rows 32 (w % 4) .. + 31 (the warp's lane quarter), columns
-    // 8 (w / 4) .. + 7; their Adam state comes while the products run
-    const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 8, c = n0 + cl;
-    AdamState<8> ad;
-    AdamState<4> ad1;
+    // accumulator row 32 (w % 4) + lane (the warp's lane quarter), columns
+    // 4 (w / 4) .. + 3; their Adam state comes while the products run
+    const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 4, c = n0 + cl;
+    const bool own = l != 1 || cl < kIn;       // dW1: the padding columns have no parameter
+    const int i0 = l == 1 ? oW1 + r * kIn + c : (l == 3 ? oW3 : oW2) + r * kH + c;
+    AdamState<4> ad;
     if (kAdam) {
+        if (own)
+            ad.load(a, i0);
         corrections();
-        if (l != 1)
-            ad.load(a, (l == 3 ? oW3 : oW2) + r * kH + c);
-        else if (cl == 0)
-            ad1.load(a, oW1 + r * kIn);
     }
     if (tid == 0) {
         bool ok = true;
@@ -657,39 +655,23 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     __syncthreads();
     if (s_ok) {
         asm volatile("tcgen05.fence::after_thread_sync;");
-        __align__(16) float gv[8];
-        tmem_ld<8>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cl, gv);
-        if (l == 1) {
-            if (cl == 0) {
-                const int i0 = oW1 + r * kIn;
-                if (kAdam) {
-                    ad1.step(a, i0, gv, bc1, bc2);
+        float gv[4];
+        tmem_ld<4>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cl, gv);
+        if (own && !kAdam)
+            *reinterpret_cast<float4 *>(a.grad + i0) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+        if (own && kAdam) {
+            ad.step(a, i0, gv, bc1, bc2);
+            __align__(8) bf16 h[4];
 #pragma unroll
-                    for (int k = 0; k < kIn; ++k)
-                        *reinterpret_cast<bf16 *>(reinterpret_cast<unsigned char *>(a.w.w1f)
-                                                  + kmajor_off(r, k, kInPad)) = __float2bfloat16(ad1.p[k]);
-                } else {
-                    *reinterpret_cast<float4 *>(a.grad + i0) = *reinterpret_cast<const float4 *>(gv);
-                }
-            }
-        } else {
-            const int i0 = (l == 3 ? oW3 : oW2) + r * kH + c;
-            if (kAdam) {
-                unsigned char *wf = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3f : a.w.w2f);
+            for (int k = 0; k < 4; ++k)
+                h[k] = __float2bfloat16(ad.p[k]);
+            unsigned char *wf = reinterpret_cast<unsigned char *>(l == 1 ? a.w.w1f : l == 3 ? a.w.w3f : a.w.w2f);
+            *reinterpret_cast<uint2 *>(wf + kmajor_off(r, c, l == 1 ? kInPad : kTile)) = *reinterpret_cast<const uint2 *>(h);
+            if (l != 1) {
                 unsigned char *wb = reinterpret_cast<unsigned char *>(l == 3 ? a.w.w3b : a.w.w2b);
-                __align__(16) bf16 h[8];
-                ad.step(a, i0, gv, bc1, bc2);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    h[i] = __float2bfloat16(ad.p[i]);
-                *reinterpret_cast<uint4 *>(wf + kmajor_off(r, c, kTile)) = *reinterpret_cast<const uint4 *>(h);
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    *reinterpret_cast<bf16 *>(wb + kmajor_off(c + i, r, kTile)) = h[i];
-            } else {
-                float4 *dst = reinterpret_cast<float4 *>(a.grad + i0);
-                dst[0] = *reinterpret_cast<const float4 *>(gv);
-                dst[1] = *reinterpret_cast<const float4 *>(gv + 4);
+                for (int k = 0; k < 4; ++k)
+                    *reinterpret_cast<bf16 *>(wb + kmajor_off(c + k, r, kTile)) = h[k];
             }
         }
     }
