@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <string>
 #include <vector>
 
@@ -58,8 +59,8 @@ constexpr Variant kVariantsF64[] = {{64, 3, 4}, {128, 1, 3}, {96, 2, 4}, {128, 1
 constexpr Variant kNoShadowF32 = {128, 3, 3};
 constexpr Variant kNoShadowF64 = {128, 1, 3};
 // Shapes for the rows past the last whole tile (see row_tail).
-constexpr Variant kTailF32[] = {{128, 1, 4}, {128, 2, 3}};
-constexpr Variant kTailF64[] = {{64, 1, 6}, {128, 1, 4}};
+constexpr Variant kTailF32[] = {{64, 1, 4}, {96, 1, 4}, {128, 1, 4}, {96, 2, 4}, {128, 2, 3}};
+constexpr Variant kTailF64[] = {{64, 1, 6}, {96, 1, 4}, {128, 1, 4}};
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
 
@@ -786,11 +787,11 @@ LaunchPlan plan_launch(int n_az, int n_t, int n_orient, int dirs_per_cta, int ct
 
 // Persistent launch: as many CTAs as fit on the device at once (at most one
 // per work item); P.work must be zero on `st` when the kernel starts.
-template <typename T, int TPB, int DPT, bool NS, int MINB>
+template <typename T, int TPB, int DPT, bool NS, int MINB, int BEAMS = default_stage<T>(TPB)>
 cudaError_t launch_one(const KParams &P, cudaStream_t st)
 {
-    auto kern = po_diffract_kernel<T, TPB, DPT, NS, MINB>;
-    const size_t smem = diffract_smem_bytes<T, TPB, DPT, NS>();
+    auto kern = po_diffract_kernel<T, TPB, DPT, NS, MINB, BEAMS>;
+    const size_t smem = diffract_smem_bytes<T, TPB, DPT, NS, BEAMS>();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
@@ -870,19 +871,26 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 
 // The zenith rows past the last whole tile of the default shape (kVariants[0]:
 // 384 rows FP32C, 192 FP64) run as a second launch with fewer directions per
-// thread, on the side stream beside the main one, when a narrower shape
+// thread, on the side stream beside the main one, in the smallest shape that
 // holds them: index into kTail*, or -1.  A thread whose slots lie past the
-// last row still evaluates them.  Time of a tail tile against a whole one
-// (64 orientations of 87 beams, 48 azimuths): FP32C 128 rows 0.50, 256 rows
-// 0.77 (0.81 with four CTAs per SM and spills); FP64 64 rows 0.45, 128 rows 0.76.  The tail shapes stage the same
-// beams at a time as the default ones, so a direction's sums are the same
-// bit for bit whichever launch holds it.
+// last row still evaluates them, so the shapes step by 32 or 64 slots; with
+// few rows the stage in shared memory sets the resident CTAs (four, three for
+// 128x2) and each of their warps has up to 200 registers and no spills.
+// Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a whole tile
+// of 384 rows: 3.04 ms): up to 64 rows 1.11 ms (1.20 in 96x1), 96 rows 1.22
+// (1.44 in 128x1, 1.22 with five CTAs per SM and spills), 128 rows 1.45, 192
+// rows 1.80 (2.28 in 128x2, 1.93 in 64x3), 256 rows 2.30; 288 rows in 96x3
+// take the whole tile's time.  FP64, 150 orientations: 96 rows 1.02 ms (1.16
+// in 128x1), 128 rows 1.17 (1.40 in 64x2).  The tail shapes stage the same
+// beams at a time as the default ones, so a direction's sums are the same bit
+// for bit whichever launch holds it.
 int row_tail(int pi, int n_t)
 {
     const Variant *tails = pi == 0 ? kTailF64 : kTailF32;
+    const int n = pi == 0 ? std::size(kTailF64) : std::size(kTailF32);
     const Variant full = pi == 0 ? kVariantsF64[0] : kVariantsF32[0];
     const int rest = n_t % (full.tpb * full.dpt);
-    for (int i = 0; i < 2 && rest > 0; ++i)
+    for (int i = 0; i < n && rest > 0; ++i)
         if (rest <= tails[i].tpb * tails[i].dpt)
             return i;
     return -1;
@@ -890,9 +898,20 @@ int row_tail(int pi, int n_t)
 
 cudaError_t launch_tail(int pi, int tail, const KParams &P, cudaStream_t st)
 {
+    constexpr int beams = default_stage<float>(kVariantsF32[0].tpb);   // the default shape's stage
     if (pi == 0)
-        return tail == 0 ? launch_one<double, 64, 1, false, 6>(P, st) : launch_one<double, 128, 1, false, 4>(P, st);
-    return tail == 0 ? launch_one<float, 128, 1, false, 4>(P, st) : launch_one<float, 128, 2, false, 3>(P, st);
+        switch (tail) {
+        case 0: return launch_one<double, 64, 1, false, 6>(P, st);
+        case 1: return launch_one<double, 96, 1, false, 4>(P, st);
+        default: return launch_one<double, 128, 1, false, 4>(P, st);
+        }
+    switch (tail) {
+    case 0: return launch_one<float, 64, 1, false, 4, beams>(P, st);
+    case 1: return launch_one<float, 96, 1, false, 4, beams>(P, st);
+    case 2: return launch_one<float, 128, 1, false, 4, beams>(P, st);
+    case 3: return launch_one<float, 96, 2, false, 4, beams>(P, st);
+    default: return launch_one<float, 128, 2, false, 3, beams>(P, st);
+    }
 }
 
 // The rows of a call: [0, main_rows) in the chosen shape, the rest (`tail` >= 0)

@@ -777,12 +777,15 @@ struct __align__(16) SVertRaw<double> {
     double2 q[3];   // (ps, pc) (p0, syx) (sxy, unused)
 };
 
-// FP64: 64 beams a stage whatever the CTA (a record is 288 bytes, and the sine
-// table takes 8 KB).  FP32C: the stage ends set where the FP32 block sums are
-// folded.
-template <typename T, int TPB>
+// Beams a stage holds.  FP64: 64 whatever the CTA (a record is 288 bytes, and
+// the sine table takes 8 KB).  FP32C: the stage ends set where the FP32 block
+// sums are folded, so shapes that must agree bit for bit have the same.
+template <typename T>
+constexpr int default_stage(int tpb) { return sizeof(T) == 8 ? 64 : tpb; }
+
+template <typename T, int BEAMS>
 struct StageCfg {
-    static constexpr int kBeams = sizeof(T) == 8 ? 64 : TPB;
+    static constexpr int kBeams = BEAMS;
     static constexpr int kVerts = 4 * kBeams;
     static constexpr size_t kBytes = kBeams * sizeof(SBeamRaw<T>) + kVerts * sizeof(SVertRaw<T>);
 };
@@ -1484,10 +1487,10 @@ __device__ __forceinline__ void jones_update(const SBeamRaw<T> &rec, const T *s_
 // (orientation chunk, azimuth bin, zenith tile) from a global counter.  Each
 // thread owns DPT directions of an item (rows trow + d*TPB + thread of the
 // item's azimuth).  T = float selects FP32C.
-template <typename T, int TPB, int DPT, bool NS, int MINB>
+template <typename T, int TPB, int DPT, bool NS, int MINB, int BEAMS = default_stage<T>(TPB)>
 __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
 {
-    using Cfg = StageCfg<T, TPB>;
+    using Cfg = StageCfg<T, BEAMS>;
     constexpr int kDirs = TPB * DPT;
     constexpr bool kF32 = sizeof(T) == 4;
     constexpr int kSets = NS ? 2 : 1;        // full and no-shadow sums
@@ -1912,12 +1915,12 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
     }   // work items
 }
 
-template <typename T, int TPB, int DPT, bool NS>
+template <typename T, int TPB, int DPT, bool NS, int BEAMS>
 constexpr size_t diffract_smem_bytes()
 {
-    return StageCfg<T, TPB>::kBytes + 8 * TPB * sizeof(T)
+    return StageCfg<T, BEAMS>::kBytes + 8 * TPB * sizeof(T)
          + (sizeof(T) == 4 ? (NS ? 2 : 1) * 16 * TPB * DPT * sizeof(float) : 0)
-         + (size_t)DPT * ((StageCfg<T, TPB>::kBeams + 31) / 32) * TPB * sizeof(uint32_t);
+         + (size_t)DPT * ((BEAMS + 31) / 32) * TPB * sizeof(uint32_t);
 }
 
 // Polar zenith rows (row_kind 1): every azimuth bin has the same direction

@@ -213,25 +213,10 @@ def test_proposal_network_step(n):
     assert np.max(np.abs((p0 - got - step)[big])) <= 1e-3 * 2e-3
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("precision,tile,rest", [
-    (p, n, r) for p, n, rs in ((abi.FP64, 192, (1, 64, 65, 128, 129)), (abi.FP32C, 384, (1, 128, 129, 256, 257)))
-    for r in rs])
-@pytest.mark.parametrize("whole", [0, 1])
-def test_row_tails(precision, tile, rest, whole):
-    """Zenith rows past the last whole tile (alone, and after a whole tile):
-    against the oracle, and bit for bit against the same directions evaluated
-    inside a whole tile of the main shape (FP32C sums included: the tail
-    shapes stage the same beams)."""
-    b, w = S.ragged(3, 70, 12.0, 17), S.wave()
-    g = S.grid(2, whole * tile + rest - 1)
-    h = GpuHandlerPO(g, w)
-    M = h.new_mueller()
-    assert h.handle_orientations_to_local_gpu(b, M, precision=precision)
-    h.close()
-    assert _l2(M, oracle.po_diffract(b, g, w)) < (FP64_L2 if precision == abi.FP64 else 2e-5)
-    # the last `tile` rows (polar row left out) as a grid of their own, padded
-    # with rows between the first ones when there are fewer
+def _in_a_whole_tile(b, w, g, M, tile, precision):
+    """The grid's last `tile` rows (polar rows left out) evaluated as a grid of
+    their own, padded with rows between the first ones when there are fewer:
+    M must hold the same values bit for bit."""
     th, vf = g.theta[1:-1][-tile:], g.vf[:, 1:-1][:, -tile:]
     n = len(th)
     fill = tile - n
@@ -247,6 +232,42 @@ def test_row_tails(precision, tile, rest, whole):
     h2.close()
     if n:
         assert np.array_equal(M[:, 1:-1][:, -n:], M2[:, fill:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tile,rest", [
+    (p, n, r) for p, n, rs in ((abi.FP64, 192, (1, 64, 65, 96, 97, 128, 129)),
+                               (abi.FP32C, 384, (1, 64, 65, 96, 97, 128, 129, 192, 193, 256, 257)))
+    for r in rs])
+@pytest.mark.parametrize("whole", [0, 1])
+def test_row_tails(precision, tile, rest, whole):
+    """Zenith rows past the last whole tile (alone, and after a whole tile):
+    against the oracle, and bit for bit against the same directions evaluated
+    inside a whole tile of the main shape (FP32C sums included: the tail
+    shapes stage the same beams)."""
+    b, w = S.ragged(3, 70, 12.0, 17), S.wave()
+    g = S.grid(2, whole * tile + rest - 1)
+    h = GpuHandlerPO(g, w)
+    M = h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, precision=precision)
+    h.close()
+    assert _l2(M, oracle.po_diffract(b, g, w)) < (FP64_L2 if precision == abi.FP64 else 2e-5)
+    _in_a_whole_tile(b, w, g, M, tile, precision)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rest", [50, 90, 120, 180, 250])
+def test_row_tails_of_several_stages(rest):
+    """FP32C tails with more beams per orientation than a stage holds: the
+    shapes end their stages at the same beams, so the sums are bit for bit
+    those of the main shape."""
+    b, w = S.batch(2, 300, 12.0, 23), S.wave()
+    g = S.grid(2, rest - 1)
+    h = GpuHandlerPO(g, w)
+    M = h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, precision=abi.FP32C)
+    h.close()
+    _in_a_whole_tile(b, w, g, M, 384, abi.FP32C)
 
 
 @pytest.mark.gpu
