@@ -877,11 +877,13 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // few rows the stage in shared memory sets the resident CTAs (four, three for
 // 128x2) and each of their warps has up to 200 registers and no spills.
 // Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a whole tile
-// of 384 rows: 3.04 ms): up to 64 rows 1.11 ms (1.20 in 96x1), 96 rows 1.22
-// (1.44 in 128x1, 1.22 with five CTAs per SM and spills), 128 rows 1.45, 192
-// rows 1.80 (2.28 in 128x2, 1.93 in 64x3), 256 rows 2.30; 288 rows in 96x3
-// take the whole tile's time.  FP64, 150 orientations: 96 rows 1.02 ms (1.16
-// in 128x1), 128 rows 1.17 (1.40 in 64x2).  The tail shapes stage the same
+// of 384 rows: 3.04 ms): up to 64 rows 1.03 ms, 96 rows 1.17, 128 rows 1.35,
+// 192 rows 1.77, 256 rows 2.25; FP64, 150 orientations (192 rows: 1.76 ms): 64
+// rows 0.77 ms, 96 rows 1.00, 128 rows 1.18.  Of the shapes compared one beam
+// per iteration: 64 rows 1.11 ms in 64x1, 1.20 in 96x1; 96 rows 1.22 in 96x1,
+// 1.44 in 128x1, 1.22 with five CTAs per SM and spills; 192 rows 1.79 in 96x2,
+// 2.28 in 128x2, 1.93 in 64x3; 288 rows in 96x3 the whole tile's time; FP64 96
+// rows 1.02 in 96x1, 1.16 in 128x1, 128 rows 1.17 in 128x1, 1.40 in 64x2.  The tail shapes stage the same
 // beams at a time as the default ones, so a direction's sums are the same bit
 // for bit whichever launch holds it.
 int row_tail(int pi, int n_t)

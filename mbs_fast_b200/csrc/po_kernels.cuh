@@ -1631,6 +1631,19 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
             static_assert(32 % kFlushEvery == 0, "mask words hold whole blocks");
             for (int j0 = 0; j0 < nb; j0 += kFlushEvery) {
             const int j1 = min(nb, j0 + kFlushEvery);
+            // Two beams per iteration where the shape leaves registers for it: one
+            // beam's loads and edge head then overlap the other's chain, which
+            // a thread with one or two directions cannot fill by itself.  300
+            // orientations of 87 beams, 48 azimuths, FP32C: 64 rows (64x1) 1108 ->
+            // 1032 us, 96 (96x1) 1219 -> 1174, 128 (128x1) 1451 -> 1353, 192 (96x2)
+            // 1790 -> 1768, 256 (128x2) 2301 -> 2246, no-shadow sums (128x3) 1041
+            // -> 1012; FP64, 150 orientations: 73 rows (96x1) 1021 -> 1002.  Slower
+            // where it adds spills or the directions fill the chain: FP32C 128x3
+            // 3043 -> 3066, FP64 64x3 1762 -> 1905, 128x1 with 128 registers 1176 ->
+            // 1215; four beams: 64x1 1143, 96x1 1311.
+            constexpr bool kRoomy = TPB * MINB <= 384;   // 168 registers or more
+            constexpr int kUnroll = (kF32 ? DPT == 1 || NS || (DPT == 2 && kRoomy) : DPT == 1 && kRoomy) ? 2 : 1;
+#pragma unroll kUnroll
             for (int j = j0; j < j1; ++j) {
                 BeamRegs<T> b;
                 load_beam(sb[j], b);
