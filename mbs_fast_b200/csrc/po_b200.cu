@@ -873,9 +873,9 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // 384 rows FP32C, 192 FP64) run as a second launch with fewer directions per
 // thread, on the side stream beside the main one, in the smallest shape that
 // holds them: index into kTail*, or -1.  A thread whose slots lie past the
-// last row still evaluates them, so the shapes step by 32 or 64 slots; with
-// few rows the stage in shared memory sets the resident CTAs (four, three for
-// 128x2) and each of their warps has up to 200 registers and no spills.
+// last row still evaluates them, so the shapes step by 32 or 64 slots.  The
+// stage in shared memory sets the resident CTAs (four, three for 128x2), so
+// all but 128x1 (128 registers) have 164 to 200 registers and no spills.
 // Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a whole tile
 // of 384 rows: 3.04 ms): up to 64 rows 1.03 ms, 96 rows 1.17, 128 rows 1.35,
 // 192 rows 1.77, 256 rows 2.25; FP64, 150 orientations (192 rows: 1.76 ms): 64
@@ -883,9 +883,9 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // per iteration: 64 rows 1.11 ms in 64x1, 1.20 in 96x1; 96 rows 1.22 in 96x1,
 // 1.44 in 128x1, 1.22 with five CTAs per SM and spills; 192 rows 1.79 in 96x2,
 // 2.28 in 128x2, 1.93 in 64x3; 288 rows in 96x3 the whole tile's time; FP64 96
-// rows 1.02 in 96x1, 1.16 in 128x1, 128 rows 1.17 in 128x1, 1.40 in 64x2.  The tail shapes stage the same
-// beams at a time as the default ones, so a direction's sums are the same bit
-// for bit whichever launch holds it.
+// rows 1.02 in 96x1, 1.16 in 128x1, 128 rows 1.17 in 128x1, 1.40 in 64x2.  The
+// tail shapes stage the same beams at a time as the default ones, so a
+// direction's sums are the same bit for bit whichever launch holds it.
 int row_tail(int pi, int n_t)
 {
     const Variant *tails = pi == 0 ? kTailF64 : kTailF32;
