@@ -60,7 +60,7 @@ constexpr Variant kNoShadowF32 = {128, 3, 3};
 constexpr Variant kNoShadowF64 = {128, 1, 3};
 // Shapes for the rows past the last whole tile (see row_tail).
 constexpr Variant kTailF32[] = {{64, 1, 4}, {96, 1, 4}, {128, 1, 4}, {96, 2, 4}, {128, 2, 3}};
-constexpr Variant kTailF64[] = {{64, 1, 6}, {96, 1, 4}, {128, 1, 4}};
+constexpr Variant kTailF64[] = {{64, 1, 6}, {96, 1, 4}, {128, 1, 4}, {160, 1, 3}};
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
 
@@ -875,17 +875,19 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // holds them: index into kTail*, or -1.  A thread whose slots lie past the
 // last row still evaluates them, so the shapes step by 32 or 64 slots.  The
 // stage in shared memory sets the resident CTAs (four, three for 128x2), so
-// all but 128x1 (128 registers) have 164 to 200 registers and no spills.
-// Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a whole tile
-// of 384 rows: 3.04 ms): up to 64 rows 1.03 ms, 96 rows 1.17, 128 rows 1.35,
-// 192 rows 1.77, 256 rows 2.25; FP64, 150 orientations (192 rows: 1.76 ms): 64
-// rows 0.77 ms, 96 rows 1.00, 128 rows 1.18.  Of the shapes compared one beam
-// per iteration: 64 rows 1.11 ms in 64x1, 1.20 in 96x1; 96 rows 1.22 in 96x1,
-// 1.44 in 128x1, 1.22 with five CTAs per SM and spills; 192 rows 1.79 in 96x2,
-// 2.28 in 128x2, 1.93 in 64x3; 288 rows in 96x3 the whole tile's time; FP64 96
-// rows 1.02 in 96x1, 1.16 in 128x1, 128 rows 1.17 in 128x1, 1.40 in 64x2.  The
-// tail shapes stage the same beams at a time as the default ones, so a
-// direction's sums are the same bit for bit whichever launch holds it.
+// all but 128x1 and 160x1 (128 registers) have 164 to 200 registers and no
+// spills.  Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a
+// whole tile of 384 rows: 3.04 ms): up to 64 rows 1.03 ms, 96 rows 1.17, 128
+// rows 1.35, 192 rows 1.77, 256 rows 2.25; FP64, 150 orientations (192 rows:
+// 1.76 ms): 64 rows 0.77 ms, 96 rows 1.00, 128 rows 1.18, 160 rows 1.64.  Of
+// the shapes compared one beam per iteration: 64 rows 1.11 ms in 64x1, 1.20 in
+// 96x1; 96 rows 1.22 in 96x1, 1.44 in 128x1, 1.22 with five CTAs per SM and
+// spills; 192 rows 1.79 in 96x2, 2.28 in 128x2, 1.93 in 64x3; 288 rows in 96x3
+// the whole tile's time; FP64 96 rows 1.02 in 96x1, 1.16 in 128x1, 128 rows
+// 1.17 in 128x1, 1.40 in 64x2, 160 rows 1.64 in 160x1 with three CTAs per SM,
+// 1.86 with two.  The tail shapes stage the same beams at a time as the
+// default ones, so a direction's sums are the same bit for bit whichever
+// launch holds it.
 int row_tail(int pi, int n_t)
 {
     const Variant *tails = pi == 0 ? kTailF64 : kTailF32;
@@ -905,7 +907,8 @@ cudaError_t launch_tail(int pi, int tail, const KParams &P, cudaStream_t st)
         switch (tail) {
         case 0: return launch_one<double, 64, 1, false, 6>(P, st);
         case 1: return launch_one<double, 96, 1, false, 4>(P, st);
-        default: return launch_one<double, 128, 1, false, 4>(P, st);
+        case 2: return launch_one<double, 128, 1, false, 4>(P, st);
+        default: return launch_one<double, 160, 1, false, 3>(P, st);
         }
     switch (tail) {
     case 0: return launch_one<float, 64, 1, false, 4, beams>(P, st);

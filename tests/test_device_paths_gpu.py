@@ -236,7 +236,7 @@ def _in_a_whole_tile(b, w, g, M, tile, precision):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision,tile,rest", [
-    (p, n, r) for p, n, rs in ((abi.FP64, 192, (1, 64, 65, 96, 97, 128, 129)),
+    (p, n, r) for p, n, rs in ((abi.FP64, 192, (1, 64, 65, 96, 97, 128, 129, 160, 161)),
                                (abi.FP32C, 384, (1, 64, 65, 96, 97, 128, 129, 192, 193, 256, 257)))
     for r in rs])
 @pytest.mark.parametrize("whole", [0, 1])
