@@ -1893,7 +1893,7 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        po_thetas_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(part, rows, n, d_m11);
+        po_thetas_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(part, rows, n, nAz, d_m11);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)

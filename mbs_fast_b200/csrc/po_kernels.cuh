@@ -2262,21 +2262,58 @@ __global__ void __launch_bounds__(256) po_csca_kernel(const double *__restrict__
 // theta_m11_kernel, GpuDiffraction.cu:1909-1956, called by DiffractThetasGpu
 // :4780-4970).  Grid: x = (azimuth bin, tile of TPB * DPT zenith points),
 // y = beam chunk.  As in po_diffract_kernel the CTA folds its azimuth into
-// per-beam and per-vertex records in shared memory once and every thread
-// evaluates its points' edge sums from them; per pair only |s|^2 |R|^2 is
-// needed, and |P0 + cos t Pc + sin t Ps|^2 is a quadratic form in
-// (cos t, sin t) whose six coefficients are part of the record.  Small-phase
+// per-beam records in shared memory once and every thread evaluates its
+// points' edge sums from them.  No common phase is needed, so the vertex phases
+// are k (A x + B y) / 2 pi: the rounding of A and B is the same in them and in
+// the edge coefficients (phases folded over the azimuth like
+// po_diffract_kernel's left 40 times the error at an edge just above eps1).
+// Per pair only |s|^2 |R|^2 is
+// needed, R = P0 + cos t Pc + sin t Ps having eight real components: the record
+// holds the triangular factor U of the 8 x 3 matrix (P0, Pc, Ps), and
+// |R| = |U (1, cos t, sin t)| takes 8 operations instead of 24, with the same
+// error of some eps |P| in R (opposite to a beam's direction R vanishes by
+// cancellation: |R|^2 as a quadratic form in (cos t, sin t) is wrong by eps |P|^2
+// there, 13 % of a shadow beam's value at 179.99 degrees).  Small-phase
 // candidates are marked and evaluated in general form after the stage.
 // Bound by the FP64 pipe.  One thread per (point, beam, azimuth) with the
 // general evaluation took 1,225 us for 2,088 beams x 48 x 181 points, now
 // 229 us.
 struct __align__(16) ThetaBeam {
     double a[6];        // A, B coefficients (see BeamRegs)
-    double q[6];        // |P0|^2 2P0.Pc 2P0.Ps |Pc|^2 |Ps|^2 2Pc.Ps, times 0.5 weight / (n_az + 1)
+    double u[6];        // U by rows: u00 u01 u02 u11 u12 u22
     double slab[4];
-    double w;           // 0.5 weight / (n_az + 1)
+    double w;           // 0.5 weight
     int nv, vs;
 };
+// Modified Gram-Schmidt steps over 8 components: x becomes a unit vector, its
+// length returned (the zero vector stays); y loses its component along the unit
+// vector x, returned.
+__device__ __forceinline__ double take_column(double *x)
+{
+    double n = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        n = fma(x[e], x[e], n);
+    n = sqrt(n);
+    const double inv = n > 0.0 ? 1.0 / n : 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        x[e] *= inv;
+    return n;
+}
+
+__device__ __forceinline__ double take_component(const double *x, double *y)
+{
+    double c = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        c = fma(x[e], y[e], c);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        y[e] = fma(-c, x[e], y[e]);
+    return c;
+}
+
 constexpr int kThetaTpb = 64;
 constexpr int kThetaBeams = 64;                // beams and vertices of a stage
 constexpr int kThetaVerts = 4 * kThetaBeams;
@@ -2292,7 +2329,7 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
     __shared__ double2 s_sincos[kSinTab];
     fill_sincos_tab(s_sincos, TPB);
     const int p = blockIdx.x / tiles, tile = blockIdx.x - p * tiles;
-    const double cp = P.cphi[p], sp = P.sphi[p];
+    const double cp = P.cphi[p], sp = P.sphi[p], kt = P.wc.k * kInvTwoPi;
     const int64_t b0 = (int64_t)blockIdx.y * beams_per_chunk;
     const int64_t b1 = min(n_beams, b0 + beams_per_chunk);
     const int t0 = tile * TPB * DPT + threadIdx.x;
@@ -2329,19 +2366,20 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
                 const int mid = (lo + hi) >> 1;
                 if (P.beam_off[mid] <= bs + i) lo = mid; else hi = mid;
             }
-            const double w = 0.5 * P.weight[lo] / (double)(P.n_az + 1);
-            double q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            const double w = 0.5 * P.weight[lo];
+            double p0[8], pc[8], ps[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const double x = sp * r.Q(e) + cp * r.Q(8 + e);
-                const double y = -(cp * r.Q(16 + e) + sp * r.Q(24 + e));
-                const double z = r.Q(32 + e);
-                q[0] = fma(x, x, q[0]); q[1] = fma(2.0 * x, y, q[1]); q[2] = fma(2.0 * x, z, q[2]);
-                q[3] = fma(y, y, q[3]); q[4] = fma(z, z, q[4]); q[5] = fma(2.0 * y, z, q[5]);
+                p0[e] = sp * r.Q(e) + cp * r.Q(8 + e);
+                pc[e] = -(cp * r.Q(16 + e) + sp * r.Q(24 + e));
+                ps[e] = r.Q(32 + e);
             }
-#pragma unroll
-            for (int e = 0; e < 6; ++e)
-                s.q[e] = w * q[e];
+            s.u[0] = take_column(p0);
+            s.u[1] = take_component(p0, pc);
+            s.u[2] = take_component(p0, ps);
+            s.u[3] = take_column(pc);
+            s.u[4] = take_component(pc, ps);
+            s.u[5] = take_column(ps);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 s.slab[e] = r.slab(e);
@@ -2349,8 +2387,12 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
             s.nv = r.nv();
             s.vs = P.vbeg[bs + i] - vb0;
         }
-        for (int i = threadIdx.x; i < nvs; i += TPB)
-            fill_vert(VrecRef{P.vrec + vb0 + i, P.vrec_stride}, cp, sp, sv[i]);
+        for (int i = threadIdx.x; i < nvs; i += TPB) {
+            const DevVert v = P.verts[vb0 + i];
+            sv[i].q[0] = make_double2(kt * v.x, kt * v.y);
+            sv[i].q[1] = make_double2(0.0, isnan(v.syx) ? kInvalidSlope : v.syx);
+            sv[i].q[2] = make_double2(isnan(v.sxy) ? kInvalidSlope : v.sxy, 0.0);
+        }
         __syncthreads();
         uint64_t marked[DPT];
 #pragma unroll
@@ -2358,13 +2400,15 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
             marked[d] = 0;
         for (int j = 0; j < nb; ++j) {
             const ThetaBeam &b = sb[j];
-            double X1[DPT], X2[DPT], sr[DPT], si[DPT], m[DPT];
+            double A_[DPT], B_[DPT], X1[DPT], X2[DPT], sr[DPT], si[DPT], m[DPT];
             uint32_t mn[DPT];
             bool useX[DPT], cand[DPT];
 #pragma unroll
             for (int d = 0; d < DPT; ++d) {
                 const double A = fma(st[d], b.a[0], fma(ct[d], b.a[1], b.a[2]));
                 const double B = fma(st[d], b.a[3], fma(ct[d], b.a[4], b.a[5]));
+                A_[d] = A;
+                B_[d] = B;
                 useX[d] = fabs(B) > fabs(A);
                 X1[d] = useX[d] ? B : A;
                 X2[d] = useX[d] ? A : B;
@@ -2372,14 +2416,16 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
                 cand[d] = fabs(fma(A, b.slab[0], B * b.slab[1])) <= 1.0
                        && fabs(fma(A, b.slab[2], B * b.slab[3])) <= 1.0;
             }
-            edge_sums<DPT, true>(sv + b.vs, b.nv, st, ct, X1, X2, useX, sr, si, mn, s_sincos, P.wc.eps1);
+            // the phases' factors are (A, B) in place of (sin t, cos t)
+            edge_sums<DPT, true>(sv + b.vs, b.nv, A_, B_, X1, X2, useX, sr, si, mn, s_sincos, P.wc.eps1);
 #pragma unroll
             for (int d = 0; d < DPT; ++d) {
-                const double q = fma(ct[d], fma(ct[d], b.q[3], b.q[1]),
-                                     fma(st[d], fma(st[d], b.q[4], fma(ct[d], b.q[5], b.q[2])), b.q[0]));
+                const double y0 = fma(st[d], b.u[2], fma(ct[d], b.u[1], b.u[0]));
+                const double y1 = fma(st[d], b.u[4], ct[d] * b.u[3]), y2 = st[d] * b.u[5];
+                const double q = fma(y0, y0, fma(y1, y1, y2 * y2));   // |R|^2
                 const double r = rcp64(m[d]);
                 const double xr = sr[d] * r, xi = si[d] * r;
-                const double e = fma(xr, xr, xi * xi) * q;
+                const double e = fma(xr, xr, xi * xi) * q * b.w;
                 // a candidate's sums may be inf or NaN: select
                 acc[d] += cand[d] || isnan(e) ? 0.0 : e;
                 if (cand[d])
@@ -2426,27 +2472,33 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
             out[t0 + d * TPB] = acc[d];
 }
 
-// m11[t] = sum over rows r of partial[r][t]: 32 points per CTA, the 32 warps
-// take rows in turn and their sums meet in warp order (deterministic).
+// m11[t] = sum over rows r of partial[r][t], over n_az + 1: 32 points per CTA, the 32 warps
+// take rows in turn, four sums a thread, and the 32 sums of a point meet in a
+// tree (deterministic).  Around the poles every azimuth bin adds the same
+// value, whose roundings go the same way: added one after the other they
+// reach ten units of the last place.
 __global__ void __launch_bounds__(1024) po_thetas_sum_kernel(const double *partial, int64_t n_rows, int n_points,
-                                                            double *m11)
+                                                            int n_az, double *m11)
 {
     __shared__ double red[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * 32 + lane;
-    double s = 0.0;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
     if (t < n_points) {
-#pragma unroll 4
-        for (int64_t r = warp; r < n_rows; r += 32)
-            s += partial[r * n_points + t];
+        for (int64_t r = warp; r < n_rows; r += 128)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (r + 32 * i < n_rows)
+                    s[i] += partial[(r + 32 * i) * n_points + t];
     }
-    red[warp][lane] = s;
+    red[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
     __syncthreads();
-    if (warp == 0 && t < n_points) {
-        for (int w = 1; w < 32; ++w)
-            s += red[w][lane];
-        m11[t] = s;
-    }
+    double v = red[lane][warp];              // point `warp` of the CTA
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (lane == 0 && blockIdx.x * 32 + warp < n_points)
+        m11[blockIdx.x * 32 + warp] = v / (double)(n_az + 1);
 }
 
 // --------------------------------------------------------- extinction

@@ -404,3 +404,24 @@ def test_small_uploads_and_results_in_parts(beams):
             assert h.handle_orientations_to_local_gpu(one, P, precision=abi.FP64)
             assert _l2(P, oracle.po_diffract(one, g, w)) < FP64_L2
         h.close()
+
+
+@pytest.mark.gpu
+def test_theta_scan_opposite_to_a_beam():
+    """Shadow beams alone, up to the direction opposite to them, where the
+    rotation vanishes by cancellation: its entries are sums of four products of
+    unit vectors' components (rounding of 4 eps) and are 1 + cos theta large;
+    their squares, on both sides, differ by up to 16 eps / (1 + cos theta)
+    beside the FP64 gate."""
+    b = S.batch(1, 2, 11.0, 1).select(0, 1)
+    n = int(b.vert_offsets[1])
+    b = type(b)(beam_offsets=np.array([0, 1]), orient_weight=np.ones(1), vert_offsets=b.vert_offsets[:2].copy(),
+                vx=b.vx[:n].copy(), vy=b.vy[:n].copy(), slope_yx=b.slope_yx[:n].copy(), slope_xy=b.slope_xy[:n].copy(),
+                edge_flags=b.edge_flags[:n].copy(), beam_geom=b.beam_geom[:1].copy(), beam_flags=b.beam_flags[:1].copy())
+    g, w = S.grid(5, 2), S.wave()
+    th = np.deg2rad(np.array([150.0, 170.0, 175.0, 179.0, 179.5, 179.9, 179.95, 179.99]))
+    want = oracle.thetas_m11(b, 5, g.az_step, th, w)
+    h = GpuHandlerPO(g, w)
+    got = h.diffract_thetas_gpu(b, th)
+    h.close()
+    assert np.all(np.abs(got / want - 1.0) < FP64_L2 + 16 * 2.3e-16 / (1.0 + np.cos(th)))
