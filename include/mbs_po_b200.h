@@ -175,14 +175,17 @@ int mbs_po_diffract_pinned(mbs_po_ctx *ctx, const mbs_po_beams *beams, int preci
  * [n_az*(n_zen+1)*16] doubles, accumulated (+=) on `stream` (a cudaStream_t,
  * NULL for the legacy default stream). */
 int mbs_po_stage(mbs_po_ctx *ctx, const mbs_po_beams *beams, mbs_po_staged **out);
+/* Waits for the diffractions that read the batch.  ctx (NULL once it is
+ * destroyed) keeps up to 256 MiB of freed batches' device memory for the next
+ * ones; mbs_po_select_batch counts it as free. */
 int mbs_po_staged_free(mbs_po_ctx *ctx, mbs_po_staged *staged);
 /* Re-fill a staged batch with another host batch, in the device memory it
  * already holds (grown in stream order when the new batch needs more).  For
  * producers that stage batch after batch: a ring of staged batches re-filled
  * this way stops allocating once its slots have grown and never frees,
- * where mbs_po_staged_free + mbs_po_stage release memory (cudaFree waits for
- * all work on the device, the next batch's diffraction included) and take
- * it again.  Every diffraction that reads `staged` must have completed
+ * where mbs_po_staged_free + mbs_po_stage release memory (where the context
+ * does not keep it, cudaFree waits for all work on the device, the next
+ * batch's diffraction included) and take it again.  Every diffraction that reads `staged` must have completed
  * before the call (synchronise its stream, or an event recorded after it).
  * On failure the staged batch holds no orientations until it is re-filled.
  * No counterpart in the reference, which uploads every batch anew

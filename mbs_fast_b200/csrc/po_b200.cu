@@ -23,7 +23,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <iterator>
+#include <memory>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 using namespace mbs;
@@ -74,10 +77,75 @@ constexpr int kResultParts = 8;
 // bytes take the pack kernel's status.
 constexpr size_t kUploadBytes = (size_t)1 << 20;
 
-// One device allocation holding every per-batch array.
+// A context's memory pool; goes with the last arena or context that holds it
+// (destroying a pool while a batch staged from it lived on left the batch's
+// later cudaFree to a destroyed pool).
+struct Pool {
+    cudaMemPool_t h = nullptr;
+    ~Pool()
+    {
+        if (h)
+            cudaMemPoolDestroy(h);
+    }
+};
+
+// One device allocation holding every per-batch array: a block of its own, or
+// (`pool` set) memory of a context's pool.
 struct Arena {
     void *base = nullptr;
     size_t cap = 0;
+    std::shared_ptr<Pool> pool;
+};
+
+// The diffractions that may still read a staged batch: an event after the last
+// one on each stream.  `untracked`: a captured call reads it too, whose replays
+// leave no event here, or more streams did than are kept.
+class Readers {
+public:
+    Readers() { last_.reserve(kMostStreams); }
+    ~Readers()
+    {
+        for (auto &r : last_)
+            cudaEventDestroy(r.second);
+    }
+    // After a call's kernels have been queued on `st`.
+    void add(cudaStream_t st)
+    {
+        std::lock_guard<std::mutex> hold(lock_);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone
+            || cudaStreamGetId(st, &id) != cudaSuccess) {
+            untracked_ = true;
+            return;
+        }
+        auto it = std::find_if(last_.begin(), last_.end(), [&](const auto &r) { return r.first == id; });
+        if (it == last_.end()) {
+            cudaEvent_t ev = nullptr;
+            if (last_.size() >= kMostStreams || cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+                untracked_ = true;
+                return;
+            }
+            it = last_.insert(last_.end(), {id, ev});
+        }
+        if (cudaEventRecord(it->second, st) != cudaSuccess)
+            untracked_ = true;
+    }
+    // Waits for them; false when some may still be running.
+    bool wait()
+    {
+        std::lock_guard<std::mutex> hold(lock_);
+        for (auto &r : last_)
+            if (cudaEventSynchronize(r.second) != cudaSuccess)
+                return false;
+        return !untracked_;
+    }
+
+private:
+    static constexpr size_t kMostStreams = 16;
+    std::mutex lock_;
+    std::vector<std::pair<unsigned long long, cudaEvent_t>> last_;
+    bool untracked_ = false;
 };
 
 }  // namespace
@@ -98,6 +166,9 @@ struct mbs_po_staged {
     int n_sets = 1;                // output planes (size instances)
     int orient_per_set = 0;
     bool reused = false;           // re-filled by mbs_po_restage: grows like a context arena
+    int device = 0;
+    std::shared_ptr<Readers> readers;   // of this batch (null: the context's own)
+    std::shared_ptr<Readers> source;    // of the batch whose records a repeated batch shares
 };
 
 struct mbs_po_ctx {
@@ -107,7 +178,10 @@ struct mbs_po_ctx {
     // which keeps freed blocks (release threshold: never) instead of
     // returning them to the driver at every synchronisation: a growth step
     // then re-uses pool memory instead of mapping new pages
-    cudaMemPool_t pool = nullptr;
+    std::shared_ptr<Pool> pool;
+    // blocks of freed staged batches, for the next ones (kSpareBytes in all)
+    std::mutex spare_lock;
+    std::vector<std::pair<void *, size_t>> spare;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;          // polar-row kernel, concurrent
     std::string err;
@@ -165,6 +239,68 @@ int cuda_fail(mbs_po_ctx *ctx, cudaError_t e, const char *where)
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, where); \
     } while (0)
 
+// Freed staged batches' blocks that a context keeps, in all: staging a batch
+// in a kept block saves the 0.5 ms of cudaMalloc and 1 to 4 ms of cudaFree
+// that a batch of this size or less pays beside a diffraction of a few ms.
+constexpr size_t kSpareBytes = (size_t)256 << 20;
+
+size_t spare_bytes(mbs_po_ctx *ctx)
+{
+    std::lock_guard<std::mutex> hold(ctx->spare_lock);
+    size_t n = 0;
+    for (const auto &b : ctx->spare)
+        n += b.second;
+    return n;
+}
+
+// Gives kept blocks back to the device, the oldest first, until at most `keep`
+// bytes are left.
+void spare_trim(mbs_po_ctx *ctx, size_t keep)
+{
+    size_t n = spare_bytes(ctx);
+    std::lock_guard<std::mutex> hold(ctx->spare_lock);
+    while (n > keep && !ctx->spare.empty() && cudaFree(ctx->spare.front().first) == cudaSuccess) {
+        n -= std::min(n, ctx->spare.front().second);
+        ctx->spare.erase(ctx->spare.begin());
+    }
+}
+
+// What the context holds unused goes back to the device (before a request is
+// refused).
+void release_unused(mbs_po_ctx *ctx)
+{
+    cudaGetLastError();
+    spare_trim(ctx, 0);
+    cudaStreamSynchronize(ctx->stream);   // frees queued there have completed
+    cudaMemPoolTrimTo(ctx->pool->h, 0);
+    cudaGetLastError();
+}
+
+cudaError_t device_malloc(mbs_po_ctx *ctx, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        release_unused(ctx);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess)
+        *p = nullptr;
+    return e;
+}
+
+// Memory from the context's pool, in stream order on `st`.
+cudaError_t pool_alloc(mbs_po_ctx *ctx, void **p, size_t bytes, cudaStream_t st)
+{
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool->h, st);
+    if (e == cudaErrorMemoryAllocation) {
+        release_unused(ctx);
+        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool->h, st);
+    }
+    if (e != cudaSuccess)
+        *p = nullptr;
+    return e;
+}
+
 template <typename T>
 int ensure(mbs_po_ctx *ctx, T *&ptr, size_t &cap, size_t n, const char *what)
 {
@@ -175,51 +311,40 @@ int ensure(mbs_po_ctx *ctx, T *&ptr, size_t &cap, size_t n, const char *what)
     ptr = nullptr;
     cap = 0;
     const size_t alloc = std::max<size_t>(n, 1);
-    cudaError_t e = cudaMalloc((void **)&ptr, alloc * sizeof(T));
+    cudaError_t e = device_malloc(ctx, (void **)&ptr, alloc * sizeof(T));
     if (e != cudaSuccess)
         return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMalloc ") + what + ": " + cudaGetErrorString(e));
     cap = alloc;
     return MBS_PO_OK;
 }
 
-// Unused memory that a context's pool may keep after a staged batch is freed.
-constexpr size_t kPoolKeep = (size_t)512 << 20;
-
-// Memory from the context's pool, in stream order on `st`; what the pool keeps
-// unused is given back to the device before the request is refused.
-cudaError_t pool_alloc(mbs_po_ctx *ctx, void **p, size_t bytes, cudaStream_t st)
-{
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        cudaDeviceSynchronize();
-        cudaMemPoolTrimTo(ctx->pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
-    }
-    if (e != cudaSuccess)
-        *p = nullptr;
-    return e;
-}
-
-// A staged batch's arena: from the context's pool (mapping and unmapping
-// device memory per batch took 0.5 ms of cudaMalloc and 1 to 4 ms of cudaFree
-// on a batch that diffracts in 5), ready for every stream on return.
+// A staged batch's block: the smallest kept one that holds it and is not far
+// larger, or a new one.  Nothing reads a kept block (release_arena).
 int ensure_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what)
 {
+    bytes = std::max<size_t>(bytes, 256);
     if (bytes <= a.cap && a.base)
         return MBS_PO_OK;
-    if (a.base) {
-        CK(cudaDeviceSynchronize(), "releasing an arena");
-        cudaFree(a.base);
+    cudaFree(a.base);
+    a = Arena();
+    {
+        std::lock_guard<std::mutex> hold(ctx->spare_lock);
+        auto best = ctx->spare.end();
+        for (auto it = ctx->spare.begin(); it != ctx->spare.end(); ++it)
+            if (it->second >= bytes && it->second <= 4 * bytes + ((size_t)1 << 20)
+                && (best == ctx->spare.end() || it->second < best->second))
+                best = it;
+        if (best != ctx->spare.end()) {
+            a.base = best->first;
+            a.cap = best->second;
+            ctx->spare.erase(best);
+            return MBS_PO_OK;
+        }
     }
-    a.base = nullptr;
-    a.cap = 0;
-    cudaError_t e = pool_alloc(ctx, &a.base, std::max<size_t>(bytes, 256), ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(ctx->stream);
+    const cudaError_t e = device_malloc(ctx, &a.base, bytes);
     if (e != cudaSuccess)
-        return fail(ctx, MBS_PO_ENOMEM, std::string("device memory for the ") + what + ": " + cudaGetErrorString(e));
-    a.cap = std::max<size_t>(bytes, 256);
+        return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMalloc ") + what + ": " + cudaGetErrorString(e));
+    a.cap = bytes;
     return MBS_PO_OK;
 }
 
@@ -290,33 +415,34 @@ int grow_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what, cudaSt
         return fail(ctx, MBS_PO_ENOMEM, std::string("cudaMallocAsync ") + what + ": " + cudaGetErrorString(e));
     }
     a.cap = cap;
+    a.pool = ctx->pool;
     return MBS_PO_OK;
 }
 
-// Waits for all work on the device (a diffraction may still read the batch on
-// any stream) and gives the arena back to the context's pool (`ctx` null: the
-// context is gone, its pool goes with the last arena).
-void staged_release(mbs_po_ctx *ctx, mbs_po_staged *s)
+// Frees a staged batch's block: one that a context may keep stays with it once
+// its readers have completed, every other one goes by cudaFree, which waits for
+// the device.  (Waiting with cudaDeviceSynchronize instead broke a capture that
+// another thread had open.)
+void arena_release(mbs_po_ctx *ctx, mbs_po_staged *s)
 {
-    if (s->arena.base && cudaDeviceSynchronize() == cudaSuccess) {
-        if (ctx)
-            cudaFreeAsync(s->arena.base, ctx->stream);
-        else
-            cudaFree(s->arena.base);
+    Arena &a = s->arena;
+    const bool idle = !s->readers || s->readers->wait();
+    if (a.base && !a.pool && idle && ctx && ctx->device == s->device && a.cap <= kSpareBytes) {
+        spare_trim(ctx, kSpareBytes - a.cap);
+        std::lock_guard<std::mutex> hold(ctx->spare_lock);
+        ctx->spare.emplace_back(a.base, a.cap);
+    } else if (a.base) {
+        if (a.pool && !idle)
+            cudaDeviceSynchronize();   // cudaFree does not wait on pool memory
+        cudaFree(a.base);
     }
-    *s = mbs_po_staged();
+    a = Arena();
 }
 
-// More than kPoolKeep unused in the pool: all of it goes back to the device
-// (the pool releases whole blocks, a large batch's at once or not at all).
-void pool_trim(mbs_po_ctx *ctx)
+void staged_release(mbs_po_ctx *ctx, mbs_po_staged *s)
 {
-    uint64_t held = 0, used = 0;
-    if (cudaStreamSynchronize(ctx->stream) == cudaSuccess   // the frees have completed
-        && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess
-        && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess
-        && held > used + kPoolKeep)
-        cudaMemPoolTrimTo(ctx->pool, 0);
+    arena_release(ctx, s);
+    *s = mbs_po_staged();
 }
 
 int validate(mbs_po_ctx *ctx, const mbs_po_beams *b)
@@ -388,14 +514,13 @@ extern "C" int mbs_po_create(mbs_po_ctx **out, int device)
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        e = cudaMemPoolCreate(&ctx->pool, &props);
+        ctx->pool = std::make_shared<Pool>();
+        e = cudaMemPoolCreate(&ctx->pool->h, &props);
         uint64_t keep = ~(uint64_t)0;
         if (e == cudaSuccess)
-            e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            e = cudaMemPoolSetAttribute(ctx->pool->h, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     if (e != cudaSuccess) {
-        if (ctx->pool)
-            cudaMemPoolDestroy(ctx->pool);
         delete ctx;
         return MBS_PO_ECUDA;
     }
@@ -422,6 +547,7 @@ extern "C" int mbs_po_destroy(mbs_po_ctx *ctx)
     cudaFree(ctx->raw.base);
     cudaFree(ctx->d_status);
     staged_release(ctx, &ctx->host_staged);
+    spare_trim(ctx, 0);
     for (int i = 0; i < 8; ++i)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->partial_done)
@@ -433,10 +559,8 @@ extern "C" int mbs_po_destroy(mbs_po_ctx *ctx)
         cudaStreamDestroy(ctx->stream);
     if (ctx->side)
         cudaStreamDestroy(ctx->side);
-    // staged batches the caller still holds keep their blocks; the pool's
-    // resources go once the last of them is freed
-    if (ctx->pool)
-        cudaMemPoolDestroy(ctx->pool);
+    // staged batches the caller still holds keep their blocks, re-filled ones
+    // the pool too
     delete ctx;
     return MBS_PO_OK;
 }
@@ -492,15 +616,15 @@ extern "C" int mbs_po_set_grid(mbs_po_ctx *ctx, const mbs_po_grid *g)
     GridDev &d = ctx->grid;
     grid_release(d);
     const size_t nvf = (size_t)nAz * nT * 3;
-    CK(cudaMalloc((void **)&d.st, nT * sizeof(double)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.ct, nT * sizeof(double)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.sphi, nAz * sizeof(double)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.cphi, nAz * sizeof(double)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.vf, nvf * sizeof(double)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.theta, nT * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.st, nT * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.ct, nT * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.sphi, nAz * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.cphi, nAz * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.vf, nvf * sizeof(double)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.theta, nT * sizeof(double)), "cudaMalloc grid");
     CK(cudaMemcpy(d.theta, g->theta, nT * sizeof(double), cudaMemcpyHostToDevice), "grid copy");
-    CK(cudaMalloc((void **)&d.row_kind, nT * sizeof(int8_t)), "cudaMalloc grid");
-    CK(cudaMalloc((void **)&d.pole_rows, std::max<size_t>(poles.size(), 1) * sizeof(int32_t)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.row_kind, nT * sizeof(int8_t)), "cudaMalloc grid");
+    CK(device_malloc(ctx, (void **)&d.pole_rows, std::max<size_t>(poles.size(), 1) * sizeof(int32_t)), "cudaMalloc grid");
     CK(cudaMemcpy(d.st, st.data(), nT * sizeof(double), cudaMemcpyHostToDevice), "grid copy");
     CK(cudaMemcpy(d.ct, ct.data(), nT * sizeof(double), cudaMemcpyHostToDevice), "grid copy");
     CK(cudaMemcpy(d.sphi, sphi.data(), nAz * sizeof(double), cudaMemcpyHostToDevice), "grid copy");
@@ -616,6 +740,8 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
     const size_t o_boff = o_vbeg + align256((iB + 1) * sizeof(int32_t));
     const size_t o_w = o_boff + align256((iO + 1) * sizeof(int32_t));
     const size_t bytes = o_w + align256(std::max<int64_t>(iO, 1) * sizeof(double));
+    if (s->reused && !s->arena.pool && bytes > s->arena.cap)
+        arena_release(ctx, s);   // the block it was first staged in
     if ((rc = (s == &ctx->host_staged || s->reused ? grow_arena(ctx, s->arena, bytes, "staged batch", st)
                                                    : ensure_arena(ctx, s->arena, bytes, "staged batch"))))
         return rc;
@@ -963,6 +1089,18 @@ cudaError_t launch_rows(int precision, int variant, bool ns, KParams P, const Va
     return e;
 }
 
+// Notes a call on `st` that reads a staged batch, however the call ends.
+struct ReadScope {
+    const mbs_po_staged *s;
+    cudaStream_t st;
+    ~ReadScope()
+    {
+        for (Readers *r : {s->readers.get(), s->source.get()})
+            if (r)
+                r->add(st);
+    }
+};
+
 // How the chunk partials reach the caller: added into its accumulators,
 // stored there, or left in ctx->partial.
 enum class Sums { kAdd, kStore, kLeave };
@@ -1027,6 +1165,7 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
     P.partial = ctx->partial;
     P.partial_ns = ns ? ctx->partial + plane * L.n_chunks : nullptr;
     P.work = ctx->d_status + 1;
+    const ReadScope reading{s, st};
     int launches = 0;
     CK(cudaEventRecord(ctx->ev[0], st), "event");
     // polar rows and a row tail on the side stream, concurrently with the
@@ -1084,7 +1223,7 @@ extern "C" int mbs_po_autotune(mbs_po_ctx *ctx, const mbs_po_staged *s, int prec
     const int nv = pi == 0 ? kNumVariantsF64 : kNumVariantsF32;
     const int64_t G = (int64_t)ctx->grid.n_az * (ctx->grid.n_zen + 1);
     double *acc = nullptr;
-    CK(cudaMalloc((void **)&acc, G * 16 * sizeof(double)), "cudaMalloc autotune");
+    CK(device_malloc(ctx, (void **)&acc, G * 16 * sizeof(double)), "cudaMalloc autotune");
     int bestv = 0;
     double bestms = 1e300;
     for (int v = 0; v < nv; ++v) {
@@ -1124,12 +1263,24 @@ extern "C" int mbs_po_set_variant(mbs_po_ctx *ctx, int precision, int variant)
     return MBS_PO_OK;
 }
 
+namespace {
+
+mbs_po_staged *new_staged(mbs_po_ctx *ctx)
+{
+    mbs_po_staged *s = new mbs_po_staged();
+    s->device = ctx->device;
+    s->readers = std::make_shared<Readers>();
+    return s;
+}
+
+}  // namespace
+
 extern "C" int mbs_po_stage(mbs_po_ctx *ctx, const mbs_po_beams *beams, mbs_po_staged **out)
 {
     if (!ctx || !out)
         return fail(ctx, MBS_PO_EINVAL, "null argument");
     *out = nullptr;
-    mbs_po_staged *s = new mbs_po_staged();
+    mbs_po_staged *s = new_staged(ctx);
     int rc = stage_into(ctx, beams, s, ctx->stream);
     if (rc) {
         staged_release(ctx, s);
@@ -1175,8 +1326,6 @@ extern "C" int mbs_po_staged_free(mbs_po_ctx *ctx, mbs_po_staged *s)
     if (ctx)
         cudaSetDevice(ctx->device);
     staged_release(ctx, s);
-    if (ctx)
-        pool_trim(ctx);
     delete s;
     return MBS_PO_OK;
 }
@@ -1221,7 +1370,8 @@ extern "C" int mbs_po_stage_repeat(mbs_po_ctx *ctx, const mbs_po_staged *src, in
         boff.push_back(0);
     if (w.size() >= ((size_t)1 << 31))
         return fail(ctx, MBS_PO_ERANGE, "repeated batch exceeds 2^31 orientations");
-    mbs_po_staged *v = new mbs_po_staged();
+    mbs_po_staged *v = new_staged(ctx);
+    v->source = src->source ? src->source : src->readers;
     const size_t o_boff = 0, o_w = align256(boff.size() * sizeof(int32_t));
     int rc = ensure_arena(ctx, v->arena, o_w + std::max<size_t>(w.size(), 1) * sizeof(double), "repeated batch");
     if (rc) {
@@ -1661,7 +1811,7 @@ extern "C" int mbs_po_stage_multisize(mbs_po_ctx *ctx, const mbs_po_beams *beams
     if (!ctx || !out || !scales)
         return fail(ctx, MBS_PO_EINVAL, "null argument");
     *out = nullptr;
-    mbs_po_staged *s = new mbs_po_staged();
+    mbs_po_staged *s = new_staged(ctx);
     int rc = stage_into(ctx, beams, s, ctx->stream, scales, n_scales, wave_index);
     if (rc) {
         staged_release(ctx, s);
@@ -1950,6 +2100,7 @@ extern "C" int mbs_po_select_batch(mbs_po_ctx *ctx, const mbs_po_beams *beams, i
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     size_t freeB = 0, totalB = 0;
     CK(cudaMemGetInfo(&freeB, &totalB), "cudaMemGetInfo");
+    freeB += spare_bytes(ctx);   // kept, but there for a request that needs it
     if (!(mem_fraction > 0.1 && mem_fraction <= 0.98))
         mem_fraction = 0.88;   // MBS_GPU_MEM_FRACTION default (GpuDiffraction.cu:391-401)
     const int64_t G = ctx->has_grid ? (int64_t)ctx->grid.n_az * (ctx->grid.n_zen + 1) : 0;
@@ -2143,6 +2294,7 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     P.partial_ns = ns ? scratch + plane * L.n_chunks : nullptr;
     P.work = work;
     cudaStream_t st = (cudaStream_t)stream;
+    const ReadScope reading{s, st};
     const RowPlan R = plan_rows(precision, variant, ns, V, nT);
     const bool on_side = ctx->grid.n_pole > 0 || R.beside();
     if (on_side) {
