@@ -1962,6 +1962,10 @@ extern "C" int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beam
     return rc;
 }
 
+// Partial sums of a zenith scan (more only where one row of 192 points per
+// azimuth bin does not fit).
+constexpr size_t kThetaPartials = (size_t)24 << 20;
+
 extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams,
                                       const double *theta_rad, int n, double *m11_out)
 {
@@ -1994,30 +1998,34 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
         tab[n + i] = std::cos(th);
     }
     const int nAz = ctx->grid.n_az;
+    // The points go in slabs whose partial sums, one row of points per azimuth
+    // bin and beam chunk, take at most kThetaPartials: they lie in the upload
+    // area, which the batch no longer needs and which holds 32 MiB at least
+    // (scratch of their own, without a bound, took 735 MiB for 1.4 million
+    // beams, 48 bins and 721 points, and 0.9 ms of a context's first scan).
+    const size_t room = kThetaPartials / sizeof(double) / nAz;
+    const int slab = (int)std::min<size_t>(n, std::max<size_t>(room / 192 * 192, 192));
     // Three points per thread where a tile of 192 is mostly used.  Beam chunks:
     // as many equal CTAs as are resident at once (whole multiples of that for
-    // many beams, up to 8 stages a CTA), so that none wait for a second round;
-    // 64 beams a CTA whatever the batch made 2.7 rounds of 2,088 beams x 48
-    // azimuths.
-    const int dpt = n > 2 * kThetaTpb ? 3 : 1;
-    const int tiles = (n + dpt * kThetaTpb - 1) / (dpt * kThetaTpb);
+    // many beams, up to 8 stages a CTA while the partial sums have room), so
+    // that none wait for a second round; 64 beams a CTA whatever the batch made
+    // 2.7 rounds of 2,088 beams x 48 azimuths.
+    const int dpt = slab > 2 * kThetaTpb ? 3 : 1;
+    const int tiles = (slab + dpt * kThetaTpb - 1) / (dpt * kThetaTpb);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const int64_t resident = (int64_t)sms * 4, columns = (int64_t)tiles * nAz;
     const int64_t rounds = std::max<int64_t>(1, s.n_beams * columns / (resident * 8 * kThetaBeams));
     int64_t chunks = std::max<int64_t>(1, resident * rounds / columns);
-    chunks = std::min<int64_t>(std::min<int64_t>(chunks, 65535), (s.n_beams + 15) / 16);
+    chunks = std::min<int64_t>({chunks, 65535, (s.n_beams + 15) / 16, std::max<int64_t>(1, room / slab)});
     const int64_t bpc = (s.n_beams + chunks - 1) / chunks;
     chunks = (s.n_beams + bpc - 1) / bpc;
     const int64_t rows = chunks * nAz;
-    // scratch from the context's pool: the partial sums take megabytes, and a
-    // cudaMalloc and cudaFree of that size per call took longer than the kernel
-    double *buf = nullptr;
-    const size_t need = 2 * (size_t)n + (size_t)rows * n + n;
-    cudaError_t e = pool_alloc(ctx, (void **)&buf, need * sizeof(double), st);
-    if (e != cudaSuccess)
-        return fail(ctx, MBS_PO_ENOMEM, std::string("theta scan scratch: ") + cudaGetErrorString(e));
-    double *d_st = buf, *d_ct = buf + n, *part = buf + 2 * n, *d_m11 = part + (size_t)rows * n;
+    const size_t need = 3 * (size_t)n + (size_t)rows * slab;
+    if ((rc = grow_arena(ctx, ctx->raw, need * sizeof(double), "theta scan scratch", st)))
+        return rc;
+    double *buf = (double *)ctx->raw.base;
+    double *d_st = buf, *d_ct = buf + n, *d_m11 = buf + 2 * (size_t)n, *part = d_m11 + n;
     KParams P{};
     P.beams = s.beams;
     P.verts = s.verts;
@@ -2033,24 +2041,25 @@ extern "C" int mbs_po_diffract_thetas(mbs_po_ctx *ctx, const mbs_po_beams *beams
     P.n_az = nAz;
     P.n_orient = s.n_orient;
     P.wc = ctx->wc;
-    e = cudaMemcpyAsync(buf, tab.data(), 2 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
-        const dim3 g((unsigned)(tiles * nAz), (unsigned)chunks);
+    cudaError_t e = cudaMemcpyAsync(buf, tab.data(), 2 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st);
+    for (int t0 = 0; t0 < n && e == cudaSuccess; t0 += slab) {
+        const int m = std::min(slab, n - t0);
+        const dim3 g((unsigned)((m + dpt * kThetaTpb - 1) / (dpt * kThetaTpb) * nAz), (unsigned)chunks);
+        const int mt = (int)g.x / nAz;
         if (dpt == 3)
-            po_thetas_kernel<3><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, tiles, d_st, d_ct, n, part);
+            po_thetas_kernel<3><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, mt, d_st + t0, d_ct + t0, m, part);
         else
-            po_thetas_kernel<1><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, tiles, d_st, d_ct, n, part);
+            po_thetas_kernel<1><<<g, kThetaTpb, 0, st>>>(P, s.n_beams, (int)bpc, mt, d_st + t0, d_ct + t0, m, part);
         e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-        po_thetas_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(part, rows, n, nAz, d_m11);
-        e = cudaGetLastError();
+        if (e == cudaSuccess) {
+            po_thetas_sum_kernel<<<(m + 31) / 32, 1024, 0, st>>>(part, rows, m, nAz, d_m11 + t0);
+            e = cudaGetLastError();
+        }
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m11_out, d_m11, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(st);
-    cudaFreeAsync(buf, st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "theta scan");
     return MBS_PO_OK;

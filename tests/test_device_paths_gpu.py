@@ -425,3 +425,58 @@ def test_theta_scan_opposite_to_a_beam():
     got = h.diffract_thetas_gpu(b, th)
     h.close()
     assert np.all(np.abs(got / want - 1.0) < FP64_L2 + 16 * 2.3e-16 / (1.0 + np.cos(th)))
+
+
+def _first_beams(b, n):
+    """The batch's first n beams as two orientations, the first of one beam."""
+    v = int(b.vert_offsets[n])
+    return type(b)(beam_offsets=np.array([0, 1, n]), orient_weight=np.array([0.6, 0.4]),
+                   vert_offsets=b.vert_offsets[:n + 1].copy(), vx=b.vx[:v].copy(), vy=b.vy[:v].copy(),
+                   slope_yx=b.slope_yx[:v].copy(), slope_xy=b.slope_xy[:v].copy(), edge_flags=b.edge_flags[:v].copy(),
+                   beam_geom=b.beam_geom[:n].copy(), beam_flags=b.beam_flags[:n].copy())
+
+
+def _bins_for_one_chunk():
+    """Azimuth bins that give each bin's CTA all beams: at least the scan's
+    resident CTAs, four an SM."""
+    import torch
+    return 4 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_points,beams,nv", [(3, 63, 0), (3, 64, 0), (3, 65, 0), (3, 128, 0), (3, 150, 0),
+                                               (3, 20, 31), (3, 70, 9), (130, 65, 0), (130, 20, 31)])
+def test_theta_scan_stages(n_points, beams, nv):
+    """Zenith scan whose CTAs take several stages: beam counts around the 64
+    and vertex counts around the 256 of a stage, one and three points per
+    thread, near-forward (marked) pairs in every stage.  The gate per point."""
+    b = _first_beams(_with_nv(2 * beams, nv, 15.0, 3) if nv else S.batch(3, beams, 4.0, 9 + beams), beams)
+    g, w = S.grid(_bins_for_one_chunk(), 2), S.wave()
+    th = np.deg2rad(np.linspace(0.0, 180.0, n_points)) if n_points > 3 else np.array([0.0, 1e-4, 0.7])
+    want = oracle.thetas_m11(b, g.n_az, g.az_step, th, w)
+    h = GpuHandlerPO(g, w)
+    got = h.diffract_thetas_gpu(b, th)
+    h.close()
+    assert np.max(np.abs(got / want - 1.0)) < FP64_L2
+
+
+@pytest.mark.gpu
+def test_theta_scan_scratch_is_bounded():
+    """A scan with many beams needs no memory beyond its batch's; many azimuth
+    bins go in slabs of points (192 and the rest)."""
+    import torch
+    w = S.wave()
+    b = S.batch(1000, 100, 12.0, 5)
+    h = GpuHandlerPO(S.grid(48, 2), w)
+    h.extinction(b)                        # the upload area and the batch have their sizes
+    free = torch.cuda.mem_get_info()[0]
+    h.diffract_thetas_gpu(b, np.linspace(0.1, 3.0, 721))
+    assert torch.cuda.mem_get_info()[0] == free
+    h.close()
+    b, g = S.batch(1, 3, 12.0, 6), S.grid(16400, 2)
+    th = np.linspace(0.2, 3.0, 200)
+    want = oracle.thetas_m11(b, g.n_az, g.az_step, th, w)
+    h = GpuHandlerPO(g, w)
+    got = h.diffract_thetas_gpu(b, th)
+    h.close()
+    assert np.max(np.abs(got / want - 1.0)) < FP64_L2
