@@ -71,12 +71,6 @@ constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
 // the caller's arrays while the next is on its way.
 constexpr int kResultParts = 8;
 
-// Batches up to this size go to the device in two copies from a page-locked
-// image instead of one copy per array (each of those costs the host about 12
-// us: 170 us of a 560 us call on 16 orientations of 80 beams).  The last 64
-// bytes take the pack kernel's status.
-constexpr size_t kUploadBytes = (size_t)1 << 20;
-
 // A context's memory pool; goes with the last arena or context that holds it
 // (destroying a pool while a batch staged from it lived on left the batch's
 // later cudaFree to a destroyed pool).
@@ -202,7 +196,6 @@ struct mbs_po_ctx {
     size_t phiW_cap = 0;
     int phiW_low = 0, phiW_full = 0;
     Arena raw;                   // raw upload area for staging
-    unsigned char *hup = nullptr;   // page-locked image of a small batch's upload, kUploadBytes
     int *d_status = nullptr;      // [0] pack status, [1], [2] work counters of the diffraction kernel
     mbs_po_staged host_staged;   // reused by mbs_po_diffract
     cudaEvent_t ev[8] = {};
@@ -543,7 +536,6 @@ extern "C" int mbs_po_destroy(mbs_po_ctx *ctx)
     cudaFree(ctx->mfull);
     cudaFree(ctx->phiW);
     cudaFreeHost(ctx->hres);
-    cudaFreeHost(ctx->hup);
     cudaFree(ctx->raw.base);
     cudaFree(ctx->d_status);
     staged_release(ctx, &ctx->host_staged);
@@ -762,48 +754,25 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
         for (int64_t o = 0; o < nO; ++o)
             boff[i * nO + o] = (int32_t)(i * nB + b->beam_offsets[o]);
     boff[iO] = (int32_t)iB;
-    // the image: the raw area, then the arena's offsets and weights as they lie
-    // there (a batch without beams returns before the image's copies complete,
-    // so it takes the plain copies)
-    const size_t tail = o_w - o_boff + iO * sizeof(double);
-    unsigned char *up = nullptr;
-    if (nB > 0 && raw_bytes + tail <= kUploadBytes - 64) {
-        if (!ctx->hup && cudaMallocHost((void **)&ctx->hup, kUploadBytes) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->hup = nullptr;
-        }
-        up = ctx->hup;
-    }
-    auto put = [&](void *dst, size_t off, const void *src, size_t bytes) {
-        if (!up)
-            return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-        std::memcpy(up + off, src, bytes);
-        return cudaSuccess;
-    };
-    CK(put(s->beam_off, raw_bytes, boff.data(), (iO + 1) * sizeof(int32_t)), "H2D offsets");
+    CK(cudaMemcpyAsync(s->beam_off, boff.data(), (iO + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, st), "H2D offsets");
     for (int i = 0; i < nI && nO > 0; ++i)
-        CK(put(s->weight + i * nO, raw_bytes + (o_w - o_boff) + i * nO * sizeof(double), b->orient_weight,
-               nO * sizeof(double)), "H2D weights");
+        CK(cudaMemcpyAsync(s->weight + i * nO, b->orient_weight, nO * sizeof(double), cudaMemcpyHostToDevice, st), "H2D weights");
     if (nB > 0) {
-        CK(put(raw + off_vo, off_vo, b->vert_offsets, (nB + 1) * 8), "H2D vert_offsets");
-        CK(put(raw + off_vx, off_vx, b->vx, nV * 8), "H2D vx");
-        CK(put(raw + off_vy, off_vy, b->vy, nV * 8), "H2D vy");
-        CK(put(raw + off_syx, off_syx, b->slope_yx, nV * 8), "H2D slope_yx");
-        CK(put(raw + off_sxy, off_sxy, b->slope_xy, nV * 8), "H2D slope_xy");
-        CK(put(raw + off_g, off_g, b->beam_geom, nB * MBS_PO_GEOM_STRIDE * 8), "H2D geom");
-        CK(put(raw + off_ef, off_ef, b->edge_flags, nV), "H2D edge_flags");
-        CK(put(raw + off_bf, off_bf, b->beam_flags, nB), "H2D beam_flags");
+        CK(cudaMemcpyAsync(raw + off_vo, b->vert_offsets, (nB + 1) * 8, cudaMemcpyHostToDevice, st), "H2D vert_offsets");
+        CK(cudaMemcpyAsync(raw + off_vx, b->vx, nV * 8, cudaMemcpyHostToDevice, st), "H2D vx");
+        CK(cudaMemcpyAsync(raw + off_vy, b->vy, nV * 8, cudaMemcpyHostToDevice, st), "H2D vy");
+        CK(cudaMemcpyAsync(raw + off_syx, b->slope_yx, nV * 8, cudaMemcpyHostToDevice, st), "H2D slope_yx");
+        CK(cudaMemcpyAsync(raw + off_sxy, b->slope_xy, nV * 8, cudaMemcpyHostToDevice, st), "H2D slope_xy");
+        CK(cudaMemcpyAsync(raw + off_g, b->beam_geom, nB * MBS_PO_GEOM_STRIDE * 8, cudaMemcpyHostToDevice, st), "H2D geom");
+        CK(cudaMemcpyAsync(raw + off_ef, b->edge_flags, nV, cudaMemcpyHostToDevice, st), "H2D edge_flags");
+        CK(cudaMemcpyAsync(raw + off_bf, b->beam_flags, nB, cudaMemcpyHostToDevice, st), "H2D beam_flags");
         if (scales) {
-            CK(put(raw + off_sc, off_sc, scales, nI * 8), "H2D scales");
-            CK(put(raw + off_raw, off_raw, b->beam_raw, nB * MBS_PO_RAW_STRIDE * 8), "H2D raw Jones");
+            CK(cudaMemcpyAsync(raw + off_sc, scales, nI * 8, cudaMemcpyHostToDevice, st), "H2D scales");
+            CK(cudaMemcpyAsync(raw + off_raw, b->beam_raw, nB * MBS_PO_RAW_STRIDE * 8, cudaMemcpyHostToDevice, st), "H2D raw Jones");
             if (has_abs) {
-                CK(put(raw + off_ao, off_ao, b->abs_offsets, (nB + 1) * 8), "H2D abs offsets");
-                CK(put(raw + off_ap, off_ap, b->abs_paths, nAbs * 8), "H2D abs paths");
+                CK(cudaMemcpyAsync(raw + off_ao, b->abs_offsets, (nB + 1) * 8, cudaMemcpyHostToDevice, st), "H2D abs offsets");
+                CK(cudaMemcpyAsync(raw + off_ap, b->abs_paths, nAbs * 8, cudaMemcpyHostToDevice, st), "H2D abs paths");
             }
-        }
-        if (up) {
-            CK(cudaMemcpyAsync(raw, up, raw_bytes, cudaMemcpyHostToDevice, st), "H2D batch");
-            CK(cudaMemcpyAsync(s->beam_off, up + raw_bytes, tail, cudaMemcpyHostToDevice, st), "H2D orientations");
         }
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), st), "memset status");
         ctx->prof[1] = host_ms() - tg1;
@@ -837,12 +806,11 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
         const dim3 blocks((unsigned)((nB + kPackBeams - 1) / kPackBeams), (unsigned)nI);
         po_pack_kernel<<<blocks, kPackThreads, 0, st>>>(P);
         CK(cudaGetLastError(), "pack kernel launch");
-        int own = 0;
-        int *status = up ? reinterpret_cast<int *>(up + kUploadBytes - 64) : &own;
-        CK(cudaMemcpyAsync(status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
+        int status = 0;
+        CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
         CK(cudaStreamSynchronize(st), "pack sync");
         ctx->prof[2] = host_ms() - tg1 - ctx->prof[1];
-        if (*status)
+        if (status)
             return fail(ctx, MBS_PO_EBEAM, "malformed beam in batch");
     }
     s->n_orient = (int)iO;
