@@ -9,6 +9,7 @@
 //                chunk, no atomics.
 //   3. reduce:   po_reduce_kernel adds the chunk partials in a fixed order
 //                into the caller's accumulator (deterministic).
+#include "host_sums.h"
 #include "mbs_po_b200.h"
 #include "po_device.cuh"
 #include "po_kernels.cuh"
@@ -66,10 +67,6 @@ constexpr Variant kTailF32[] = {{64, 1, 4}, {96, 1, 4}, {128, 1, 4}, {96, 2, 4},
 constexpr Variant kTailF64[] = {{64, 1, 6}, {96, 1, 4}, {128, 1, 4}, {160, 1, 3}};
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
-
-// A host call's result comes back in up to this many parts, each added into
-// the caller's arrays while the next is on its way.
-constexpr int kResultParts = 8;
 
 // A context's memory pool; goes with the last arena or context that holds it
 // (destroying a pool while a batch staged from it lived on left the batch's
@@ -190,6 +187,8 @@ struct mbs_po_ctx {
     size_t macc_cap = 0;
     double *hres = nullptr;      // pinned [2][G*16]
     size_t hres_cap = 0;
+    double *kept = nullptr;      // the caller's values while a result is added in parts
+    size_t kept_cap = 0;
     double *mfull = nullptr;     // [2][n_full*(n_zen+1)*16] interpolated planes (FFT-phi calls)
     size_t mfull_cap = 0;
     double *phiW = nullptr;      // azimuth interpolation weights [n_full][n_low]
@@ -536,6 +535,7 @@ extern "C" int mbs_po_destroy(mbs_po_ctx *ctx)
     cudaFree(ctx->mfull);
     cudaFree(ctx->phiW);
     cudaFreeHost(ctx->hres);
+    std::free(ctx->kept);
     cudaFree(ctx->raw.base);
     cudaFree(ctx->d_status);
     staged_release(ctx, &ctx->host_staged);
@@ -1541,7 +1541,7 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
     // copy and 2 ms to add
     const size_t total = n_out * two;
     const int parts = view ? 1 : (int)std::min<size_t>(kResultParts, std::max<size_t>(1, total >> 18));
-    auto part_at = [&](int i) { return total * i / parts; };
+    auto part_at = [&](int i) { return result_part(total, parts, i); };
     for (int i = 0; i < parts; ++i) {
         CK(cudaMemcpyAsync(ctx->hres + part_at(i), dev_out + part_at(i), (part_at(i + 1) - part_at(i)) * sizeof(double),
                            cudaMemcpyDeviceToHost, st), "D2H");
@@ -1557,14 +1557,19 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
         view[0] = ctx->hres;
         view[1] = ns ? ctx->hres + n_out : nullptr;
     } else {
-        for (int p = 0; p < parts; ++p) {
-            if (p > 0)
-                CK(cudaEventSynchronize(ctx->part[p]), "sync");
-            const size_t a = part_at(p), b = part_at(p + 1);
-            for (size_t i = a; i < std::min(b, n_out); ++i)
-                M_accum[i] += ctx->hres[i];
-            for (size_t i = std::max(a, n_out); i < b; ++i)
-                Mns_accum[i - n_out] += ctx->hres[i];
+        if (parts > 1 && ctx->kept_cap < total) {
+            std::free(ctx->kept);
+            ctx->kept = static_cast<double *>(std::malloc(total * sizeof(double)));   // 16-byte aligned
+            ctx->kept_cap = ctx->kept ? total : 0;
+        }
+        cudaError_t e = cudaSuccess;
+        const bool ok = add_in_parts(
+            ctx->hres, total, n_out, parts, M_accum, Mns_accum, parts > 1 ? ctx->kept : nullptr,
+            [&](int p) { return (e = cudaEventSynchronize(ctx->part[p])) == cudaSuccess; },
+            [&]() { return cudaEventQuery(ctx->part[parts - 1]) == cudaSuccess; });
+        if (!ok) {
+            cudaStreamSynchronize(st);   // the copies still under way
+            return cuda_fail(ctx, e, "sync");
         }
     }
     CK(cudaStreamSynchronize(st), "sync");
