@@ -40,11 +40,14 @@ const char *mbs_mlp_last_error(const mbs_mlp *net);
 
 /* Watchdog of the tensor-core products (no counterpart in the reference).
  * Every layer product waits on its MMA-completion barrier for at most `poll_limit`
- * polls (<= 0: the default 2^22); when the wait runs out the kernel sets the
+ * polls, counted from when its weights have arrived (<= 0: the default 2^22);
+ * when the wait runs out the kernel sets the
  * network's device error flag, waits (bounded) for any MMA in flight, frees
  * its tensor memory and returns without storing, and the call fails with
  * "tensor-core barrier wait timed out" (mbs_mlp_last_error); the network
- * stays usable.  skip_mma != 0 is the test hook that exercises this path:
+ * stays usable.  In training the kernels behind it see the flag and store
+ * nothing either: the parameters and Adam moments stay as the steps before
+ * the failed one left them.  skip_mma != 0 is the test hook that exercises this path:
  * the products then issue no MMA and no commit, so the barrier never completes
  * and no asynchronous operation is pending when the wait gives up. */
 int mbs_mlp_set_watchdog(mbs_mlp *net, int poll_limit, int skip_mma);

@@ -264,6 +264,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
         grid_release();
         grid_wait();
     }
+    int failed = 0;
     if (tid == 0) {
         mbar_expect(bars + 8, kH * kInPad * 2 + 2 * kImg);
         bulk_load(sbase + L::W1, a.w.w1f, kH * kInPad * 2, bars + 8);
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             bulk_load(sbase + L::W3b, a.w.w3b, 2 * kImg, bars + 24);
             bulk_load(sbase + L::W2b, a.w.w2b, 2 * kImg, bars + 24);
         }
+        failed = *a.watch.err;   // a step before this one failed: nothing more is computed
     }
     if (tid < kRows) {   // a sample's input row: the quaternion, zeros to 16 columns
         const int r = r0 + tid;
@@ -297,23 +299,20 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
     const float b4 = a.params[ob4];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
+    bool ok = !__syncthreads_or(failed);
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tslot;
-    bool ok = true;
     uint32_t phase = 0;
     int loaded = 0;            // weight barriers waited for so far
     // One layer product W (128 x kt) times the staged samples: this thread's
     // accumulators.  `wbar`: the barrier of the weight operand.
     auto layer = [&](int woff, int soff, int kt, int wbar, float *v) {
-        if (tid == 0 && ok) {
-            while (loaded < wbar && ok) {
-                ++loaded;
-                ok = mbar_wait(bars + 8 * loaded, 0, kDefaultPollLimit);
-            }
-            if (ok && !a.watch.skip_mma)
-                mma_chain(tmem, sbase + woff, sbase + soff, kt, kRows, false, bars);
+        while (loaded < wbar && ok) {   // every thread: the MMA's own wait starts after it
+            ++loaded;
+            ok = mbar_wait(bars + 8 * loaded, 0, kDefaultPollLimit);
         }
+        if (tid == 0 && ok && !a.watch.skip_mma)
+            mma_chain(tmem, sbase + woff, sbase + soff, kt, kRows, false, bars);
         const bool done = mbar_wait(bars, phase, a.watch.poll_limit);
         phase ^= 1u;
         ok = __syncthreads_and(ok && done);
@@ -363,7 +362,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_chain(ChainArgs a)
             v[i] = v[i] * g[i];
         put(v, img, tile);
     };
-    layer(L::W1, L::X, kInPad, 1, v);
+    if (ok)
+        layer(L::W1, L::X, kInPad, 1, v);
     if (ok) {
         forward(g1, 0, a.img.h1);
         layer(L::W2f, L::H, kH, 1, v);
@@ -572,12 +572,15 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         }
         part[g][lane] = s;
         AdamState<1> ad;
+        int failed = 0;
+        if (g == 0)
+            failed = *a.watch.err;
         if (g == 0 && idx >= 0 && kAdam) {
             ad.load(a, idx);
             corrections();
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (g == 0 && idx >= 0) {
+        if (g == 0 && idx >= 0 && !failed) {
             float t = part[0][lane];
             for (int k = 1; k < 8; ++k)
                 t += part[k][lane];
@@ -594,10 +597,6 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
     const bf16 *B = l == 3 ? a.img.h2 : l == 2 ? a.img.h1 : a.img.x0;
     const size_t bstep = l == 1 ? kImgX : kImg;
     B += n0 * kTile;         // 8 rows of an image are 8 * 128 consecutive elements
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = *tslot;
     const int nblk = a.bp / kTile;
     int issued = 0, waited = 0, committed = 0;
     auto load = [&]() {
@@ -607,11 +606,17 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         bulk_load(d + 2 * kImg, B + (size_t)issued * bstep, kUpN * kTile * 2, bar);
         ++issued;
     };
+    int failed = 0;
     if (tid == 0) {
         load();
         if (nblk > 1)
             load();
+        failed = *a.watch.err;   // the chain or a step before it failed: nothing is stored
     }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    const bool run = !__syncthreads_or(failed);
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = *tslot;
     // accumulator row 32 (w % 4) + lane (the warp's lane quarter), columns
     // 4 (w / 4) .. + 3; their Adam state comes while the products run
     const int r = (warp & 3) * 32 + lane, cl = (warp >> 2) * 4, c = n0 + cl;
@@ -624,7 +629,7 @@ __global__ void __launch_bounds__(kUpThreads) k_update(UpdateArgs a)
         corrections();
     }
     if (tid == 0) {
-        bool ok = true;
+        bool ok = run;
         for (int i = 0; i < nblk && ok; ++i) {
             ok = mbar_wait(bars + 8 * (i & 1), (i >> 1) & 1, kDefaultPollLimit);
             waited = i + 1;
@@ -1210,7 +1215,6 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
                 return rc;
             return mfail(net, -3, std::string("training graph: ") + cudaGetErrorString(e));
         }
-        net->step += (int)steps;
     }
     if (rc == 0 && final_loss) {
         // loss over the whole set with the trained parameters
@@ -1229,5 +1233,7 @@ extern "C" int mbs_mlp_train(mbs_mlp *net, const float *q, const float *t, int n
         return rc;
     if (e != cudaSuccess)
         return mfail(net, -3, std::string("training: ") + cudaGetErrorString(e));
-    return check_err(net);
+    if ((rc = check_err(net)) == 0)
+        net->step += (int)steps;
+    return rc;
 }

@@ -480,3 +480,32 @@ def test_theta_scan_scratch_is_bounded():
     got = h.diffract_thetas_gpu(b, th)
     h.close()
     assert np.max(np.abs(got / want - 1.0)) < FP64_L2
+
+
+@pytest.mark.gpu
+def test_failed_training_leaves_the_network_alone():
+    """A tensor-core wait that runs out during training (the MMAs left out): the
+    call fails, the parameters are bit for bit what they were, and training
+    afterwards gives what an untouched network gives (moments and step count
+    included).  In a network that has trained before, and in a new one whose
+    activation memory nothing has written."""
+    from mbs_fast_b200.mlp import ProposalNet
+    rng = np.random.default_rng(5)
+    q = rng.normal(size=(300, 4))
+    q = (q / np.linalg.norm(q, axis=1, keepdims=True)).astype(np.float32)
+    t = np.sin(3 * q[:, 0]).astype(np.float32)
+    for before in (0, 2):
+        a, b = ProposalNet(seed=6), ProposalNet(seed=6)
+        for net in (a, b):
+            if before:
+                net.train(q, t, epochs=before, batch=128, lr=1e-3, seed=1)
+        p0 = a.params
+        a.set_watchdog(poll_limit=64, skip_mma=True)
+        with pytest.raises(RuntimeError, match="timed out"):
+            a.train(q, t, epochs=3, batch=128, lr=1e-3, seed=2)
+        a.set_watchdog(0, False)
+        assert np.array_equal(a.params, p0)
+        la, lb = (net.train(q, t, epochs=2, batch=128, lr=1e-3, seed=3) for net in (a, b))
+        assert la == lb and np.array_equal(a.params, b.params)
+        a.close()
+        b.close()
