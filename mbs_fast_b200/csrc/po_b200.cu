@@ -1027,11 +1027,23 @@ RowPlan plan_rows(int precision, int variant, bool ns, const Variant &V, int n_t
     return {tail < 0 ? n_t : n_t / rows * rows, tail};
 }
 
-// The diffraction launches: the main rows on `st`, a tail beside them on
-// `side` (which already waits for the start of the call), or alone on `st`.
-// P.work: two counters.
+// Whether a tail beside the main launch goes to the side stream.  In a captured
+// call only when polar rows go there anyway: a stream that the capture takes in
+// is closed to the context's other calls until the capture ends, and a grid
+// without polar rows lets those run meanwhile.
+bool tail_on_side(mbs_po_ctx *ctx, const RowPlan &R, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return R.beside()
+        && (ctx->grid.n_pole > 0
+            || (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone));
+}
+
+// The diffraction launches: the main rows on `st`, a tail beside them on `ts`
+// (the side stream, which already waits for the start of the call) or after
+// them on `st`.  P.work: two counters.
 cudaError_t launch_rows(int precision, int variant, bool ns, KParams P, const Variant &V, const RowPlan &R,
-                        int n_chunks, cudaStream_t st, cudaStream_t side)
+                        int n_chunks, cudaStream_t st, cudaStream_t ts)
 {
     cudaError_t e = cudaSuccess;
     if (R.main_rows > 0) {
@@ -1049,7 +1061,6 @@ cudaError_t launch_rows(int precision, int variant, bool ns, KParams P, const Va
         P.tiles_per_row = 1;
         P.n_items = n_chunks * P.n_az;
         ++P.work;
-        cudaStream_t ts = R.beside() ? side : st;
         e = cudaMemsetAsync(P.work, 0, sizeof(int), ts);
         if (e == cudaSuccess)
             e = launch_tail(precision == MBS_PO_FP64 ? 0 : 1, R.tail, P, ts);
@@ -1139,7 +1150,8 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
     // polar rows and a row tail on the side stream, concurrently with the
     // main kernel
     const RowPlan R = plan_rows(precision, variant, ns, V, nT);
-    const bool on_side = ctx->grid.n_pole > 0 || R.beside();
+    const bool tail_side = tail_on_side(ctx, R, st);
+    const bool on_side = ctx->grid.n_pole > 0 || tail_side;
     if (on_side)
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
     if (ctx->grid.n_pole > 0) {
@@ -1147,7 +1159,7 @@ int run_diffract(mbs_po_ctx *ctx, const mbs_po_staged *s, int precision, double 
            "pole kernel launch");
         ++launches;
     }
-    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, ctx->side);
+    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, tail_side ? ctx->side : st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "diffraction kernel launch");
     launches += R.beside() ? 2 : 1;
@@ -2170,7 +2182,7 @@ namespace {
 
 constexpr size_t kNoAllocScratchBytes = MBS_PO_NOALLOC_SCRATCH_BYTES;
 constexpr size_t kNoAllocScratchDoubles = kNoAllocScratchBytes / sizeof(double);
-constexpr size_t kNoAllocHead = 32;   // work counter, 256 bytes
+constexpr size_t kNoAllocHead = 32;   // two work counters, 256 bytes
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
 
@@ -2224,7 +2236,7 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     const bool ns = Mns_dev != nullptr;
     const size_t plane = (size_t)16 * G;
     const size_t sets = ns ? 2 : 1;
-    // the first kNoAllocHead doubles hold the work counter of the kernel
+    // the first kNoAllocHead doubles hold the kernels' two work counters
     int *work = reinterpret_cast<int *>(scratch);
     scratch += kNoAllocHead;
     // one partial plane per orientation chunk (and per output set) must fit
@@ -2278,7 +2290,8 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     cudaStream_t st = (cudaStream_t)stream;
     const ReadScope reading{s, st};
     const RowPlan R = plan_rows(precision, variant, ns, V, nT);
-    const bool on_side = ctx->grid.n_pole > 0 || R.beside();
+    const bool tail_side = tail_on_side(ctx, R, st);
+    const bool on_side = ctx->grid.n_pole > 0 || tail_side;
     if (on_side) {
         CK(cudaEventRecord(ctx->ev[0], st), "event");
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev[0], 0), "side wait");
@@ -2286,7 +2299,7 @@ extern "C" int mbs_po_diffract_staged_noalloc(mbs_po_ctx *ctx, const mbs_po_stag
     if (ctx->grid.n_pole > 0)
         CK(launch_pole(P, L, s->n_beams, s->n_orient, ctx->grid.pole_rows, ctx->grid.n_pole, ns, ctx->side),
            "pole kernel launch");
-    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, ctx->side);
+    const cudaError_t e = launch_rows(precision, variant, ns, P, V, R, L.n_chunks, st, tail_side ? ctx->side : st);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "diffraction kernel launch");
     if (on_side) {

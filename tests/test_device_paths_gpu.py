@@ -509,3 +509,51 @@ def test_failed_training_leaves_the_network_alone():
         assert la == lb and np.array_equal(a.params, b.params)
         a.close()
         b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_calls_beside_an_open_capture(noalloc):
+    """A grid without polar rows and with a row tail: while a capture of one
+    call is open, the context's other calls run, a second capture is taken, and
+    all give what the plain call gives."""
+    import torch
+    w, phi = S.wave(), np.arange(4) * (2 * np.pi / 4)
+    g = S.grid(4, 500)
+    vf = np.repeat(np.stack([-np.sin(phi), np.cos(phi), np.zeros(4)], -1)[:, None], 501, 1)
+    g = type(g)(4, 500, g.az_step, np.linspace(0.1, 3.0, 501), np.ascontiguousarray(vf), None)
+    h = GpuHandlerPO(g, w)
+    b = S.batch(3, 30, 12.0, 2)
+    st = h.stage(b)
+    accs = [torch.zeros(g.n_dirs * 16, dtype=torch.float64, device="cuda:0") for _ in range(3)]
+
+    def call(acc, stream):
+        if noalloc:
+            h.diffract_staged_noalloc(st, acc.data_ptr(), precision=abi.FP64, stream=stream.cuda_stream)
+        else:
+            h.diffract_staged(st, acc.data_ptr(), precision=abi.FP64, stream=stream.cuda_stream, stats=False)
+
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    call(accs[2], streams[0])
+    torch.cuda.synchronize()
+    graphs = [torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()]
+    with torch.cuda.stream(streams[0]):
+        graphs[0].capture_begin(capture_error_mode="relaxed")
+    call(accs[0], streams[0])
+    M = h.new_mueller()
+    assert h.handle_orientations_to_local_gpu(b, M, precision=abi.FP64)
+    with torch.cuda.stream(streams[1]):
+        graphs[1].capture_begin(capture_error_mode="relaxed")
+    call(accs[1], streams[1])
+    for s, gr in zip(streams, graphs):
+        with torch.cuda.stream(s):
+            gr.capture_end()
+    for gr in graphs:
+        gr.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(accs[0], accs[2]) and torch.equal(accs[1], accs[2])
+    assert np.max(np.abs(M.ravel() - accs[2].cpu().numpy())) <= 1e-12 * np.max(np.abs(M))
+    del graphs
+    st.free()
+    h.close()
