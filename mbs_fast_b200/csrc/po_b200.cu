@@ -93,12 +93,25 @@ struct Arena {
 // leave no event here, or more streams did than are kept.
 class Readers {
 public:
-    Readers() { last_.reserve(kMostStreams); }
+    // The first streams' events are made here, not in the call that reads (the
+    // allocation-free one among them).
+    Readers()
+    {
+        last_.reserve(kMostStreams);
+        for (cudaEvent_t &e : ready_)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+                e = nullptr;
+    }
     ~Readers()
     {
         for (auto &r : last_)
             cudaEventDestroy(r.second);
+        for (cudaEvent_t e : ready_)
+            if (e)
+                cudaEventDestroy(e);
     }
+    Readers(const Readers &) = delete;
+    Readers &operator=(const Readers &) = delete;
     // After a call's kernels have been queued on `st`.
     void add(cudaStream_t st)
     {
@@ -113,7 +126,10 @@ public:
         auto it = std::find_if(last_.begin(), last_.end(), [&](const auto &r) { return r.first == id; });
         if (it == last_.end()) {
             cudaEvent_t ev = nullptr;
-            if (last_.size() >= kMostStreams || cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+            if (last_.size() < std::size(ready_))
+                std::swap(ev, ready_[last_.size()]);
+            if (last_.size() >= kMostStreams
+                || (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)) {
                 untracked_ = true;
                 return;
             }
@@ -136,6 +152,7 @@ private:
     static constexpr size_t kMostStreams = 16;
     std::mutex lock_;
     std::vector<std::pair<unsigned long long, cudaEvent_t>> last_;
+    cudaEvent_t ready_[2] = {};
     bool untracked_ = false;
 };
 
