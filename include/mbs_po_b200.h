@@ -286,7 +286,7 @@ int mbs_po_phi_average(mbs_po_ctx *ctx, const double *M_dev, const double *dcos2
  * reference): rows_out[n_orient][(n_zen+1)*16] (host, overwritten), each
  * orientation's Mueller grid times its orientation weight, averaged over
  * azimuth as mbs_po_phi_average does.  The batch runs in groups of
- * orientations whose grids fit about 1 GiB of device memory. */
+ * orientations whose grids fit 256 MiB of device memory. */
 int mbs_po_orientation_rows(mbs_po_ctx *ctx, const mbs_po_beams *beams, int precision,
                             double *rows_out);
 

@@ -681,7 +681,7 @@ namespace {
 // orientations are [i nO, (i+1) nO) and its results go to output set i.
 // `what`: the records the call reads (a batch kept for later calls has all;
 // one staged for a single call leaves out what its kernels do not read).
-constexpr unsigned kStageDiffract = 1;   // BeamRec and VertRec
+constexpr unsigned kStageDiffract = 1;   // beam and vertex records
 constexpr unsigned kStageMoments = 2;    // FP32C near-forward moments
 constexpr unsigned kStageAll = kStageDiffract | kStageMoments;
 

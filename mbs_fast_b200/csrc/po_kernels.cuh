@@ -17,7 +17,7 @@ namespace mbs {
 
 // ------------------------------------------------------------------ records
 
-// Azimuth-independent per-beam coefficients, precomputed at staging.
+// A beam record: azimuth-independent coefficients, precomputed at staging.
 //   A(t, phi) = sin t (-(cos phi h0 + sin phi h1)) + cos t h2 + a0, B likewise.
 //   With vf = (-sin phi, cos phi, 0) off the poles, u = vt = -(cos phi cos t,
 //   sin phi cos t, sin t) and w = vt x dir = -vf, so the rotation of
@@ -29,15 +29,9 @@ namespace mbs {
 //   Q holds complWave * (X J_phased) for X1, X2, Y1, Y2, Z (4 complex
 //   entries each), so d = s m (P0 + cos t Pc + sin t Ps) with
 //   P0 = sin phi Q1 + cos phi Q2, Pc = -(cos phi Q3 + sin phi Q4), Ps = Q5.
-struct __align__(16) BeamRec {
-    double ab[8];     // h0 h1 h2 a0 v0 v1 v2 b0
-    double Q[40];
-    double slab[4];   // k (xa, ya) / 1.25e-3, k (xb, yb) / 1.25e-3 (see pack kernel)
-    float nearr2;     // FP32C near-forward zone: A^2+B^2 <= nearr2
-    int32_t vbeg;
-    int32_t nv;
-    int32_t pad;
-};
+//   slab: k (xa, ya) / 1.25e-3, k (xb, yb) / 1.25e-3, the small-phase candidate
+//   test (see the pack kernel); nearr2 (float): FP32C near-forward zone,
+//   A^2+B^2 <= nearr2.
 
 // Per vertex, azimuth-independent parts of the phase in turns:
 //   phase(t, phi) = sin t ps + cos t pc + p0,  ps = -(cos phi X + sin phi Y)
@@ -55,7 +49,9 @@ struct __align__(16) VertRec {
 // at base[w * stride + i], so the lanes of a warp that fill consecutive
 // records read consecutive words (full 32-byte sectors) instead of one
 // scattered sector per lane.
-constexpr int kBrecWords = 54;   // ab[8] Q[40] slab[4] (nearr2 | vbeg) (nv | beam flags)
+// Words of a beam record (low | high half of the last two): h0 h1 h2 a0 v0 v1 v2
+// b0, Q[40], slab[4], (nearr2 | vbeg), (nv | beam flags).
+constexpr int kBrecWords = 54;
 constexpr int kVrecWords = 6;    // X Y pc p0 syx sxy
 
 struct BrecRef {
@@ -82,19 +78,6 @@ struct VrecRef {
     __device__ __forceinline__ double syx() const { return p[4 * s]; }
     __device__ __forceinline__ double sxy() const { return p[5 * s]; }
 };
-
-__device__ __forceinline__ void store_brec(double *base, int64_t s, int64_t i, const BeamRec &r)
-{
-    double *p = base + i;
-    for (int w = 0; w < 8; ++w)
-        p[w * s] = r.ab[w];
-    for (int w = 0; w < 40; ++w)
-        p[(8 + w) * s] = r.Q[w];
-    for (int w = 0; w < 4; ++w)
-        p[(48 + w) * s] = r.slab[w];
-    p[52 * s] = __hiloint2double(r.vbeg, __float_as_int(r.nearr2));
-    p[53 * s] = __hiloint2double(0, r.nv);
-}
 
 __device__ __forceinline__ void store_vrec(double *base, int64_t s, int64_t i, const VertRec &r)
 {
@@ -423,7 +406,7 @@ __global__ void __launch_bounds__(kPackThreads) po_pack_kernel(PackParams P)
                 out[w * P.brec_stride] = d[(w & 3) == 3 ? w >> 2 : 2 + 3 * (w >> 2) + (w & 3)];
             } else if (w < 28) {
                 // group q of X1, X2, Y1, Y2, Z (rows r of the real 2x2
-                // matrix X, see BeamRec), entry e = 2 r + c of X J
+                // matrix X, see kBrecWords), entry e = 2 r + c of X J
                 const int q = (w - 8) >> 2, e = (w - 8) & 3, r = e >> 1, c = e & 1;
                 const int comp = q == 4 ? 2 : q & 1;       // x, y or z component
                 // vectors of row 0 / 1: (NT, NP) or (DT, DP); sign per group and row
@@ -691,7 +674,7 @@ __device__ __noinline__ void near_forward_s(const DevBeam &g, const double *mom,
 // lane of a warp reads the same record (a broadcast), so a beam costs ten
 // (FP32C) or eighteen (FP64) shared loads per thread for all DPT directions.
 //   A(t) = sin t a[0] + cos t a[1] + a[2],  B(t) = sin t a[3] + cos t a[4] + a[5]
-//   P0, Pc, Ps: complWave (R J) parts, 4 complex entries each (see BeamRec)
+//   P0, Pc, Ps: complWave (R J) parts, 4 complex entries each (see kBrecWords)
 //   slab: small-phase candidate test, nearr2: FP32C near-forward zone
 
 //   zone: nonzero when some direction of the CTA's zenith tile may fall in
@@ -2088,18 +2071,14 @@ __global__ void __launch_bounds__(256) po_phi_interp_kernel(const double *__rest
 // (L the Stokes rotation [1 0 0 0; 0 c s 0; 0 -s c 0; 0 0 0 1]), the polar
 // rows unrotated and projected (PoleMueller ApplyForward / ApplyBackward),
 // as HandlerPOTotal::WriteMatricesToFile writes them (reference
-// src/handler/HandlerPOTotal.cpp:49-96).  One CTA per row (grid y: one
-// Mueller grid after another); threads stride over azimuth bins, fixed-order
-// tree sum (deterministic).  rows[y][t][16].
+// src/handler/HandlerPOTotal.cpp:49-96).  One CTA per row; threads stride over
+// azimuth bins, fixed-order tree sum (deterministic).  rows[t][16].
 __global__ void __launch_bounds__(128) po_phi_average_kernel(const double *__restrict__ M, int n_az,
                                                             int n_t, const double *__restrict__ theta,
                                                             double *__restrict__ rows)
 {
     __shared__ double red[16][128];
     const int t = blockIdx.x;
-    // y: independent grids (one per orientation for per-orientation rows)
-    M += (size_t)blockIdx.y * n_az * n_t * 16;
-    rows += (size_t)blockIdx.y * n_t * 16;
     const double th = theta[t];
     const double tol = 256.0 * 2.220446049250313e-16;   // PoleMueller angular tolerance
     const bool fwd = fabs(th) <= tol;
@@ -2425,9 +2404,10 @@ __global__ void __launch_bounds__(kThetaTpb, 4) po_thetas_kernel(
                 const double q = fma(y0, y0, fma(y1, y1, y2 * y2));   // |R|^2
                 const double r = rcp64(m[d]);
                 const double xr = sr[d] * r, xi = si[d] * r;
-                const double e = fma(xr, xr, xi * xi) * q * b.w;
-                // a candidate's sums may be inf or NaN: select
-                acc[d] += cand[d] || isnan(e) ? 0.0 : e;
+                const double s2 = fma(xr, xr, xi * xi);
+                // a candidate's sums may be inf or NaN: select; a beam without a
+                // finite integral is left out, a NaN weight or Jones matrix is not
+                acc[d] += cand[d] || !isfinite(s2) ? 0.0 : s2 * q * b.w;
                 if (cand[d])
                     marked[d] |= 1ull << j;
             }

@@ -557,3 +557,27 @@ def test_calls_beside_an_open_capture(noalloc):
     del graphs
     st.free()
     h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["weight", "jones", "vertex"])
+def test_theta_scan_with_nan(what):
+    """A NaN weight or Jones matrix reaches every point of the scan; a beam whose
+    aperture integral is NaN (a NaN vertex) is left out (reference
+    GpuDiffraction.cu:1909-1956): as the oracle, point by point."""
+    b, g, w = S.batch(2, 30, 12.0, 8), S.grid(3, 2), S.wave()
+    th = np.array([0.3, 1.1, 2.6])
+    if what == "weight":
+        b.orient_weight = np.array([0.5, np.nan])
+    elif what == "jones":
+        b.beam_geom = b.beam_geom.copy()
+        b.beam_geom[7, abi.G_JP + 3] = np.nan
+    else:
+        b.vx = b.vx.copy()
+        b.vx[b.vert_offsets[7]] = np.nan
+    want = oracle.thetas_m11(b, 3, g.az_step, th, w)
+    assert np.isnan(want).all() == (what != "vertex") == np.isnan(want).any()
+    h = GpuHandlerPO(g, w)
+    got = h.diffract_thetas_gpu(b, th)
+    h.close()
+    np.testing.assert_allclose(got, want, rtol=FP64_L2)
