@@ -68,6 +68,15 @@ constexpr Variant kTailF64[] = {{64, 1, 6}, {96, 1, 4}, {128, 1, 4}, {160, 1, 3}
 constexpr int kNumVariantsF32 = sizeof(kVariantsF32) / sizeof(Variant);
 constexpr int kNumVariantsF64 = sizeof(kVariantsF64) / sizeof(Variant);
 
+// Host calls' batches up to this size go to the device in two copies from a
+// page-locked image instead of one copy per array (each of those costs the host
+// 2 to 12 us).  The image lies behind the page-locked result buffer, in the same
+// allocation, where that is at most 2 MiB with it or leaves the other set's
+// half to it: page-locking takes 0.9 to 3 ms up to 2 MiB and 1 ms a MiB beyond,
+// so an image of its own made a context's first call that much longer.  The last
+// 64 bytes take the pack kernel's status.
+constexpr size_t kUploadBytes = (size_t)1 << 20;
+
 // A context's memory pool; goes with the last arena or context that holds it
 // (destroying a pool while a batch staged from it lived on left the batch's
 // later cudaFree to a destroyed pool).
@@ -202,8 +211,9 @@ struct mbs_po_ctx {
     size_t partial_cap = 0;      // doubles
     double *macc = nullptr;      // [2][G*16] device accumulators for host calls
     size_t macc_cap = 0;
-    double *hres = nullptr;      // pinned [2][G*16]
+    double *hres = nullptr;      // pinned [2][G*16], then the upload image
     size_t hres_cap = 0;
+    unsigned char *hup = nullptr;   // image of a small host call's upload, kUploadBytes, behind hres
     double *kept = nullptr;      // the caller's values while a result is added in parts
     size_t kept_cap = 0;
     double *mfull = nullptr;     // [2][n_full*(n_zen+1)*16] interpolated planes (FFT-phi calls)
@@ -771,25 +781,42 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
         for (int64_t o = 0; o < nO; ++o)
             boff[i * nO + o] = (int32_t)(i * nB + b->beam_offsets[o]);
     boff[iO] = (int32_t)iB;
-    CK(cudaMemcpyAsync(s->beam_off, boff.data(), (iO + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, st), "H2D offsets");
+    // the image: the raw area, then the arena's offsets and weights as they lie
+    // there (a batch without beams returns before the image's copies complete,
+    // so it takes the plain copies; so does a batch that the caller keeps, which
+    // another thread may stage beside a host call)
+    const size_t tail = o_w - o_boff + iO * sizeof(double);
+    unsigned char *up = s == &ctx->host_staged && nB > 0 && raw_bytes + tail <= kUploadBytes - 64 ? ctx->hup : nullptr;
+    auto put = [&](void *dst, size_t off, const void *src, size_t bytes) {
+        if (!up)
+            return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        std::memcpy(up + off, src, bytes);
+        return cudaSuccess;
+    };
+    CK(put(s->beam_off, raw_bytes, boff.data(), (iO + 1) * sizeof(int32_t)), "H2D offsets");
     for (int i = 0; i < nI && nO > 0; ++i)
-        CK(cudaMemcpyAsync(s->weight + i * nO, b->orient_weight, nO * sizeof(double), cudaMemcpyHostToDevice, st), "H2D weights");
+        CK(put(s->weight + i * nO, raw_bytes + (o_w - o_boff) + i * nO * sizeof(double), b->orient_weight,
+               nO * sizeof(double)), "H2D weights");
     if (nB > 0) {
-        CK(cudaMemcpyAsync(raw + off_vo, b->vert_offsets, (nB + 1) * 8, cudaMemcpyHostToDevice, st), "H2D vert_offsets");
-        CK(cudaMemcpyAsync(raw + off_vx, b->vx, nV * 8, cudaMemcpyHostToDevice, st), "H2D vx");
-        CK(cudaMemcpyAsync(raw + off_vy, b->vy, nV * 8, cudaMemcpyHostToDevice, st), "H2D vy");
-        CK(cudaMemcpyAsync(raw + off_syx, b->slope_yx, nV * 8, cudaMemcpyHostToDevice, st), "H2D slope_yx");
-        CK(cudaMemcpyAsync(raw + off_sxy, b->slope_xy, nV * 8, cudaMemcpyHostToDevice, st), "H2D slope_xy");
-        CK(cudaMemcpyAsync(raw + off_g, b->beam_geom, nB * MBS_PO_GEOM_STRIDE * 8, cudaMemcpyHostToDevice, st), "H2D geom");
-        CK(cudaMemcpyAsync(raw + off_ef, b->edge_flags, nV, cudaMemcpyHostToDevice, st), "H2D edge_flags");
-        CK(cudaMemcpyAsync(raw + off_bf, b->beam_flags, nB, cudaMemcpyHostToDevice, st), "H2D beam_flags");
+        CK(put(raw + off_vo, off_vo, b->vert_offsets, (nB + 1) * 8), "H2D vert_offsets");
+        CK(put(raw + off_vx, off_vx, b->vx, nV * 8), "H2D vx");
+        CK(put(raw + off_vy, off_vy, b->vy, nV * 8), "H2D vy");
+        CK(put(raw + off_syx, off_syx, b->slope_yx, nV * 8), "H2D slope_yx");
+        CK(put(raw + off_sxy, off_sxy, b->slope_xy, nV * 8), "H2D slope_xy");
+        CK(put(raw + off_g, off_g, b->beam_geom, nB * MBS_PO_GEOM_STRIDE * 8), "H2D geom");
+        CK(put(raw + off_ef, off_ef, b->edge_flags, nV), "H2D edge_flags");
+        CK(put(raw + off_bf, off_bf, b->beam_flags, nB), "H2D beam_flags");
         if (scales) {
-            CK(cudaMemcpyAsync(raw + off_sc, scales, nI * 8, cudaMemcpyHostToDevice, st), "H2D scales");
-            CK(cudaMemcpyAsync(raw + off_raw, b->beam_raw, nB * MBS_PO_RAW_STRIDE * 8, cudaMemcpyHostToDevice, st), "H2D raw Jones");
+            CK(put(raw + off_sc, off_sc, scales, nI * 8), "H2D scales");
+            CK(put(raw + off_raw, off_raw, b->beam_raw, nB * MBS_PO_RAW_STRIDE * 8), "H2D raw Jones");
             if (has_abs) {
-                CK(cudaMemcpyAsync(raw + off_ao, b->abs_offsets, (nB + 1) * 8, cudaMemcpyHostToDevice, st), "H2D abs offsets");
-                CK(cudaMemcpyAsync(raw + off_ap, b->abs_paths, nAbs * 8, cudaMemcpyHostToDevice, st), "H2D abs paths");
+                CK(put(raw + off_ao, off_ao, b->abs_offsets, (nB + 1) * 8), "H2D abs offsets");
+                CK(put(raw + off_ap, off_ap, b->abs_paths, nAbs * 8), "H2D abs paths");
             }
+        }
+        if (up) {
+            CK(cudaMemcpyAsync(raw, up, raw_bytes, cudaMemcpyHostToDevice, st), "H2D batch");
+            CK(cudaMemcpyAsync(s->beam_off, up + raw_bytes, tail, cudaMemcpyHostToDevice, st), "H2D orientations");
         }
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), st), "memset status");
         ctx->prof[1] = host_ms() - tg1;
@@ -823,11 +850,12 @@ int stage_into(mbs_po_ctx *ctx, const mbs_po_beams *b, mbs_po_staged *s, cudaStr
         const dim3 blocks((unsigned)((nB + kPackBeams - 1) / kPackBeams), (unsigned)nI);
         po_pack_kernel<<<blocks, kPackThreads, 0, st>>>(P);
         CK(cudaGetLastError(), "pack kernel launch");
-        int status = 0;
-        CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
+        int own = 0;
+        int *status = up ? reinterpret_cast<int *>(up + kUploadBytes - 64) : &own;
+        CK(cudaMemcpyAsync(status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
         CK(cudaStreamSynchronize(st), "pack sync");
         ctx->prof[2] = host_ms() - tg1 - ctx->prof[1];
-        if (status)
+        if (*status)
             return fail(ctx, MBS_PO_EBEAM, "malformed beam in batch");
     }
     s->n_orient = (int)iO;
@@ -1539,9 +1567,14 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
     if (ctx->hres_cap < n_out * two || !ctx->hres) {
         cudaFreeHost(ctx->hres);
         ctx->hres = nullptr;
+        ctx->hup = nullptr;
         ctx->hres_cap = 0;
-        CK(cudaMallocHost((void **)&ctx->hres, n_out * two * sizeof(double)), "cudaMallocHost");
+        const size_t bytes = n_out * two * sizeof(double);
+        const bool image = bytes + kUploadBytes <= std::max((size_t)2 << 20, 2 * n_out * sizeof(double));
+        CK(cudaMallocHost((void **)&ctx->hres, bytes + (image ? kUploadBytes : 0)), "cudaMallocHost");
         ctx->hres_cap = n_out * two;
+        if (image)
+            ctx->hup = reinterpret_cast<unsigned char *>(ctx->hres + n_out * two);
     }
     for (double &v : ctx->prof)
         v = 0.0;
