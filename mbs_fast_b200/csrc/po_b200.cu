@@ -1018,7 +1018,7 @@ cudaError_t launch_reduce(const double *partial, int chunks_per_set, int64_t G, 
 // spills.  Kernel time, 300 orientations of 87 beams, 48 azimuths, FP32C (a
 // whole tile of 384 rows: 3.04 ms): up to 64 rows 1.03 ms, 96 rows 1.17, 128
 // rows 1.35, 192 rows 1.77, 256 rows 2.25; FP64, 150 orientations (192 rows:
-// 1.76 ms): 64 rows 0.77 ms, 96 rows 1.00, 128 rows 1.18, 160 rows 1.64.  Of
+// 1.77 ms): 64 rows 0.78 ms, 96 rows 1.01, 128 rows 1.24, 160 rows 1.70.  Of
 // the shapes compared one beam per iteration: 64 rows 1.11 ms in 64x1, 1.20 in
 // 96x1; 96 rows 1.22 in 96x1, 1.44 in 128x1, 1.22 with five CTAs per SM and
 // spills; 192 rows 1.79 in 96x2, 2.28 in 128x2, 1.93 in 64x3; 288 rows in 96x3

@@ -1621,7 +1621,9 @@ __global__ void __launch_bounds__(TPB, MINB) po_diffract_kernel(KParams P)
             // orientations of 87 beams, 48 azimuths, FP32C: 64 rows (64x1) 1108 ->
             // 1032 us, 96 (96x1) 1219 -> 1174, 128 (128x1) 1451 -> 1353, 192 (96x2)
             // 1790 -> 1768, 256 (128x2) 2301 -> 2246, no-shadow sums (128x3) 1041
-            // -> 1012; FP64, 150 orientations: 73 rows (96x1) 1021 -> 1002.  Slower
+            // -> 1012; FP64, 150 orientations: 64 rows (64x1) 797 -> 782, 96 (96x1)
+            // 1021 -> 1013, no-shadow sums (128x1 with 168 registers) of 61
+            // orientations on 47 x 358 1645 -> 1605.  Slower
             // where it adds spills or the directions fill the chain: FP32C 128x3
             // 3043 -> 3066, FP64 64x3 1762 -> 1905, 128x1 with 128 registers 1176 ->
             // 1215; four beams: 64x1 1143, 96x1 1311.
@@ -2257,7 +2259,7 @@ __global__ void __launch_bounds__(256) po_csca_kernel(const double *__restrict__
 // candidates are marked and evaluated in general form after the stage.
 // Bound by the FP64 pipe.  One thread per (point, beam, azimuth) with the
 // general evaluation took 1,225 us for 2,088 beams x 48 x 181 points, now
-// 229 us.
+// 245 us (229 with the quadratic form).
 struct __align__(16) ThetaBeam {
     double a[6];        // A, B coefficients (see BeamRegs)
     double u[6];        // U by rows: u00 u01 u02 u11 u12 u22
