@@ -455,6 +455,7 @@ void arena_release(mbs_po_ctx *ctx, mbs_po_staged *s)
             cudaDeviceSynchronize();   // cudaFree does not wait on pool memory
         cudaFree(a.base);
     }
+    cudaGetLastError();   // what a capture refused here is no error of the next call's
     a = Arena();
 }
 
@@ -1628,7 +1629,12 @@ int diffract_host(mbs_po_ctx *ctx, const mbs_po_beams *beams, const double *scal
         const bool ok = add_in_parts(
             ctx->hres, total, n_out, parts, M_accum, Mns_accum, parts > 1 ? ctx->kept : nullptr,
             [&](int p) { return (e = cudaEventSynchronize(ctx->part[p])) == cudaSuccess; },
-            [&]() { return cudaEventQuery(ctx->part[parts - 1]) == cudaSuccess; });
+            [&]() {
+                const bool all = cudaEventQuery(ctx->part[parts - 1]) == cudaSuccess;
+                if (!all)
+                    cudaGetLastError();   // "not ready" is no error of the next call's
+                return all;
+            });
         if (!ok) {
             cudaStreamSynchronize(st);   // the copies still under way
             return cuda_fail(ctx, e, "sync");
