@@ -151,7 +151,8 @@ int mbs_po_set_wave(mbs_po_ctx *ctx, const mbs_po_wave *wave);
 /* Host-buffer entry point: copy the batch to the device, run the fused
  * diffraction -> coherent Jones sum -> Mueller accumulation, and ADD the
  * weighted Mueller sums into M_accum (and, when non-NULL, the sum over
- * non-external beams into Mns_accum), both [n_az*(n_zen+1)*16] host arrays.
+ * non-external beams into Mns_accum), both [n_az*(n_zen+1)*16] host arrays; an
+ * error leaves both as they were.
  * Replaces HandlerPO::HandleOrientationsToLocalGpu
  * (reference src/handler/HandlerPO.h:108-120, GpuDiffraction.cu:4159-4778). */
 int mbs_po_diffract(mbs_po_ctx *ctx, const mbs_po_beams *beams, int precision,

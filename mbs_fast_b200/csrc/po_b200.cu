@@ -338,7 +338,7 @@ int ensure(mbs_po_ctx *ctx, T *&ptr, size_t &cap, size_t n, const char *what)
 }
 
 // A staged batch's block: the smallest kept one that holds it and is not far
-// larger, or a new one.  Nothing reads a kept block (release_arena).
+// larger, or a new one.  Nothing reads a kept block (arena_release).
 int ensure_arena(mbs_po_ctx *ctx, Arena &a, size_t bytes, const char *what)
 {
     bytes = std::max<size_t>(bytes, 256);
